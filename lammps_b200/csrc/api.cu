@@ -269,22 +269,28 @@ int init_replica_cells(b200_ctx *c) {
   const int R = c->nrep;
   c->rep_cell_base.assign(R, 0);
   c->rep_tile_base.assign(R + 1, 0);
+  const int ncells_before = c->ncells;
   long long cells = 0, tiles = 0;
   for (int r = 0; r < R; r++) {
     long long nc = 0;
     int rc = box_cells(c, c->rep_box[r], &nc);
     if (rc) return set_err(c, rc, "replica %d: %s", r, c->err.c_str());
     c->rep_cell_base[r] = (int)cells;
-    c->rep_tile_base[r] = (int)tiles;
     cells += nc;
+  }
+  c->ncells = (int)std::min(cells, 1LL << 30);
+  const int tc = md_tile_cells(c);
+  for (int r = 0; r < R; r++) {
     const BoxGeom &b = c->rep_box[r];
-    tiles += (long long)((b.ncell[0] + MD_TILE_CELLS - 1) / MD_TILE_CELLS) * b.ncell[1] * b.ncell[2];
+    c->rep_tile_base[r] = (int)tiles;
+    tiles += (long long)((b.ncell[0] + tc - 1) / tc) * b.ncell[1] * b.ncell[2];
   }
   c->rep_tile_base[R] = (int)tiles;
   if (cells > (long long)4096 * 4096 - 1 || tiles > 0x7fffffffLL)
     return set_err(c, B200_ERR_ARG, "too many cells (%lld)", cells);
-  if ((int)cells != c->ncells || (int)tiles != c->ntiles) invalidate_graphs(c);
-  c->ncells = (int)cells;
+  if ((int)cells != ncells_before || (int)tiles != c->ntiles || tc != c->tile_cells)
+    invalidate_graphs(c);
+  c->tile_cells = tc;
   c->ntiles = (int)tiles;
   c->box = c->rep_box[0];
   std::vector<int> tile_rep(tiles), rep_of_atom(c->n);
@@ -365,6 +371,7 @@ int init_cutoffs_and_cells(b200_ctx *c) {
     return set_err(c, B200_ERR_ARG, "too many cells (%lld)", ncells);
   if ((int)ncells != c->ncells) invalidate_graphs(c);  // scan launch shape changes
   c->ncells = (int)ncells;
+  c->tile_cells = md_tile_cells(c);  // set by n and ncells, which both invalidate the graphs
   return B200_OK;
 }
 

@@ -18,7 +18,6 @@
 #include <stdint.h>
 
 #define MD_MAXTYPES 8
-#define MD_TILE_CELLS 4    // cells along x owned by one neighbor-builder CTA
 #define MD_ADJ_MAXTYPES 4  // types of the force-matching adjoint (16 type pairs)
 #define MD_JBITS 26
 #define MD_JMASK ((1u << MD_JBITS) - 1u)
@@ -40,7 +39,7 @@ enum {
   ST_STEP_LO = 9,    // current timestep (low/high 32 bits)
   ST_STEP_HI = 10,
   ST_FORCE_BUILD = 11,  // rebuild on the next step regardless of the schedule
-  ST_MAXSTAGE = 12,     // most atoms staged by one neighbor-builder tile since setup
+  ST_MAXSTAGE = 12,     // most shared memory (16-byte units) one builder tile needed
   ST_HALO_BAD = 13,     // a halo pack/unpack index was outside [0, n)
   ST_BADTYPE = 14,      // 1 + index of an uploaded atom with a type outside [1, ntypes]
   ST_COUNT = 16

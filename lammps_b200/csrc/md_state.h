@@ -146,7 +146,8 @@ struct b200_ctx {
   // neighbor list
   int *nlist = nullptr, *numneigh = nullptr;
   int capacity = 0;     // entries per atom
-  int stage_need = 0;   // staged atoms per builder tile seen by earlier builds
+  int stage_need = 0;   // shared memory (16-byte units) per builder tile seen by earlier builds
+  int tile_cells = 1;   // cells along x owned by one builder CTA (md_tile_cells)
   long long nlist_alloc = 0;
 
   // run-chunk snapshot for overflow replay (x4, v, f, xhold planes + ids)
@@ -242,6 +243,7 @@ inline bool md_q_iso(const b200_ctx *c) {
 // ---- launchers (neigh.cu) -------------------------------------------------
 // full rebuild: wrap, cell counting sort, permute, neighbor list
 cudaError_t md_rebuild(b200_ctx *c, const int *d_flag);
+int md_tile_cells(const b200_ctx *c);
 int md_stage_cap(const b200_ctx *c);
 bool md_stage_feedback(b200_ctx *c, int staged_max);
 // LAMMPS half list derived from the full list; returns entry count via *total

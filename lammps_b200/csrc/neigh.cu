@@ -18,6 +18,11 @@
 // formed as x_j + s*L in FP64 and rsq = dx*dx + dy*dy + dz*dz is rounded
 // after every operation, then compared with `<=` to (rc+skin)^2
 // (src/neigh_half_bin.cpp:355-360, src/atom_vec_atomic.cpp:297-299).
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <atomic>
+#include <cmath>
 #include <cstdio>
 
 #include "md_state.h"
@@ -243,49 +248,64 @@ __global__ void k_copyback(int n, int stride, const double4 *__restrict__ x4b,
   image[k] = imageb[k];
 }
 
-// Full neighbor list with shared-memory staging of neighbor-cell tiles.
-// A CTA owns kTileCells consecutive cells along x; the 3 x 3 x (kTileCells+2)
-// block of cells around them is staged in shared memory as 9 contiguous
-// ranges of the cell-sorted atom arrays (positions as FP32 offsets from the
-// CTA's reference point, with the periodic image already applied).  Each
-// thread takes one atom of the owned cells and scans its 27 neighbor cells
-// from shared memory.  The FP32 distance decides every pair whose rsq lies
-// outside a relative band of 1e-5 around (rc+skin)^2; pairs inside the band
-// are decided by the reference's FP64 arithmetic on the global FP64
-// positions, so the list is bit-identical to the FP64 criterion.
-constexpr int kTileCells = MD_TILE_CELLS;
-// staged atoms per tile at most: 8192 x 16 B = 128 KB of shared memory, with
-// the opt-in above the default 48 KB (set on the first build)
-constexpr int kStageCapMax = 8192;
-constexpr int kStageCells = 3 * 3 * (kTileCells + 2);
-constexpr int kNeighThreads = 32 * kTileCells;  // one warp per owned cell
+// Full neighbor list from staged neighbor-cell tiles.
+// A CTA owns TC consecutive cells along x (their atoms are contiguous in the
+// cell-sorted order) and stages the 3 x 3 x (TC+2) block of cells around
+// them in shared memory, periodic images applied.  Three phases:
+//   test    r^2 - cut^2 of every (candidate, owned atom) pair.  It is a
+//           contraction, |a|^2 + (|b|^2 - cut^2) - 2 a.b, so the tensor cores
+//           do it: coordinates relative to the tile centre are split into
+//           FP16 hi + lo halves, whose products are exact in the FP32
+//           accumulator, and one mma.m16n8k16 evaluates 128 pairs (all four
+//           half products of three dimensions, the candidate's norm, and the
+//           owned atom's norm less the cutoff fill K = 16).  The sign bit is the decision; a
+//           funnel shift collects it, one instruction per value.  Pairs
+//           within `eps` of the cutoff are decided by the reference's FP64
+//           arithmetic on the FP64 positions, so the list is bit-identical
+//           to the FP64 criterion.
+//   order   eight atoms x four 32-candidate chunks a warp: the acceptance
+//           bits are brought into candidate order (two 2-bit index fields
+//           swap) and empty words dropped.
+//   append  one thread per owned atom walks its words; with no empty words
+//           the threads of a warp are at the same entry, so the slabs they
+//           store are contiguous.
+// Bound by instruction issue: one FP32 distance test per pair and lane, with a
+// ballot per owned atom, took 788 warp instructions per atom (0.82 us per
+// 1,000 atoms at 4,000,000); this form takes about 330 (0.5 us).  With the
+// wider grid of small tiles a 32,000-atom build went from 69 us to 25 us and
+// an 864-atom one from 89 us to 20 us.
+// (mma.sync rather than tcgen05: the operands are a few cells, 56 x 19
+// values, and the result is wanted as bits per lane, not as a tile in TMEM.)
+//
+// Error bound behind eps.  Let rb bound the owned atoms' distance from the
+// tile centre and ra = rb + cutoff that of a candidate near an owned atom's
+// cutoff.  Relative to 2^-20: a coordinate's FP32 rounding (2^-24, both sides
+// of the separation) moves r^2 by at most 0.25 ra^2, the FP16 hi + lo split
+// (2^-22, in the product only) by ra^2, the FP32 norms and their splits by
+// 1.2 ra^2, and 16 accumulations, each truncated at 2^-23 of a sum below
+// (ra + rb)^2, by 2 (ra + rb)^2.  eps = 1.25 x 2^-19 ((ra + rb)^2 + 2 ra^2) is
+// above 1.25 x their sum.  (A pair further apart has a larger error, but its
+// value grows 2 x cutoff per unit length, far faster than the bound.)
+constexpr int kNeighThreads = 128;
+constexpr int kMaxCols = 384;  // owned atoms of a tile, padded to eight per cell, at most
+// 32-candidate chunks of one cell's nine rows, at most
+constexpr int max_chunks(int tc) { return 192 / tc; }
+// most dynamic shared memory a tile may take (opt-in), in 16-byte units
+constexpr int kStageUnitsMax = 200 * 1024 / 16;
 
-// The last four list entries of a thread rotate through an int4 register
-// buffer; every fourth append stores the slab with one 16-byte write.
-__device__ __forceinline__ void append_entry(int *__restrict__ nlist, int stride, int i,
-                                             int &count, int capacity, int e, int4 &buf) {
-  buf.x = buf.y;
-  buf.y = buf.z;
-  buf.z = buf.w;
-  buf.w = e;
-  if ((count & 3) == 3 && count < capacity)
-    reinterpret_cast<int4 *>(nlist)[(size_t)(count >> 2) * stride + i] = buf;
-  count++;
-}
-
-// store the last, partly filled slab (its r entries sit at the end of buf;
-// the rest of the slab is filled with the atom's pad entry)
-__device__ __forceinline__ void flush_entries(int *__restrict__ nlist, int stride, int i,
-                                              int count, int capacity, const int4 &buf) {
-  const int r = count & 3;
-  if (r == 0 || count - 1 >= capacity) return;
-  const int pad = md_pad_entry(i);
-  int4 o = make_int4(pad, pad, pad, pad);
-  if (r == 1) o.x = buf.w;
-  else if (r == 2) { o.x = buf.z; o.y = buf.w; }
-  else { o.x = buf.y; o.y = buf.z; o.z = buf.w; }
-  reinterpret_cast<int4 *>(nlist)[(size_t)(count >> 2) * stride + i] = o;
-}
+struct NeighArgs {
+  int n, stride, capacity, units, ntp1, pass, units1;
+  BoxGeom box;
+  Reps reps;
+  double scale;   // power of two that brings the largest list cutoff into [2, 4)
+  float cmax;     // largest list cutoff, scaled, squared
+  float dmax;     // largest difference of a type pair's from it, scaled, squared
+  const double *cutneighsq;
+  const double4 *x4;
+  const int *cell_start;
+  int *nlist, *numneigh, *status;
+  const int *flag;
+};
 
 // exact reference criterion for one candidate (FP64, no contraction)
 __device__ __forceinline__ bool exact_pair(const double4 &xi, const double4 &xj, double shx,
@@ -296,239 +316,508 @@ __device__ __forceinline__ bool exact_pair(const double4 &xi, const double4 &xj,
   return dsq3(delx, dely, delz) <= cutsq;
 }
 
-// Shared memory of k_neigh_tiles: stage_cap + 32 float4 staged atoms (32
-// spare slots: a chunk may read past a row).  The .w word of a staged atom
-// packs its list entry and type: bits 6..31 the atom index, bits 3..5 the
-// type minus one, bits 0..2 the staged column sx (0 .. kTileCells+1).
-static size_t neigh_smem(int stage_cap) { return (size_t)(stage_cap + 32) * sizeof(float4); }
+// staged word: (atom index << 6) + the staged cell's row code (dy+1)<<2 |
+// (dz+1)<<4 + its column sx (0 .. TC+1); less the owned cell's column (0 ..
+// TC-1) it is the list entry
+__device__ __forceinline__ int row_code(int row) { return ((row % 3) << 2) + ((row / 3) << 4); }
 
-__device__ __forceinline__ int stage_word(int j, int type, int sx) {
-  return (int)(((unsigned)j << 6) | ((unsigned)(type - 1) << 3) | (unsigned)sx);
+// FP16 hi + lo of three coordinates and of their squared norm plus `add`,
+// one word each (hi in the low half)
+__device__ __forceinline__ uint4 record(float x, float y, float z, float add) {
+  const float n = fmaf(x, x, fmaf(y, y, fmaf(z, z, add)));
+  const __half2 hxy = __floats2half2_rn(x, y), hzn = __floats2half2_rn(z, n);
+  const __half2 lxy = __floats2half2_rn(x - __low2float(hxy), y - __high2float(hxy));
+  const __half2 lzn = __floats2half2_rn(z - __low2float(hzn), n - __high2float(hzn));
+  const unsigned h0 = *reinterpret_cast<const unsigned *>(&hxy),
+                 h1 = *reinterpret_cast<const unsigned *>(&hzn),
+                 l0 = *reinterpret_cast<const unsigned *>(&lxy),
+                 l1 = *reinterpret_cast<const unsigned *>(&lzn);
+  return make_uint4(__byte_perm(h0, l0, 0x5410), __byte_perm(h0, l0, 0x7632),
+                    __byte_perm(h1, l1, 0x5410), __byte_perm(h1, l1, 0x7632));
 }
-__device__ __forceinline__ int stage_type(float w) { return ((__float_as_int(w) >> 3) & 7) + 1; }
-// the list entry (j << 6 | sx) of a staged atom
-__device__ __forceinline__ unsigned stage_entry(float w) {
-  return (unsigned)__float_as_int(w) & ~0x38u;
+__device__ __forceinline__ float join16(unsigned w) {
+  return __half2float(__ushort_as_half((unsigned short)w)) +
+         __half2float(__ushort_as_half((unsigned short)(w >> 16)));
 }
 
-template <bool SINGLE, bool BATCH>
-__global__ void __launch_bounds__(kNeighThreads, 8) k_neigh_tiles(
-    int n, int stride, int capacity, int stage_cap, BoxGeom box1, Reps reps, int ntp1,
-    const double *__restrict__ cutneighsq_g, const double4 *__restrict__ x4,
-    const int *__restrict__ cell_start_g, int *__restrict__ nlist, int *__restrict__ numneigh,
-    int *__restrict__ status, const int *flag, int pass, int cap1) {
-  if (!rebuild_on(flag)) return;
+__device__ __forceinline__ void mma16(float (&d)[4], unsigned a0, unsigned a1, unsigned a2,
+                                      unsigned a3, unsigned b0, unsigned b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ void mma8(float (&d)[4], unsigned a0, unsigned a1, unsigned b0) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+      "{%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(b0));
+}
+
+// least magnitude of a lane's eight values and `m`
+__device__ __forceinline__ float least(float m, const float (&d)[4], const float (&e)[4]) {
+  asm("min.abs.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(d[0]), "f"(d[1]));
+  asm("min.abs.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(d[2]), "f"(d[3]));
+  asm("min.abs.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(e[0]), "f"(e[1]));
+  asm("min.abs.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(e[2]), "f"(e[3]));
+  return m;
+}
+
+// acceptance byte of one lane: the sign bits of its eight values, the even
+// owned atom's four (candidates g, g+8, g+16, g+24) in the low nibble
+__device__ __forceinline__ unsigned sign_byte(const float (&d)[4], const float (&e)[4]) {
+  unsigned r = 0;
+  r = __funnelshift_l(__float_as_uint(e[3]), r, 1);
+  r = __funnelshift_l(__float_as_uint(e[1]), r, 1);
+  r = __funnelshift_l(__float_as_uint(d[3]), r, 1);
+  r = __funnelshift_l(__float_as_uint(d[1]), r, 1);
+  r = __funnelshift_l(__float_as_uint(e[2]), r, 1);
+  r = __funnelshift_l(__float_as_uint(e[0]), r, 1);
+  r = __funnelshift_l(__float_as_uint(d[2]), r, 1);
+  return __funnelshift_l(__float_as_uint(d[0]), r, 1);
+}
+
+// bit 8 (g & 3) + 4 (g >> 2) + m of a lane-order word is candidate g + 8 m:
+// exchange the index fields (bits 4,3) and (bits 1,0)
+__device__ __forceinline__ unsigned candidate_order(unsigned x) {
+  unsigned t = ((x >> 14) ^ x) & 0x0000CCCCu;
+  x = x ^ t ^ (t << 14);
+  t = ((x >> 7) ^ x) & 0x00AA00AAu;
+  return x ^ t ^ (t << 7);
+}
+
+// 16-byte units of shared memory of a tile: staged records (16 B), words
+// (4 B) and, with several types, types (1 B) with 32 spare slots, and the
+// acceptance words (4 B) with their first slots (2 B)
+__host__ __device__ inline int tile_units(int nstage, int chunks, int cols, bool single) {
+  const int m = nstage + 32, c = chunks * cols;
+  return m + (m + 3) / 4 + (single ? 0 : (m + 15) / 16) + (c + 3) / 4 + (c + 7) / 8;
+}
+// the units of a tile of tc cells at a mean of `per_cell` atoms per cell
+inline int tile_units_of(double per_cell, int tc, bool single) {
+  const int stage = (int)(1.15 * 9 * (tc + 2) * per_cell) + 32;
+  const int chunks = 9 * ((int)(3.0 * per_cell / 32.0) + 1) + 3;
+  const int cols = tc * (((int)(per_cell + 2.0) + 7) & ~7) + 8;
+  return tile_units(stage, chunks, cols, single);
+}
+
+template <int TC, bool SINGLE, bool BATCH>
+__global__ void __launch_bounds__(kNeighThreads, 8) k_neigh_tiles(NeighArgs A) {
+  if (!rebuild_on(A.flag)) return;
+  constexpr int NSX = TC + 2, NST = 9 * NSX;
+  constexpr int WPC = kNeighThreads / 32 / TC;  // warps per owned cell
   // batched: this tile's replica, its box and its cells' slice of cell_start
-  const int rep = BATCH ? reps.tile_rep[blockIdx.x] : 0;
-  const int tile = BATCH ? blockIdx.x - reps.tile_base[rep] : blockIdx.x;
-  const BoxGeom &box = BATCH ? reps.box[rep] : box1;
-  const int *__restrict__ cell_start = BATCH ? cell_start_g + reps.cell_base[rep] : cell_start_g;
-  extern __shared__ float4 s_stage[];
-  float4 *sp = s_stage;
-  __shared__ int s_start[kStageCells + 1];
-  __shared__ int s_src[kStageCells];
-  __shared__ double s_sh[kStageCells][3];
-  __shared__ double cns[(MD_MAXTYPES + 1) * (MD_MAXTYPES + 1)];
-  __shared__ float cns_lo[(MD_MAXTYPES + 1) * (MD_MAXTYPES + 1)];
-  __shared__ float cns_hi[(MD_MAXTYPES + 1) * (MD_MAXTYPES + 1)];
+  const int rep = BATCH ? A.reps.tile_rep[blockIdx.x] : 0;
+  const int tile = BATCH ? blockIdx.x - A.reps.tile_base[rep] : blockIdx.x;
+  const BoxGeom &box = BATCH ? A.reps.box[rep] : A.box;
+  const int *__restrict__ cell_start = BATCH ? A.cell_start + A.reps.cell_base[rep] : A.cell_start;
+  const double4 *__restrict__ x4 = A.x4;
+  extern __shared__ uint4 s_rec[];
+  __shared__ int s_start[NST + 1];
+  __shared__ int s_src[NST];               // first atom of the staged cell
+  __shared__ signed char s_img[NST][4];    // periodic image of the staged cell
+  __shared__ int s_chunk[TC][max_chunks(TC)];  // first slot | row << 16 | candidates << 20
+  __shared__ int s_nchunk[TC];
+  __shared__ unsigned short s_count[kMaxCols];  // neighbors of each owned atom
+  __shared__ double cns[SINGLE ? 1 : (MD_MAXTYPES + 1) * (MD_MAXTYPES + 1)];
+  __shared__ __half s_delta[SINGLE ? 1 : MD_MAXTYPES * MD_MAXTYPES];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ncx = box.ncell[0], ncy = box.ncell[1], ncz = box.ncell[2];
-  const int tiles_x = (ncx + kTileCells - 1) / kTileCells;
+  const int tiles_x = (ncx + TC - 1) / TC;
   const int bx = tile % tiles_x;
   const int cy = (tile / tiles_x) % ncy;
   const int cz = tile / (tiles_x * ncy);
-  const int cx0 = bx * kTileCells;
-  const int ow = min(kTileCells, ncx - cx0);  // owned cells in this tile
-  for (int k = threadIdx.x; k < ntp1 * ntp1; k += blockDim.x) {
-    const double c = cutneighsq_g[k];
-    cns[k] = c;
-    cns_lo[k] = (float)(c * (1.0 - 1.0e-5));
-    cns_hi[k] = (float)(c * (1.0 + 1.0e-5));
+  const int cx0 = bx * TC;
+  const int ow = min(TC, ncx - cx0);  // owned cells in this tile
+  if (!SINGLE) {
+    const int nt = A.ntp1 - 1;
+    for (int k = tid; k < A.ntp1 * A.ntp1; k += kNeighThreads) cns[k] = A.cutneighsq[k];
+    for (int k = tid; k < MD_MAXTYPES * MD_MAXTYPES; k += kNeighThreads) {
+      const int a = k / MD_MAXTYPES, b = k % MD_MAXTYPES;
+      float d = 0.f;
+      if (a < nt && b < nt)
+        d = A.cmax - (float)(A.cutneighsq[(a + 1) * A.ntp1 + b + 1] * A.scale * A.scale);
+      s_delta[k] = __float2half_rn(d);
+    }
   }
-  // staged cells: id = sx + (kTileCells+2)*(sy + 3*sz) is global cell
-  // (cx0-1+sx, cy-1+sy, cz-1+sz), wrapped, with the shift of its image
-  if (threadIdx.x < kStageCells) {
-    const int id = threadIdx.x;
-    const int sx = id % (kTileCells + 2), sy = (id / (kTileCells + 2)) % 3,
-              sz = id / (3 * (kTileCells + 2));
-    int g = 0, ix = 0, iy = 0, iz = 0, cnt = 0;
+  // staged cells: id = sx + NSX*(sy + 3*sz) is global cell
+  // (cx0-1+sx, cy-1+sy, cz-1+sz), wrapped
+  if (tid < NST) {
+    const int id = tid;
+    const int sx = id % NSX, sy = (id / NSX) % 3, sz = id / (3 * NSX);
+    int s0 = 0, ix = 0, iy = 0, iz = 0, cnt = 0;
     if (sx <= ow + 1) {  // columns past the box edge are not neighbours of any owned cell
       int gx = cx0 - 1 + sx, gy = cy - 1 + sy, gz = cz - 1 + sz;
       if (gx < 0) { gx += ncx; ix = -1; } else if (gx >= ncx) { gx -= ncx; ix = 1; }
       if (gy < 0) { gy += ncy; iy = -1; } else if (gy >= ncy) { gy -= ncy; iy = 1; }
       if (gz < 0) { gz += ncz; iz = -1; } else if (gz >= ncz) { gz -= ncz; iz = 1; }
-      g = gx + ncx * (gy + ncy * gz);
-      cnt = cell_start[g + 1] - cell_start[g];
+      const int g = gx + ncx * (gy + ncy * gz);
+      s0 = cell_start[g];
+      cnt = cell_start[g + 1] - s0;
     }
-    s_src[id] = g;
-    s_sh[id][0] = ix * box.prd[0];
-    s_sh[id][1] = iy * box.prd[1];
-    s_sh[id][2] = iz * box.prd[2];
+    s_src[id] = s0;
+    s_img[id][0] = (signed char)ix;
+    s_img[id][1] = (signed char)iy;
+    s_img[id][2] = (signed char)iz;
     s_start[id + 1] = cnt;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    s_start[0] = 0;
-    for (int id = 0; id < kStageCells; id++) s_start[id + 1] += s_start[id];
+  if (warp == 0) {  // prefix sum of the counts, two per lane
+    const int i0 = 2 * lane, i1 = 2 * lane + 1;
+    const int c0 = i0 < NST ? s_start[i0 + 1] : 0, c1 = i1 < NST ? s_start[i1 + 1] : 0;
+    int incl = c0 + c1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (i0 < NST) s_start[i0 + 1] = incl - c1;
+    if (i1 < NST) s_start[i1 + 1] = incl;
+    if (lane == 0) s_start[0] = 0;
   }
   __syncthreads();
+  // chunk table: the nine candidate rows (three cells along x) of each owned
+  // cell in chunks of 32
+  if (tid < 9 * TC) {
+    const int c = tid / 9, r = tid % 9;
+    int off = 0;
+    if (c < ow) {
+      for (int q = 0; q < r; q++)
+        off += (s_start[c + 3 + NSX * q] - s_start[c + NSX * q] + 31) >> 5;
+      const int r0 = s_start[c + NSX * r], r1 = s_start[c + 3 + NSX * r];
+      for (int b = r0; b < r1; b += 32, off++)
+        if (off < max_chunks(TC))
+          s_chunk[c][off] = (b & 0xffff) | (r << 16) | (min(32, r1 - b) << 20);
+    }
+    if (r == 8) s_nchunk[c] = off;
+  }
+  __syncthreads();
+  const int nstage = s_start[NST];
+  // owned atoms: contiguous; acceptance columns padded to eight per cell
+  const int own0 = 1 + NSX * 4;  // staged id of the first owned cell
+  int maxw = 0, cols = 0;
+#pragma unroll
+  for (int c = 0; c < TC; c++) {
+    maxw = max(maxw, s_nchunk[c]);
+    if (c < ow) cols += (s_start[own0 + c + 1] - s_start[own0 + c] + 7) & ~7;
+  }
+  const int need = tile_units(nstage, maxw, cols, SINGLE);
   // pass 0: every tile (staged, or the global-memory path when it does not
-  // fit); pass 1: the tiles that fit stage_cap; pass 2: only the tiles that
-  // pass 1 left (more than cap1 atoms), with a larger stage_cap
-  const int nstage = s_start[kStageCells];
-  if ((pass == 1 && nstage > stage_cap) || (pass == 2 && nstage <= cap1)) return;
-  const bool staged = nstage <= stage_cap;
-  if (threadIdx.x == 0) atomicMax(&status[ST_MAXSTAGE], nstage);
-  // FP32 reference point: centre of cell (cx0, cy, cz)
-  const double rx = box.lo[0] + (cx0 + 0.5) * box.cs[0];
-  const double ry = box.lo[1] + (cy + 0.5) * box.cs[1];
-  const double rz = box.lo[2] + (cz + 0.5) * box.cs[2];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // fit); pass 1: the tiles that fit `units`; pass 2: only the tiles that
+  // pass 1 left (more than units1), with more shared memory
+  if ((A.pass == 1 && need > A.units) || (A.pass == 2 && need <= A.units1)) return;
+  if (tid == 0) atomicMax(&A.status[ST_MAXSTAGE], need);
+  // rb: extent of the owned atoms from the tile centre; a candidate near the
+  // cutoff of one lies within ra
+  const float fscale = (float)A.scale;
+  const float ux = 0.5f * (float)ow * (float)box.cs[0] * fscale;
+  const float uy = 0.5f * (float)box.cs[1] * fscale, uz = 0.5f * (float)box.cs[2] * fscale;
+  const float rb = sqrtf(ux * ux + uy * uy + uz * uz), ra = rb + sqrtf(A.cmax);
+  const float eps = ((ra + rb) * (ra + rb) + 2.0f * ra * ra) * (1.25f / 524288.0f) +
+                    (SINGLE ? 0.f : A.dmax * (1.0f / 2048.0f));
+  // cells far wider than the cutoff would overflow FP16 or put every pair
+  // inside the band
+  const bool staged = need <= A.units && maxw <= max_chunks(TC) && nstage < 65504 &&
+                      cols <= kMaxCols && ra < 32.f;
+  const int a0 = s_src[own0];
+  const int nown = s_start[own0 + ow] - s_start[own0];
+
   if (staged) {
-    for (int id = warp; id < kStageCells; id += kNeighThreads / 32) {
-      const int g0 = cell_start[s_src[id]];
-      const int cnt = s_start[id + 1] - s_start[id];
-      const double shx = s_sh[id][0], shy = s_sh[id][1], shz = s_sh[id][2];
-      for (int t = lane; t < cnt; t += 32) {
+    unsigned *recw = reinterpret_cast<unsigned *>(s_rec);
+    int *word = reinterpret_cast<int *>(s_rec + nstage + 32);
+    unsigned char *type = reinterpret_cast<unsigned char *>(s_rec + nstage + 32 +
+                                                            (nstage + 32 + 3) / 4);
+    unsigned char *mask = SINGLE ? type : type + ((nstage + 32 + 15) & ~15);
+    // first slots of the words that the order phase keeps
+    unsigned short *slot = reinterpret_cast<unsigned short *>(mask + ((maxw * cols + 3) & ~3) * 4);
+    const double rx = box.lo[0] + (cx0 + 0.5 * ow) * box.cs[0];
+    const double ry = box.lo[1] + (cy + 0.5) * box.cs[1];
+    const double rz = box.lo[2] + (cz + 0.5) * box.cs[2];
+    // stage: a group of eight lanes per cell
+    for (int id = tid >> 3; id < NST; id += kNeighThreads / 8) {
+      const int o0 = s_start[id], cnt = s_start[id + 1] - o0, g0 = s_src[id];
+      const int code = row_code(id / NSX) + id % NSX;
+      const double shx = (s_img[id][0] * box.prd[0] - rx) * A.scale,
+                   shy = (s_img[id][1] * box.prd[1] - ry) * A.scale,
+                   shz = (s_img[id][2] * box.prd[2] - rz) * A.scale;
+      for (int t = tid & 7; t < cnt; t += 8) {
         const double4 p = x4[g0 + t];
-        const int o = s_start[id] + t;
-        sp[o] = make_float4((float)(__dadd_rn(p.x, shx) - rx), (float)(__dadd_rn(p.y, shy) - ry),
-                            (float)(__dadd_rn(p.z, shz) - rz),
-                            __int_as_float(stage_word(g0 + t, (int)p.w, id % (kTileCells + 2))));
+        const float x = (float)fma(p.x, A.scale, shx), y = (float)fma(p.y, A.scale, shy),
+                    z = (float)fma(p.z, A.scale, shz);
+        s_rec[o0 + t] = record(x, y, z, 0.f);
+        word[o0 + t] = (int)((unsigned)(g0 + t) << 6) + code;
+        if (!SINGLE) type[o0 + t] = (unsigned char)((int)p.w - 1);
       }
     }
-  }
-  // the spare slots after the last staged row: far away, type 1
-  if (staged && threadIdx.x < 32)
-    sp[s_start[kStageCells] + threadIdx.x] =
-        make_float4(1.0e30f, 1.0e30f, 1.0e30f, __int_as_float(stage_word(0, 1, 0)));
-  __syncthreads();
-  // Warp w owns cell (cx0 + w, cy, cz); each lane takes one of its atoms.
-  // The 27 neighbour cells are 9 contiguous staged ranges (3 cells along x
-  // each), scanned 32 candidates at a time.  Test phase: each lane holds one
-  // candidate and the warp steps through the owned atoms (broadcast shared
-  // reads); one ballot per owned atom gives that atom's 32-bit acceptance
-  // mask, which the atom's own lane keeps.  Append phase: each lane walks the
-  // set bits of its mask in candidate order.
-  if (warp >= ow) return;
-  const int own_id = (warp + 1) + (kTileCells + 2) * (1 + 3 * 1);
-  const int cown = cx0 + warp + ncx * (cy + ncy * cz);
-  const int a0 = cell_start[cown], a1 = cell_start[cown + 1];
-  const float lo1 = SINGLE ? cns_lo[ntp1 + 1] : 0.f, hi1 = SINGLE ? cns_hi[ntp1 + 1] : 0.f;
-  const double cut1 = SINGLE ? cns[ntp1 + 1] : 0.0;
-  if (staged) {
-    const int o0 = s_start[own_id];
-    for (int base = a0; base < a1; base += 32) {
-      const int i = base + lane;
-      const bool act = i < a1;
-      // the FP64 position is read again only for a pair in the FP32 band
-      const int ti = SINGLE ? 1 : (int)x4[act ? i : a0].w;
-      const int my_m = act ? o0 + (i - a0) : -1;
-      // the owned atoms of this batch, staged as sp[ob .. ob + na) with the
-      // same FP32 offsets from the tile centre as every candidate
-      const int ob = o0 + (base - a0), na = min(32, a1 - base);
-      int count = 0;
-      int4 buf = make_int4(0, 0, 0, 0);
-      for (int dz = -1; dz <= 1; dz++)
-        for (int dy = -1; dy <= 1; dy++) {
-          const int idL = warp + (kTileCells + 2) * ((1 + dy) + 3 * (1 + dz));  // dx = -1
-          const int r0 = s_start[idL], r1 = s_start[idL + 3];
-          // entry code of a candidate in staged column sx: dx + 1 = sx - warp
-          const unsigned rowadd = (unsigned)(((dy + 1) << 2) + ((dz + 1) << 4) - warp);
-          for (int cb = r0; cb < r1; cb += 32) {
-            const int nc = min(32, r1 - cb);
-            // this lane's candidate (the spare slots past the last row are
-            // far away, and candidates past the row end are masked below)
-            const float4 pc = sp[cb + lane];
-            const int tc = stage_type(pc.w);
-            unsigned acc = 0u, band = 0u;
-            for (int a = 0; a < na; a++) {
-              const float4 q = sp[ob + a];
-              const float ddx = q.x - pc.x, ddy = q.y - pc.y, ddz = q.z - pc.z;
-              const float r2 = ddx * ddx + ddy * ddy + ddz * ddz;
-              float lo = lo1, hi = hi1;
+    // the spare slots after the last staged row: far away, type 1
+    if (tid < 32) {
+      s_rec[nstage + tid] = record(64.f, 64.f, 64.f, 0.f);
+      word[nstage + tid] = 0;
+      if (!SINGLE) type[nstage + tid] = 0;
+    }
+    __syncthreads();
+    // test: warps WPC*c .. WPC*c + WPC-1 take owned cell c, chunk by chunk
+    const int c = warp / WPC, sub = warp % WPC;
+    const int g = lane >> 2, t = lane & 3;
+    if (c < ow) {
+      const int o0 = s_start[own0 + c], cnt = s_start[own0 + c + 1] - o0;
+      const int nch = s_nchunk[c];
+      int colb = 0;
+#pragma unroll
+      for (int q = 0; q < TC; q++)
+        if (q < c) colb += (s_start[own0 + q + 1] - s_start[own0 + q] + 7) & ~7;
+      for (int ab = 0; ab < cnt; ab += 32) {
+        const int na = min(32, cnt - ab), nt = (na + 7) >> 3;
+        // owned atoms as the B operand: -2 b in both halves of each dimension
+        unsigned b0[4], b1[4], bt[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const int ia = o0 + ab + min(8 * q + g, na - 1);
+          const unsigned w = recw[ia * 4 + t];
+          const __half2 m2 = __floats2half2_rn(-2.f, -2.f);
+          const __half2 h2 = __half2half2(__ushort_as_half((unsigned short)w));
+          const __half2 l2 = __half2half2(__ushort_as_half((unsigned short)(w >> 16)));
+          const __half2 ph = __hmul2(h2, m2), pl = __hmul2(l2, m2);
+          b0[q] = *reinterpret_cast<const unsigned *>(&ph);
+          b1[q] = *reinterpret_cast<const unsigned *>(&pl);
+          if (t == 3) {  // candidate norm x 1; 1 x (norm - cutoff)
+            const float v = join16(w) - A.cmax;
+            const __half vh = __float2half_rn(v);
+            const __half2 v2 = __halves2half2(vh, __float2half_rn(v - __half2float(vh)));
+            b0[q] = 0x3C003C00u;
+            b1[q] = *reinterpret_cast<const unsigned *>(&v2);
+          }
+          bt[q] = 0;
+          if (!SINGLE)
+            bt[q] = *reinterpret_cast<const unsigned *>(
+                &s_delta[type[ia] * MD_MAXTYPES + 2 * t]);
+        }
+        for (int w = sub; w < nch; w += WPC) {
+          const int info = s_chunk[c][w];
+          const int cb = info & 0xffff;
+          const unsigned *ap = recw + (cb + g) * 4 + t;
+          const unsigned a00 = ap[0], a01 = ap[32], a10 = ap[64], a11 = ap[96];
+          // the second half of K: the same coordinates against the lo halves;
+          // ones against the owned side's norm
+          const unsigned one = 0x3C003C00u;
+          const unsigned a02 = t == 3 ? one : a00, a03 = t == 3 ? one : a01,
+                         a12 = t == 3 ? one : a10, a13 = t == 3 ? one : a11;
+          unsigned y00 = 0, y01 = 0, y10 = 0, y11 = 0;  // one-hot types
+          if (!SINGLE) {
+            auto hot = [&](int s) {
+              const int ty = type[s];
+              return (ty >> 1) == t ? ((ty & 1) ? 0x3C000000u : 0x00003C00u) : 0u;
+            };
+            y00 = hot(cb + g), y01 = hot(cb + g + 8), y10 = hot(cb + g + 16),
+            y11 = hot(cb + g + 24);
+          }
+          unsigned char *mw = mask + (w * cols + colb + ab) * 4 + t * 8 + g;
+          float near = 1.0e30f;
+          float d[4], e[4];
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            if (q < nt) {
+              mma16(d, a00, a01, a02, a03, b0[q], b1[q]);
+              mma16(e, a10, a11, a12, a13, b0[q], b1[q]);
               if (!SINGLE) {
-                const int tt = stage_type(q.w) * ntp1 + tc;
-                lo = cns_lo[tt];
-                hi = cns_hi[tt];
+                mma8(d, y00, y01, bt[q]);
+                mma8(e, y10, y11, bt[q]);
               }
-              const bool in = r2 <= hi;
-              const unsigned m = __ballot_sync(0xffffffffu, in);
-              const unsigned b = __ballot_sync(0xffffffffu, in && r2 >= lo);
-              if (lane == a) {
-                acc = m;
-                band = b;
-              }
+              near = least(near, d, e);
+              mw[q * 32] = (unsigned char)sign_byte(d, e);
             }
-            // candidates past the row end are not neighbours
-            acc &= nc == 32 ? 0xffffffffu : ((1u << nc) - 1u);
-            if (my_m >= cb && my_m < cb + nc) acc &= ~(1u << (my_m - cb));
-            band &= acc;
-            if (band == 0u) {
-              while (acc) {
-                const int t = __ffs(acc) - 1;
-                acc &= acc - 1u;
-                append_entry(nlist, stride, i, count, capacity,
-                             (int)(stage_entry(sp[cb + t].w) + rowadd), buf);
+          }
+          if (__any_sync(0xffffffffu, near <= eps)) {
+            // some pair lies in the band: the reference's FP64 test for those
+            const int row = (info >> 16) & 15, nc = info >> 20;
+#pragma unroll 1
+            for (int q = 0; q < nt; q++) {
+              // (b0[q] etc. by selects: the loop is rolled)
+              const unsigned p0 = q == 0 ? b0[0] : q == 1 ? b0[1] : q == 2 ? b0[2] : b0[3];
+              const unsigned p1 = q == 0 ? b1[0] : q == 1 ? b1[1] : q == 2 ? b1[2] : b1[3];
+              mma16(d, a00, a01, a02, a03, p0, p1);
+              mma16(e, a10, a11, a12, a13, p0, p1);
+              if (!SINGLE) {
+                const unsigned pt = q == 0 ? bt[0] : q == 1 ? bt[1] : q == 2 ? bt[2] : bt[3];
+                mma8(d, y00, y01, pt);
+                mma8(e, y10, y11, pt);
               }
-            } else {
-              while (acc) {
-                const int t = __ffs(acc) - 1;
-                acc &= acc - 1u;
-                const int m = cb + t;
-                const unsigned bits = stage_entry(sp[m].w);
-                // inside the FP32 uncertainty band: the reference's FP64 test
-                if ((band >> t) & 1u) {
-                  const int id = idL - warp + (int)(bits & 7u);
-                  if (!exact_pair(x4[i], x4[md_entry_j(bits)], s_sh[id][0], s_sh[id][1], s_sh[id][2],
-                                  SINGLE ? cut1 : cns[ti * ntp1 + stage_type(sp[m].w)]))
-                    continue;
-                }
-                append_entry(nlist, stride, i, count, capacity, (int)(bits + rowadd), buf);
+              unsigned r = sign_byte(d, e), band = 0;
+              const float val[8] = {d[0], d[2], e[0], e[2], d[1], d[3], e[1], e[3]};
+#pragma unroll
+              for (int k = 0; k < 8; k++) band |= fabsf(val[k]) <= eps ? 1u << k : 0u;
+              while (band) {
+                const int k = __ffs(band) - 1;
+                band &= band - 1u;
+                const int ci = g + 8 * (k & 3), ai = 8 * q + 2 * t + (k >> 2);
+                if (ci >= nc || ai >= na) continue;
+                const int cw = word[cb + ci];
+                const int id = (cw & 63) - row_code(row) + NSX * row;
+                const int i = a0 + (o0 - s_start[own0]) + ab + ai;
+                const double cut =
+                    SINGLE ? A.cutneighsq[A.ntp1 + 1]
+                           : cns[(type[o0 + ab + ai] + 1) * A.ntp1 + type[cb + ci] + 1];
+                const bool in = exact_pair(x4[i], x4[(unsigned)cw >> 6], s_img[id][0] * box.prd[0],
+                                           s_img[id][1] * box.prd[1], s_img[id][2] * box.prd[2],
+                                           cut);
+                r = in ? r | (1u << k) : r & ~(1u << k);
               }
+              mw[q * 32] = (unsigned char)r;
             }
           }
         }
-      if (act) {
-        flush_entries(nlist, stride, i, count, capacity, buf);
-        // the stored count never exceeds the capacity, so readers stay in
-        // bounds; an overflow is reported through the status word
-        numneigh[i] = count < capacity ? count : capacity;
       }
-      // one status update per warp
-      const int cmax = __reduce_max_sync(0xffffffffu, act ? count : 0);
-      if (lane == 0) {
-        atomicMax(&status[ST_MAXNEIGH], cmax);
-        if (cmax > capacity) atomicExch(&status[ST_OVERFLOW], 1);
+    }
+    __syncthreads();
+    // order: groups of eight owned atoms of a cell, lane = (atom, one of four
+    // chunks); candidates past the row end and the atom itself are cleared,
+    // empty words dropped.  Candidate k is bit 31 - k: the next candidate is
+    // then the leading one.
+    {
+      const int a = lane & 7, ws = lane >> 3;
+      int grp = 0, colb = 0;
+      for (int ca = 0; ca < ow; ca++) {
+        const int o0 = s_start[own0 + ca], cnt = s_start[own0 + ca + 1] - o0;
+        const int nch = s_nchunk[ca];
+        for (int ab = 0; ab < cnt; ab += 8, colb += 8, grp++) {
+          if (grp % (kNeighThreads / 32) != warp) continue;
+          unsigned *mp = reinterpret_cast<unsigned *>(mask) + colb + a;
+          unsigned short *sp = slot + colb + a;
+          const int self = o0 + ab + a, sh = 4 * (a & 1);
+          const bool act = ab + a < cnt;
+          int tot = 0, kept = 0;  // kept: cols x the words kept so far
+          const unsigned below = 0x01010101u & ((1u << (8 * ws)) - 1u);
+          const uint2 *rp = reinterpret_cast<const uint2 *>(mp - (a & 1) + ws * cols);
+          for (int w = ws; w < nch + ws; w += 4, rp += 2 * cols) {
+            unsigned x = 0;
+            int info = 0;
+            if (w < nch) {
+              info = s_chunk[ca][w];
+              const uint2 raw = *rp;
+              x = __brev(candidate_order(((raw.x >> sh) & 0x0F0F0F0Fu) |
+                                         (((raw.y >> sh) << 4) & 0xF0F0F0F0u)));
+              x &= 0xffffffffu << (32 - (info >> 20));
+              const unsigned me = (unsigned)(self - (info & 0xffff));
+              if (me < 32u && (info & 0xF0000) == 0x40000) x &= ~(0x80000000u >> me);
+              if (!act) x = 0;
+            }
+            // words kept of this atom in this round: bits 0, 8, 16, 24
+            const unsigned full = (__ballot_sync(0xffffffffu, x != 0u) >> a) & 0x01010101u;
+            if (x) {
+              const int k = kept + cols * __popc(full & below);
+              mp[k] = x;
+              sp[k] = (unsigned short)info;
+            }
+            kept += cols * __popc(full);
+            tot += __popc(x);
+            __syncwarp();
+          }
+          tot += __shfl_xor_sync(0xffffffffu, tot, 8);
+          tot += __shfl_xor_sync(0xffffffffu, tot, 16);
+          if (ws == 0) s_count[colb + a] = (unsigned short)tot;
+          const int most = __reduce_max_sync(0xffffffffu, tot);
+          if (lane == 0) {
+            atomicMax(&A.status[ST_MAXNEIGH], most);
+            if (most > A.capacity) atomicExch(&A.status[ST_OVERFLOW], 1);
+          }
+        }
+      }
+    }
+    __syncthreads();
+    // append
+    for (int la = tid; la < nown; la += kNeighThreads) {
+      const int i = a0 + la;
+      int ca = 0, col = la;
+#pragma unroll
+      for (int q = 0; q < TC - 1; q++)
+        if (q + 1 < ow && la >= s_start[own0 + q + 1] - s_start[own0]) {
+          ca = q + 1;
+          // padding of the cells before this one
+          const int cq = s_start[own0 + q + 1] - s_start[own0 + q];
+          col += ((cq + 7) & ~7) - cq;
+        }
+      const int tot = s_count[col];
+      // the stored count never exceeds the capacity, so readers stay in
+      // bounds; an overflow is reported through the status word
+      const int num = min(tot, A.capacity);
+      A.numneigh[i] = num;
+      const unsigned *mp = reinterpret_cast<const unsigned *>(mask) + col;
+      const unsigned short *sp = slot + col;
+      unsigned x = 0;
+      const int *cw = word;
+      auto next = [&]() -> int {
+        if (x == 0u) {
+          x = *mp;
+          cw = word + *sp + 31;
+          mp += cols;
+          sp += cols;
+        }
+        const int b = 31 - __clz(x);
+        x ^= 1u << b;
+        return cw[-b] - ca;
+      };
+      int4 *out = reinterpret_cast<int4 *>(A.nlist) + i;
+      for (int s = num >> 2; s > 0; s--, out += A.stride) {
+        int4 e;
+        e.x = next();
+        e.y = next();
+        e.z = next();
+        e.w = next();
+        *out = e;
+      }
+      if (num & 3) {
+        // the last, partly filled slab ends in pad entries
+        const int pad = md_pad_entry(i);
+        int4 e = make_int4(pad, pad, pad, pad);
+        e.x = next();
+        if ((num & 3) > 1) e.y = next();
+        if ((num & 3) > 2) e.z = next();
+        *out = e;
       }
     }
     return;
   }
-  // fallback (a tile or a cell too crowded for shared memory): one thread
-  // per owned atom, candidates read from global memory, FP64 test
-  for (int i = a0 + lane; i < a1; i += 32) {
+  // fallback (a tile too crowded for shared memory, or cells far wider than
+  // the cutoff): one thread per owned atom, candidates read from global
+  // memory, FP64 test
+  for (int la = tid; la < nown; la += kNeighThreads) {
+    const int i = a0 + la;
+    int ca = 0;
+#pragma unroll
+    for (int q = 0; q < TC - 1; q++)
+      if (q + 1 < ow && la >= s_start[own0 + q + 1] - s_start[own0]) ca = q + 1;
     const double4 xi = x4[i];
     const int ti = (int)xi.w;
+    const int pad = md_pad_entry(i);
     int count = 0;
-    int4 buf = make_int4(0, 0, 0, 0);
-    for (int dz = -1; dz <= 1; dz++)
-      for (int dy = -1; dy <= 1; dy++)
-        for (int dx = -1; dx <= 1; dx++) {
-          const int id = (warp + 1 + dx) + (kTileCells + 2) * ((1 + dy) + 3 * (1 + dz));
-          const int code = md_code(dx, dy, dz);
-          const int g = s_src[id];
-          const int j1 = cell_start[g + 1];
-          for (int j = cell_start[g]; j < j1; j++) {
-            if (code == MD_CODE_SELF && j == i) continue;
-            const double4 xj = x4[j];
-            if (exact_pair(xi, xj, s_sh[id][0], s_sh[id][1], s_sh[id][2],
-                           cns[ti * ntp1 + (int)xj.w]))
-              append_entry(nlist, stride, i, count, capacity, md_make_entry(j, code), buf);
-          }
+    int4 buf = make_int4(pad, pad, pad, pad);
+    int4 *out = reinterpret_cast<int4 *>(A.nlist) + i;
+    const int slabs = A.capacity >> 2;
+    for (int r = 0; r < 9; r++)
+      for (int dx = 0; dx < 3; dx++) {
+        const int id = ca + dx + NSX * r;
+        const int code = dx + row_code(r);
+        const double shx = s_img[id][0] * box.prd[0], shy = s_img[id][1] * box.prd[1],
+                     shz = s_img[id][2] * box.prd[2];
+        const int j0 = s_src[id], j1 = j0 + s_start[id + 1] - s_start[id];
+        for (int j = j0; j < j1; j++) {
+          if (code == MD_CODE_SELF && j == i) continue;
+          const double4 xj = x4[j];
+          const double cut = SINGLE ? A.cutneighsq[A.ntp1 + 1] : cns[ti * A.ntp1 + (int)xj.w];
+          if (!exact_pair(xi, xj, shx, shy, shz, cut)) continue;
+          const int e = md_make_entry(j, code), k = count & 3;
+          if (k == 0) buf = make_int4(e, pad, pad, pad);
+          else if (k == 1) buf.y = e;
+          else if (k == 2) buf.z = e;
+          else buf.w = e;
+          count++;
+          if (k == 3 && (count >> 2) <= slabs) out[(size_t)((count >> 2) - 1) * A.stride] = buf;
         }
-    flush_entries(nlist, stride, i, count, capacity, buf);
-    numneigh[i] = count < capacity ? count : capacity;
-    atomicMax(&status[ST_MAXNEIGH], count);
-    if (count > capacity) atomicExch(&status[ST_OVERFLOW], 1);
+      }
+    if ((count & 3) && (count >> 2) < slabs) out[(size_t)(count >> 2) * A.stride] = buf;
+    A.numneigh[i] = count < A.capacity ? count : A.capacity;
+    atomicMax(&A.status[ST_MAXNEIGH], count);
+    if (count > A.capacity) atomicExch(&A.status[ST_OVERFLOW], 1);
   }
 }
 
@@ -634,27 +923,26 @@ __global__ void k_prefix_ll(int n, const int *__restrict__ cnt, long long *__res
 
 }  // namespace
 
-// Staging capacity of a builder tile: 1.25 x the atoms of kStageCells cells
-// at the densest replica's mean count per cell, or the most any tile staged
-// in an earlier build if that is larger, rounded up to 128 and at most
-// kStageCapMax.  A tile that stages more atoms takes the global-memory path
-// (same list, slower); a smaller capacity leaves room for more resident
-// CTAs per SM.
-static int round_cap(int cap) {
-  cap = (cap + 127) & ~127;
-  if (cap < 256) cap = 256;
-  return cap < kStageCapMax ? cap : kStageCapMax;
+// Cells along x per builder tile.  A tile of two stages 18 cells per owned
+// cell instead of 27, but gives half the CTAs: a 4,000,000-atom run of 60 steps
+// takes 41.1 ms with two and 43.2 with one (four: 41.5), 1,728 cells of copper
+// 3.86 against 3.96, 27 cells 1.35 against 1.32.  Replica boxes are a few
+// cells wide, so half of their two-cell tiles would own one cell (11.78
+// against 11.66 ms).
+int md_tile_cells(const b200_ctx *c) {
+  return !c->nrep && c->ncells >= 148 * 7 ? 2 : 1;
 }
 
-// Staging capacity of the builder tiles: 1.25 x the mean atom count of the 54
-// staged cells, raised when a build reports a more crowded tile.  For a batch
-// the mean is the batch's (the common case, at full occupancy); the densest
-// replicas' tiles are rebuilt in a second pass with md_stage_cap2.
+// Shared memory of the builder tiles, in 16-byte units: what a tile of the
+// mean density takes, with some room, raised when a build reports a larger
+// tile.  For a batch the mean is the batch's (the common case, at full
+// occupancy); the densest replicas' tiles are built in a second pass with
+// md_stage_cap2.
 int md_stage_cap(const b200_ctx *c) {
   const double per_cell = c->ncells > 0 ? (double)c->n / c->ncells : 0.0;
-  int cap = (int)(1.25 * kStageCells * per_cell) + 64;
+  int cap = tile_units_of(per_cell, c->tile_cells, c->ntypes == 1);
   if (!c->nrep && c->stage_need > cap) cap = c->stage_need;
-  return round_cap(cap);
+  return std::min((cap + 31) & ~31, kStageUnitsMax);
 }
 
 // second-pass capacity of a batch: the densest replica's tiles (0 when the
@@ -667,23 +955,24 @@ int md_stage_cap2(const b200_ctx *c) {
     const double d = (double)c->rep_natoms[r] / ((double)b.ncell[0] * b.ncell[1] * b.ncell[2]);
     per_cell = d > per_cell ? d : per_cell;
   }
-  int cap = (int)(1.25 * kStageCells * per_cell) + 64;
+  int cap = tile_units_of(per_cell, c->tile_cells, c->ntypes == 1);
   if (c->stage_need > cap) cap = c->stage_need;
-  cap = round_cap(cap);
+  cap = std::min((cap + 31) & ~31, kStageUnitsMax);
   return cap > md_stage_cap(c) ? cap : 0;
 }
 
-// After a build: raise the staging capacity when some tile staged more atoms
-// than the current one holds.  Returns true when the capacity changed (the
-// caller re-captures its graphs).
+// After a build: raise the capacity when some tile needed more than the
+// current one holds.  Returns true when the capacity changed (the caller
+// re-captures its graphs).
 bool md_stage_feedback(b200_ctx *c, int staged_max) {
-  const int cap = c->nrep ? (md_stage_cap2(c) > 0 ? md_stage_cap2(c) : md_stage_cap(c))
-                          : md_stage_cap(c);
-  if (staged_max <= cap || cap >= kStageCapMax) return false;
+  auto cap_now = [&] {
+    const int cap2 = md_stage_cap2(c);
+    return cap2 > 0 ? cap2 : md_stage_cap(c);
+  };
+  const int cap = cap_now();
+  if (staged_max <= cap || cap >= kStageUnitsMax) return false;
   c->stage_need = staged_max + staged_max / 10;
-  const int now = c->nrep ? (md_stage_cap2(c) > 0 ? md_stage_cap2(c) : md_stage_cap(c))
-                          : md_stage_cap(c);
-  return now != cap;
+  return cap_now() != cap;
 }
 
 static cudaError_t launch_scan(b200_ctx *c, int m, const int *in, int *out, const int *flag) {
@@ -698,6 +987,83 @@ static cudaError_t launch_scan(b200_ctx *c, int m, const int *in, int *out, cons
     c->launches += 2;
   }
   return cudaGetLastError();
+}
+
+template <int TC>
+static cudaError_t launch_tiles(b200_ctx *c, const NeighArgs &A, int tiles, cudaStream_t st) {
+  // the shared-memory opt-in, once per device this process uses
+  static std::atomic<unsigned long long> opt_in{0ull};
+  const unsigned long long dev_bit = 1ull << (c->device & 63);
+  if (!(opt_in.load() & dev_bit)) {
+    const int most = kStageUnitsMax * 16;
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_neigh_tiles<TC, true, false>, attr, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_neigh_tiles<TC, true, true>, attr, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_neigh_tiles<TC, false, false>, attr, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_neigh_tiles<TC, false, true>, attr, most);
+    if (e != cudaSuccess) return e;
+    opt_in.fetch_or(dev_bit);
+  }
+  const size_t smem = (size_t)A.units * 16;
+  if (c->ntypes == 1 && !c->nrep)
+    k_neigh_tiles<TC, true, false><<<tiles, kNeighThreads, smem, st>>>(A);
+  else if (c->ntypes == 1)
+    k_neigh_tiles<TC, true, true><<<tiles, kNeighThreads, smem, st>>>(A);
+  else if (!c->nrep)
+    k_neigh_tiles<TC, false, false><<<tiles, kNeighThreads, smem, st>>>(A);
+  else
+    k_neigh_tiles<TC, false, true><<<tiles, kNeighThreads, smem, st>>>(A);
+  c->launches++;
+  return cudaGetLastError();
+}
+
+static cudaError_t launch_list(b200_ctx *c, const int *d_flag) {
+  const int tc = c->tile_cells;
+  const int tiles = c->nrep ? c->ntiles
+                            : ((c->box.ncell[0] + tc - 1) / tc) * c->box.ncell[1] * c->box.ncell[2];
+  NeighArgs A;
+  A.n = c->n;
+  A.stride = c->stride;
+  A.capacity = c->capacity;
+  A.ntp1 = c->ntypes + 1;
+  A.box = c->box;
+  A.reps = c->reps();
+  A.scale = std::exp2(1.0 - std::floor(std::log2(c->cutneighmax)));
+  double cmax = 0.0, cmin = 1.0e300;
+  for (int i = 1; i <= c->ntypes; i++)
+    for (int j = 1; j <= c->ntypes; j++) {
+      cmax = std::max(cmax, c->cutneighsq[i * A.ntp1 + j]);
+      cmin = std::min(cmin, c->cutneighsq[i * A.ntp1 + j]);
+    }
+  A.cmax = (float)(cmax * A.scale * A.scale);
+  A.dmax = (float)((cmax - cmin) * A.scale * A.scale);
+  A.cutneighsq = c->cutneighsq_dev;
+  A.x4 = c->x4;
+  A.cell_start = c->cell_start;
+  A.nlist = c->nlist;
+  A.numneigh = c->numneigh;
+  A.status = c->status;
+  A.flag = d_flag;
+  const int cap = md_stage_cap(c);
+  const int cap2 = md_stage_cap2(c);  // a batch's densest tiles, or 0
+  A.units1 = cap;
+  auto launch = [&](int units, int pass, cudaStream_t st) {
+    A.units = units;
+    A.pass = pass;
+    return tc == 2 ? launch_tiles<2>(c, A, tiles, st) : launch_tiles<1>(c, A, tiles, st);
+  };
+  if (cap2 == 0) return launch(cap, 0, c->stream);
+  // The two passes build disjoint tiles, so the second (the densest tiles,
+  // large staging, few blocks per SM) runs on the side stream beside the
+  // first instead of after it; the join makes the main stream wait for both.
+  // Inside a graph capture the fork and join become graph dependencies.
+  cudaError_t e = cudaEventRecord(c->ev_fork, c->stream);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(c->s_aux, c->ev_fork, 0);
+  if (e == cudaSuccess) e = launch(cap, 1, c->stream);
+  if (e == cudaSuccess) e = launch(cap2, 2, c->s_aux);
+  if (e == cudaSuccess) e = cudaEventRecord(c->ev_join, c->s_aux);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, c->ev_join, 0);
+  return e;
 }
 
 cudaError_t md_rebuild(b200_ctx *c, const int *d_flag) {
@@ -732,61 +1098,8 @@ cudaError_t md_rebuild(b200_ctx *c, const int *d_flag) {
   k_copyback<<<md_blocks(n, B), B, 0, c->stream>>>(n, c->stride, c->x4b, c->x4, c->vb, c->v,
                                                    c->origb, c->orig, c->imageb, c->image,
                                                    c->where, c->status, d_flag);
-  {
-    const int tiles = c->nrep ? c->ntiles
-                              : ((c->box.ncell[0] + kTileCells - 1) / kTileCells) *
-                                    c->box.ncell[1] * c->box.ncell[2];
-    // the shared-memory opt-in, once per device this process uses
-    static unsigned long long smem_opt_in = 0ull;
-    const unsigned long long dev_bit = 1ull << (c->device & 63);
-    if (!(smem_opt_in & dev_bit)) {
-      const int most = (int)neigh_smem(kStageCapMax);
-      cudaFuncSetAttribute(k_neigh_tiles<true, false>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-      cudaFuncSetAttribute(k_neigh_tiles<true, true>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-      cudaFuncSetAttribute(k_neigh_tiles<false, false>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-      cudaFuncSetAttribute(k_neigh_tiles<false, true>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-      smem_opt_in |= dev_bit;
-    }
-    const int cap = md_stage_cap(c);
-    const int cap2 = md_stage_cap2(c);  // a batch's densest tiles, or 0
-    auto launch = [&](int stage_cap, int pass, cudaStream_t st) {
-      const size_t smem = neigh_smem(stage_cap);
-#define MD_NEIGH_ARGS                                                                         \
-  n, c->stride, c->capacity, stage_cap, c->box, R, c->ntypes + 1, c->cutneighsq_dev, c->x4,  \
-      c->cell_start, c->nlist, c->numneigh, c->status, d_flag, pass, cap
-      if (c->ntypes == 1 && !c->nrep)
-        k_neigh_tiles<true, false><<<tiles, kNeighThreads, smem, st>>>(MD_NEIGH_ARGS);
-      else if (c->ntypes == 1)
-        k_neigh_tiles<true, true><<<tiles, kNeighThreads, smem, st>>>(MD_NEIGH_ARGS);
-      else if (!c->nrep)
-        k_neigh_tiles<false, false><<<tiles, kNeighThreads, smem, st>>>(MD_NEIGH_ARGS);
-      else
-        k_neigh_tiles<false, true><<<tiles, kNeighThreads, smem, st>>>(MD_NEIGH_ARGS);
-#undef MD_NEIGH_ARGS
-      c->launches++;
-    };
-    if (cap2 > 0) {
-      // The two passes build disjoint tiles, so the second (the densest
-      // tiles, large staging, few blocks per SM) runs on the side stream
-      // beside the first instead of after it; the join makes the main stream
-      // wait for both.  Inside a graph capture the fork and join become
-      // graph dependencies.
-      cudaError_t e = cudaEventRecord(c->ev_fork, c->stream);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(c->s_aux, c->ev_fork, 0);
-      if (e != cudaSuccess) return e;
-      launch(cap, 1, c->stream);
-      launch(cap2, 2, c->s_aux);
-      e = cudaEventRecord(c->ev_join, c->s_aux);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, c->ev_join, 0);
-      if (e != cudaSuccess) return e;
-    } else {
-      launch(cap, 0, c->stream);
-    }
-  }
+  e = launch_list(c, d_flag);
+  if (e != cudaSuccess) return e;
   c->launches += 3;
   return cudaGetLastError();
 }
