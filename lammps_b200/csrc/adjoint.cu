@@ -33,156 +33,278 @@ struct AdjTables {
   double lj1[kAdjNP], lj2[kAdjNP], cutsq[kAdjNP];  // [(ti-1)*ntypes + (tj-1)]
 };
 
-template <bool MIXED>
-__device__ __forceinline__ void pair_geom(const AdjTables &T, int i, unsigned e,
-                                          const double4 *__restrict__ x4,
-                                          const int4 *__restrict__ xq, const Shift3 &sx,
-                                          const Shift3 &sy, const Shift3 &sz, const float *qh,
-                                          const float *ql, double &dx, double &dy,
-                                          double &dz, double &rsq, int &tt) {
-  const int j = md_entry_j(e);
-  if (MIXED) {
-    // minimum-image separation from the fixed-point coordinates
-    const int4 xi = xq[i], xj = xq[j];
-    const float fx = md_qlen(md_qdiff(xi.x, xj.x), qh[0], ql[0]);
-    const float fy = md_qlen(md_qdiff(xi.y, xj.y), qh[1], ql[1]);
-    const float fz = md_qlen(md_qdiff(xi.z, xj.z), qh[2], ql[2]);
-    dx = fx;
-    dy = fy;
-    dz = fz;
-    rsq = (double)(fx * fx + fy * fy + fz * fz);
-    tt = (xi.w - 1) * T.ntypes + (xj.w - 1);
-  } else {
-    const double4 xi = x4[i], xj = x4[j];
-    int jj, ex, ey, ez;
-    md_entry(e, jj, ex, ey, ez);
-    dx = xi.x - (xj.x + pick(sx, ex));
-    dy = xi.y - (xj.y + pick(sy, ey));
-    dz = xi.z - (xj.z + pick(sz, ez));
-    rsq = dx * dx + dy * dy + dz * dz;
-    tt = ((int)xi.w - 1) * T.ntypes + ((int)xj.w - 1);
+struct AdjArgs {
+  int n, stride;
+  AdjTables T;
+  BoxGeom box;
+  const double4 *x4;
+  const int4 *xq;
+  const int *cell, *nlist, *numneigh, *orig;
+  const double4 *gs;  // backward: G in the sorted order
+  double *out;        // forces, or dL/dx, in the caller's order
+  double *partial, *gtab;
+  unsigned int *counter;
+};
+
+// The type-pair tables in shared memory: a lane looks its pair up by an index
+// of its own, which the parameter (constant) bank would serve one by one.
+struct AdjShared {
+  double lj1[kAdjNP], lj2[kAdjNP], cutsq[kAdjNP];
+  float lj1f[kAdjNP], lj2f[kAdjNP];
+};
+__device__ __forceinline__ void load_tables(AdjShared &S, const AdjTables &T) {
+  if (threadIdx.x < kAdjNP) {
+    const int k = threadIdx.x;
+    S.lj1[k] = T.lj1[k];
+    S.lj2[k] = T.lj2[k];
+    S.cutsq[k] = T.cutsq[k];
+    S.lj1f[k] = (float)T.lj1[k];
+    S.lj2f[k] = (float)T.lj2[k];
   }
+  __syncthreads();
 }
 
-// forces in the caller's order: f[3*orig[i] + k]
+// Atom i's side of its pairs: position, type row and periodic shifts (FP64),
+// or fixed-point position and unit lengths (mixed).
 template <bool MIXED>
-__global__ void __launch_bounds__(kAdjThreads)
-    k_adj_forward(int n, int stride, AdjTables T, BoxGeom box, const double4 *__restrict__ x4,
-                  const int4 *__restrict__ xq, const int *__restrict__ cell,
-                  const int *__restrict__ nlist, const int *__restrict__ numneigh,
-                  const int *__restrict__ orig, double *__restrict__ f) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int cx, cy, cz;
-  md_cell_unpack(cell[i], cx, cy, cz);
-  const Shift3 sx = shifts(cx, box.ncell[0], box.prd[0]);
-  const Shift3 sy = shifts(cy, box.ncell[1], box.prd[1]);
-  const Shift3 sz = shifts(cz, box.ncell[2], box.prd[2]);
-  const int num = numneigh[i];
+struct AdjAtom {
+  double4 p;
+  int4 q;
+  int row;  // (ti - 1) * ntypes
+  Shift3 sx, sy, sz;
+  float qh[3], ql[3];
+  __device__ __forceinline__ AdjAtom(const AdjArgs &a, int i) {
+    if (MIXED) {
+      q = a.xq[i];
+      row = (q.w - 1) * a.T.ntypes;
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        qh[d] = a.box.qs[d];
+        ql[d] = a.box.qs_lo[d];
+      }
+    } else {
+      p = a.x4[i];
+      row = ((int)p.w - 1) * a.T.ntypes;
+      int cx, cy, cz;
+      md_cell_unpack(a.cell[i], cx, cy, cz);
+      sx = shifts(cx, a.box.ncell[0], a.box.prd[0]);
+      sy = shifts(cy, a.box.ncell[1], a.box.prd[1]);
+      sz = shifts(cz, a.box.ncell[2], a.box.prd[2]);
+    }
+  }
+  // separation, squared length and neighbour type (0-based) of entry e
+  __device__ __forceinline__ void geom(unsigned e, const double4 &xj, const int4 &qj, double &dx,
+                                       double &dy, double &dz, double &rsq, int &tj) const {
+    if (MIXED) {
+      // minimum-image separation from the fixed-point coordinates
+      const float fx = md_qlen(md_qdiff(q.x, qj.x), qh[0], ql[0]);
+      const float fy = md_qlen(md_qdiff(q.y, qj.y), qh[1], ql[1]);
+      const float fz = md_qlen(md_qdiff(q.z, qj.z), qh[2], ql[2]);
+      dx = fx;
+      dy = fy;
+      dz = fz;
+      rsq = (double)(fx * fx + fy * fy + fz * fz);
+      tj = qj.w - 1;
+    } else {
+      int j, ex, ey, ez;
+      md_entry(e, j, ex, ey, ez);
+      dx = p.x - (xj.x + pick(sx, ex));
+      dy = p.y - (xj.y + pick(sy, ey));
+      dz = p.z - (xj.z + pick(sz, ez));
+      rsq = dx * dx + dy * dy + dz * dz;
+      tj = (int)xj.w - 1;
+    }
+  }
+};
+
+// Forces in the caller's order.  TPA threads per atom take consecutive list
+// entries (walk_list) and issue four gathers at a time.
+template <bool MIXED, int TPA>
+__global__ void __launch_bounds__(kAdjThreads) k_adj_forward(AdjArgs a) {
+  __shared__ AdjShared S;
+  load_tables(S, a.T);
+  const int t = blockIdx.x * kAdjThreads + threadIdx.x;
+  const int i = t / TPA, lane = t % TPA;
+  const bool active = i < a.n;
   double fx = 0.0, fy = 0.0, fz = 0.0;
-  for (int k = 0; k < num; k++) {
-    const unsigned e = (unsigned)nlist[md_slab(k, i, stride)];
-    double dx, dy, dz, rsq;
-    int tt;
-    pair_geom<MIXED>(T, i, e, x4, xq, sx, sy, sz, box.qs, box.qs_lo, dx, dy, dz, rsq, tt);
-    if (rsq < T.cutsq[tt]) {
-      double phi;
-      if (MIXED) {
-        const float r2i = 1.0f / (float)rsq, r6i = r2i * r2i * r2i;
-        phi = (double)(((float)T.lj1[tt] * r6i - (float)T.lj2[tt]) * r6i * r2i);
-      } else {
-        const double r2i = 1.0 / rsq, r6i = r2i * r2i * r2i;
-        phi = (T.lj1[tt] * r6i - T.lj2[tt]) * r6i * r2i;
+  if (active) {
+    const AdjAtom<MIXED> me(a, i);
+    auto four = [&](const unsigned (&ee)[4], int m) {
+      double4 xj[4];
+      int4 qj[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int j = u < m ? md_entry_j(ee[u]) : i;
+        if (MIXED) qj[u] = __ldg(&a.xq[j]);
+        else xj[u] = a.x4[j];
       }
-      fx += phi * dx;
-      fy += phi * dy;
-      fz += phi * dz;
-    }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        if (u >= m) break;
+        double dx, dy, dz, rsq;
+        int tj;
+        me.geom(ee[u], xj[u], qj[u], dx, dy, dz, rsq, tj);
+        const int tt = me.row + tj;
+        if (rsq < S.cutsq[tt]) {
+          double phi;
+          if (MIXED) {
+            const float r2i = 1.0f / (float)rsq, r6i = r2i * r2i * r2i;
+            phi = (double)((S.lj1f[tt] * r6i - S.lj2f[tt]) * r6i * r2i);
+          } else {
+            const double r2i = 1.0 / rsq, r6i = r2i * r2i * r2i;
+            phi = (S.lj1[tt] * r6i - S.lj2[tt]) * r6i * r2i;
+          }
+          fx += phi * dx;
+          fy += phi * dy;
+          fz += phi * dz;
+        }
+      }
+    };
+    walk_list<TPA>(a.nlist, a.stride, i, a.numneigh[i], lane, four);
   }
-  const int o = orig[i];
-  f[3 * o] = fx;
-  f[3 * o + 1] = fy;
-  f[3 * o + 2] = fz;
+  fx = lane_sum<TPA>(fx);
+  fy = lane_sum<TPA>(fy);
+  fz = lane_sum<TPA>(fz);
+  if (active && lane == 0) {
+    const int o = a.orig[i];
+    a.out[3 * o] = fx;
+    a.out[3 * o + 1] = fy;
+    a.out[3 * o + 2] = fz;
+  }
 }
 
-// G in the caller's order -> G in the sorted order
+// G in the caller's order -> G in the sorted order, one 32-byte record per
+// atom (a pair's gather is then one sector)
 __global__ void k_adj_gather(int n, const int *__restrict__ orig, const double *__restrict__ g,
-                             double *__restrict__ gs) {
+                             double4 *__restrict__ gs) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int o = orig[i];
-  gs[3 * i] = g[3 * o];
-  gs[3 * i + 1] = g[3 * o + 1];
-  gs[3 * i + 2] = g[3 * o + 2];
+  gs[i] = make_double4(g[3 * o], g[3 * o + 1], g[3 * o + 2], 0.0);
 }
 
-template <bool MIXED>
-__global__ void __launch_bounds__(kAdjThreads)
-    k_adj_backward(int n, int stride, AdjTables T, BoxGeom box, const double4 *__restrict__ x4,
-                   const int4 *__restrict__ xq, const int *__restrict__ cell,
-                   const int *__restrict__ nlist, const int *__restrict__ numneigh,
-                   const int *__restrict__ orig, const double *__restrict__ gs,
-                   double *__restrict__ gx, double *partial, unsigned int *counter,
-                   double *gtab) {
-  __shared__ double red[2 * kAdjNP * (kAdjThreads / 32)];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  // per type pair: dL/dlj1, dL/dlj2 (selected by a compile-time unrolled
-  // loop so the accumulators stay in registers)
-  double acc[2 * kAdjNP];
+// dL/dx in the caller's order, and dL/dlj1, dL/dlj2 per type pair.  An atom's
+// type is the row of all its pairs, so a thread keeps sums for its row's NT
+// columns only (2 NT accumulators; one per type pair of the whole table, 32
+// of them, made the table update the largest part of the pair loop: 138 us at
+// 8,000 atoms, mixed, and 182 us at 54,647, FP64).  A block
+// adds its threads' sums by row in shared memory in a fixed order, the last
+// block the blocks' sums.
+template <bool MIXED, int NT, int TPA>
+__global__ void __launch_bounds__(kAdjThreads) k_adj_backward(AdjArgs a) {
+  constexpr int NV = 2 * NT * NT;
+  __shared__ AdjShared S;
+  __shared__ double s_acc[2 * NT][kAdjThreads];
+  __shared__ int s_row[kAdjThreads];
+  __shared__ bool last;
+  load_tables(S, a.T);
+  const int t = blockIdx.x * kAdjThreads + threadIdx.x;
+  const int i = t / TPA, lane = t % TPA;
+  const bool active = i < a.n;
+  double acc[2 * NT];
 #pragma unroll
-  for (int k = 0; k < 2 * kAdjNP; k++) acc[k] = 0.0;
-  if (i < n) {
-    int cx, cy, cz;
-    md_cell_unpack(cell[i], cx, cy, cz);
-    const Shift3 sx = shifts(cx, box.ncell[0], box.prd[0]);
-    const Shift3 sy = shifts(cy, box.ncell[1], box.prd[1]);
-    const Shift3 sz = shifts(cz, box.ncell[2], box.prd[2]);
-      const double gix = gs[3 * i], giy = gs[3 * i + 1], giz = gs[3 * i + 2];
-    const int num = numneigh[i];
-    double hx = 0.0, hy = 0.0, hz = 0.0;
-    for (int k = 0; k < num; k++) {
-      const unsigned e = (unsigned)nlist[md_slab(k, i, stride)];
-      const int j = md_entry_j(e);
-      double dx, dy, dz, rsq;
-      int tt;
-      pair_geom<MIXED>(T, i, e, x4, xq, sx, sy, sz, box.qs, box.qs_lo, dx, dy, dz, rsq, tt);
-      if (rsq < T.cutsq[tt]) {
-        const double wx = gix - gs[3 * j], wy = giy - gs[3 * j + 1], wz = giz - gs[3 * j + 2];
-        double phi, phis, r14, r8;
-        if (MIXED) {
-          const float r2i = 1.0f / (float)rsq, r6i = r2i * r2i * r2i;
-          const float l1 = (float)T.lj1[tt], l2 = (float)T.lj2[tt];
-          phi = (double)((l1 * r6i - l2) * r6i * r2i);
-          phis = (double)((4.0f * l2 - 7.0f * l1 * r6i) * r6i * r2i * r2i);
-          r14 = (double)(r6i * r6i * r2i);
-          r8 = (double)(r6i * r2i);
-        } else {
-          const double r2i = 1.0 / rsq, r6i = r2i * r2i * r2i;
-          const double l1 = T.lj1[tt], l2 = T.lj2[tt];
-          phi = (l1 * r6i - l2) * r6i * r2i;
-          phis = (4.0 * l2 - 7.0 * l1 * r6i) * r6i * r2i * r2i;
-          r14 = r6i * r6i * r2i;
-          r8 = r6i * r2i;
-        }
-        const double dw = dx * wx + dy * wy + dz * wz;
-        const double s = 2.0 * phis * dw;
-        hx += phi * wx + s * dx;
-        hy += phi * wy + s * dy;
-        hz += phi * wz + s * dz;
-        const double gd = gix * dx + giy * dy + giz * dz;
+  for (int k = 0; k < 2 * NT; k++) acc[k] = 0.0;
+  double hx = 0.0, hy = 0.0, hz = 0.0;
+  int myrow = -1;
+  if (active) {
+    const AdjAtom<MIXED> me(a, i);
+    myrow = me.row / a.T.ntypes;
+    const double4 gi = a.gs[i];
+    auto four = [&](const unsigned (&ee)[4], int m) {
+      double4 xj[4], gj[4];
+      int4 qj[4];
 #pragma unroll
-        for (int p = 0; p < kAdjNP; p++) {
-          acc[2 * p] += p == tt ? gd * r14 : 0.0;
-          acc[2 * p + 1] += p == tt ? -gd * r8 : 0.0;
+      for (int u = 0; u < 4; u++) {
+        const int j = u < m ? md_entry_j(ee[u]) : i;
+        if (MIXED) qj[u] = __ldg(&a.xq[j]);
+        else xj[u] = a.x4[j];
+        gj[u] = a.gs[j];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        if (u >= m) break;
+        double dx, dy, dz, rsq;
+        int tj;
+        me.geom(ee[u], xj[u], qj[u], dx, dy, dz, rsq, tj);
+        const int tt = me.row + tj;
+        if (rsq < S.cutsq[tt]) {
+          const double wx = gi.x - gj[u].x, wy = gi.y - gj[u].y, wz = gi.z - gj[u].z;
+          double phi, phis, r14, r8;
+          if (MIXED) {
+            const float r2i = 1.0f / (float)rsq, r6i = r2i * r2i * r2i;
+            const float l1 = S.lj1f[tt], l2 = S.lj2f[tt];
+            phi = (double)((l1 * r6i - l2) * r6i * r2i);
+            phis = (double)((4.0f * l2 - 7.0f * l1 * r6i) * r6i * r2i * r2i);
+            r14 = (double)(r6i * r6i * r2i);
+            r8 = (double)(r6i * r2i);
+          } else {
+            const double r2i = 1.0 / rsq, r6i = r2i * r2i * r2i;
+            const double l1 = S.lj1[tt], l2 = S.lj2[tt];
+            phi = (l1 * r6i - l2) * r6i * r2i;
+            phis = (4.0 * l2 - 7.0 * l1 * r6i) * r6i * r2i * r2i;
+            r14 = r6i * r6i * r2i;
+            r8 = r6i * r2i;
+          }
+          const double dw = dx * wx + dy * wy + dz * wz;
+          const double s = 2.0 * phis * dw;
+          hx += phi * wx + s * dx;
+          hy += phi * wy + s * dy;
+          hz += phi * wz + s * dz;
+          const double gd = gi.x * dx + gi.y * dy + gi.z * dz;
+#pragma unroll
+          for (int p = 0; p < NT; p++)
+            if (NT == 1 || p == tj) {
+              acc[2 * p] += gd * r14;
+              acc[2 * p + 1] -= gd * r8;
+            }
         }
       }
-    }
-    const int o = orig[i];
-    gx[3 * o] = hx;
-    gx[3 * o + 1] = hy;
-    gx[3 * o + 2] = hz;
+    };
+    walk_list<TPA>(a.nlist, a.stride, i, a.numneigh[i], lane, four);
   }
-  block_partials_finish<2 * kAdjNP>(acc, red, partial, counter, gtab, false);
+  hx = lane_sum<TPA>(hx);
+  hy = lane_sum<TPA>(hy);
+  hz = lane_sum<TPA>(hz);
+  if (active && lane == 0) {
+    const int o = a.orig[i];
+    a.out[3 * o] = hx;
+    a.out[3 * o + 1] = hy;
+    a.out[3 * o + 2] = hz;
+  }
+  // parameter gradients: value k = 2 (ti NT + tj) + q of the block
+#pragma unroll
+  for (int k = 0; k < 2 * NT; k++) s_acc[k][threadIdx.x] = acc[k];
+  s_row[threadIdx.x] = myrow;
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, l = threadIdx.x & 31;
+  for (int k = warp; k < NV; k += kAdjThreads / 32) {
+    const int ti = (k >> 1) / NT, col = 2 * ((k >> 1) % NT) + (k & 1);
+    double v = 0.0;
+#pragma unroll
+    for (int q = 0; q < kAdjThreads / 32; q++)
+      v += s_row[l + 32 * q] == ti ? s_acc[col][l + 32 * q] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (l == 0) a.partial[(size_t)blockIdx.x * NV + k] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(a.counter, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int k = warp; k < NV; k += kAdjThreads / 32) {
+    double v = 0.0;
+    for (unsigned b = l; b < gridDim.x; b += 32) v += __ldcg(&a.partial[(size_t)b * NV + k]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    // the table is (ntypes x ntypes)
+    const int ti = (k >> 1) / NT, tj = (k >> 1) % NT, nt = a.T.ntypes;
+    if (l == 0 && ti < nt && tj < nt) a.gtab[2 * (ti * nt + tj) + (k & 1)] = v;
+  }
+  if (threadIdx.x == 0) *a.counter = 0u;
 }
 
 AdjTables make_tables(const b200_ctx *c, const double *lj1, const double *lj2,
@@ -202,18 +324,56 @@ AdjTables make_tables(const b200_ctx *c, const double *lj1, const double *lj2,
 
 }  // namespace
 
+// Threads per atom of both passes.  With one, the chip is full from about
+// 32,000 atoms on (54,647 atoms, FP64, forward and backward: 1,072 us with
+// one, 1,088 two, 1,108 four, 1,141 eight); smaller boxes take up to eight
+// (8,000 atoms, mixed: 861 us with eight, 901 with one).
+static int adj_tpa(int n) {
+  return n >= 32000 ? 1 : n >= 16000 ? 2 : n >= 10000 ? 4 : 8;
+}
+
+static AdjArgs adj_args(b200_ctx *c, const double *lj1, const double *lj2, const double *cutsq) {
+  AdjArgs a{};
+  a.n = c->n;
+  a.stride = c->stride;
+  a.T = make_tables(c, lj1, lj2, cutsq);
+  a.box = c->box;
+  a.x4 = c->x4;
+  a.xq = c->xq;
+  a.cell = c->cell;
+  a.nlist = c->nlist;
+  a.numneigh = c->numneigh;
+  a.orig = c->orig;
+  a.partial = c->partial;
+  a.counter = c->counter;
+  return a;
+}
+
+template <bool MIXED>
+static void launch_forward(b200_ctx *c, const AdjArgs &a, int tpa) {
+  const int grid = md_blocks((long long)a.n * tpa, kAdjThreads);
+  if (tpa == 1) k_adj_forward<MIXED, 1><<<grid, kAdjThreads, 0, c->stream>>>(a);
+  else if (tpa == 2) k_adj_forward<MIXED, 2><<<grid, kAdjThreads, 0, c->stream>>>(a);
+  else if (tpa == 4) k_adj_forward<MIXED, 4><<<grid, kAdjThreads, 0, c->stream>>>(a);
+  else k_adj_forward<MIXED, 8><<<grid, kAdjThreads, 0, c->stream>>>(a);
+}
+
+template <bool MIXED, int NT>
+static void launch_backward(b200_ctx *c, const AdjArgs &a, int tpa) {
+  const int grid = md_blocks((long long)a.n * tpa, kAdjThreads);
+  if (tpa == 1) k_adj_backward<MIXED, NT, 1><<<grid, kAdjThreads, 0, c->stream>>>(a);
+  else if (tpa == 2) k_adj_backward<MIXED, NT, 2><<<grid, kAdjThreads, 0, c->stream>>>(a);
+  else if (tpa == 4) k_adj_backward<MIXED, NT, 4><<<grid, kAdjThreads, 0, c->stream>>>(a);
+  else k_adj_backward<MIXED, NT, 8><<<grid, kAdjThreads, 0, c->stream>>>(a);
+}
+
 cudaError_t md_adj_forward(b200_ctx *c, const double *lj1, const double *lj2, const double *cutsq,
                            double *f) {
-  const AdjTables T = make_tables(c, lj1, lj2, cutsq);
-  const int grid = md_blocks(c->n, kAdjThreads);
-  if (c->prec == B200_PREC_MIXED)
-    k_adj_forward<true><<<grid, kAdjThreads, 0, c->stream>>>(c->n, c->stride, T, c->box, c->x4,
-                                                             c->xq, c->cell, c->nlist,
-                                                             c->numneigh, c->orig, f);
-  else
-    k_adj_forward<false><<<grid, kAdjThreads, 0, c->stream>>>(c->n, c->stride, T, c->box, c->x4,
-                                                              c->xq, c->cell, c->nlist,
-                                                              c->numneigh, c->orig, f);
+  AdjArgs a = adj_args(c, lj1, lj2, cutsq);
+  a.out = f;
+  const int tpa = adj_tpa(c->n);
+  if (c->prec == B200_PREC_MIXED) launch_forward<true>(c, a, tpa);
+  else launch_forward<false>(c, a, tpa);
   c->launches++;
   return cudaGetLastError();
 }
@@ -221,17 +381,22 @@ cudaError_t md_adj_forward(b200_ctx *c, const double *lj1, const double *lj2, co
 cudaError_t md_adj_backward(b200_ctx *c, const double *lj1, const double *lj2,
                             const double *cutsq, const double *g, double *gx, double *gs,
                             double *gtab) {
-  const AdjTables T = make_tables(c, lj1, lj2, cutsq);
-  const int grid = md_blocks(c->n, kAdjThreads);
-  k_adj_gather<<<md_blocks(c->n, 256), 256, 0, c->stream>>>(c->n, c->orig, g, gs);
-  if (c->prec == B200_PREC_MIXED)
-    k_adj_backward<true><<<grid, kAdjThreads, 0, c->stream>>>(
-        c->n, c->stride, T, c->box, c->x4, c->xq, c->cell, c->nlist, c->numneigh, c->orig, gs, gx,
-        c->partial, c->counter, gtab);
-  else
-    k_adj_backward<false><<<grid, kAdjThreads, 0, c->stream>>>(
-        c->n, c->stride, T, c->box, c->x4, c->xq, c->cell, c->nlist, c->numneigh, c->orig, gs, gx,
-        c->partial, c->counter, gtab);
+  AdjArgs a = adj_args(c, lj1, lj2, cutsq);
+  double4 *gs4 = reinterpret_cast<double4 *>(gs);
+  a.gs = gs4;
+  a.out = gx;
+  a.gtab = gtab;
+  const int tpa = adj_tpa(c->n), nt = c->ntypes;
+  k_adj_gather<<<md_blocks(c->n, 256), 256, 0, c->stream>>>(c->n, c->orig, g, gs4);
+  if (c->prec == B200_PREC_MIXED) {
+    if (nt == 1) launch_backward<true, 1>(c, a, tpa);
+    else if (nt == 2) launch_backward<true, 2>(c, a, tpa);
+    else launch_backward<true, 4>(c, a, tpa);
+  } else {
+    if (nt == 1) launch_backward<false, 1>(c, a, tpa);
+    else if (nt == 2) launch_backward<false, 2>(c, a, tpa);
+    else launch_backward<false, 4>(c, a, tpa);
+  }
   c->launches += 2;
   return cudaGetLastError();
 }

@@ -2150,7 +2150,7 @@ int b200_adj_backward(b200_ctx *c, const double *lj1, const double *lj2, const d
   if (rc) return rc;
   if (!g || !gx) return set_err(c, B200_ERR_ARG, "null gradient array");
   if (c->adj_n < c->n) {
-    CK(dalloc(&c->adj_gs, 3 * (size_t)c->stride));
+    CK(dalloc(&c->adj_gs, 4 * (size_t)c->stride));
     c->adj_n = c->stride;
   }
   if (!c->adj_gtab) CK(dalloc(&c->adj_gtab, 2 * MD_ADJ_MAXTYPES * MD_ADJ_MAXTYPES));

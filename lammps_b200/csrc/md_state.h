@@ -300,7 +300,7 @@ cudaError_t md_zero_ev(b200_ctx *c);
 
 // ---- force-matching adjoint (adjoint.cu) ------------------------------------
 // lj1, lj2, cutsq: host (ntypes+1)^2 tables; f, g, gx: device, 3n doubles in
-// the caller's order; gs: device scratch of 3n doubles; gtab: device, 2 *
+// the caller's order; gs: device scratch of 4n doubles; gtab: device, 2 *
 // MD_ADJ_MAXTYPES^2 doubles (dL/dlj1, dL/dlj2 per type pair)
 cudaError_t md_adj_forward(b200_ctx *c, const double *lj1, const double *lj2, const double *cutsq,
                            double *f);
