@@ -1061,7 +1061,7 @@ int b200_destroy(b200_ctx *c) {
   dfree(c->x4); dfree(c->x4b); dfree(c->v); dfree(c->vb); dfree(c->f);
   dfree(c->orig); dfree(c->origb); dfree(c->image); dfree(c->imageb); dfree(c->cell);
   dfree(c->where); dfree(c->ghost);
-  dfree(c->xq); dfree(c->xqb); dfree(c->xhold); dfree(c->xfer); dfree(c->rho); dfree(c->fp); dfree(c->fpf); dfree(c->mass_dev);
+  dfree(c->xq); dfree(c->xqb); dfree(c->xhold); dfree(c->xfer); dfree(c->rho); dfree(c->fp); dfree(c->fpf); dfree(c->xf); dfree(c->mass_dev);
   dfree(c->eam_eatom); dfree(c->d_rep_grp_first); dfree(c->d_rep_ranges);
   dfree(c->cell_count); dfree(c->cell_start); dfree(c->scan_tmp);
   dfree(c->slot); dfree(c->perm); dfree(c->cell_tmp);
@@ -1074,7 +1074,7 @@ int b200_destroy(b200_ctx *c) {
   dfree(c->snap_orig); dfree(c->snap_image); dfree(c->snap_cell); dfree(c->snap_xq);
   dfree(c->snap_status);
   dfree(c->eam.frho); dfree(c->eam.rhor); dfree(c->eam.z2r);
-  dfree(c->eam.frho_f); dfree(c->eam.rhor_f); dfree(c->eam.z2r_f); dfree(c->eam.fz_f);
+  dfree(c->eam.frho_f); dfree(c->eam.rhor_f); dfree(c->eam.z2r_f); dfree(c->eam.fz); dfree(c->eam.fz_f);
   for (auto &ev : c->ph_event)
     if (ev) cudaEventDestroy(ev);
   for (auto ev : c->ev_pool) cudaEventDestroy(ev);
@@ -1238,13 +1238,16 @@ int b200_set_eam(b200_ctx *c, int ntypes, int nrho, double drho, int nr, double 
     // one element: the z2 value and rho' coefficients of each knot in one
     // 32-byte record for the mixed force kernel
     const size_t ri = (size_t)E.type2rhor[ntp1 + 1], zi = (size_t)E.type2z2r[ntp1 + 1];
-    std::vector<float> fz((size_t)(nr + 1) * 8, 0.0f);
+    std::vector<double> fz((size_t)(nr + 1) * 8, 0.0);
     for (size_t m = 0; m <= (size_t)nr; m++) {
-      for (int k = 0; k < 4; k++) fz[m * 8 + k] = (float)z2r_spline[(zi * (nr + 1) + m) * 7 + 3 + k];
-      for (int k = 0; k < 3; k++) fz[m * 8 + 4 + k] = (float)rhor_spline[(ri * (nr + 1) + m) * 7 + k];
+      for (int k = 0; k < 4; k++) fz[m * 8 + k] = z2r_spline[(zi * (nr + 1) + m) * 7 + 3 + k];
+      for (int k = 0; k < 3; k++) fz[m * 8 + 4 + k] = rhor_spline[(ri * (nr + 1) + m) * 7 + k];
     }
-    CK(dalloc(&E.fz_f, fz.size()));
-    CK(cudaMemcpy(E.fz_f, fz.data(), fz.size() * sizeof(float), cudaMemcpyHostToDevice));
+    const std::vector<float> fzf(fz.begin(), fz.end());
+    CK(dalloc(&E.fz, fz.size()));
+    CK(cudaMemcpy(E.fz, fz.data(), fz.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CK(dalloc(&E.fz_f, fzf.size()));
+    CK(cudaMemcpy(E.fz_f, fzf.data(), fzf.size() * sizeof(float), cudaMemcpyHostToDevice));
   }
   c->ntypes = ntypes;
   c->pstyle = B200_PAIR_EAM;
@@ -1343,6 +1346,7 @@ int b200_upload_atoms(b200_ctx *c, int n, const double *x, const double *v, cons
   c->sorted_once = false;
   return B200_OK;
 }
+    CK(dalloc(&c->xf, stride));
 
 int b200_natoms(const b200_ctx *c) { return c ? c->n : 0; }
 

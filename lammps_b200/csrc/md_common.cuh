@@ -198,6 +198,31 @@ __device__ __forceinline__ float rcp_approx_f32(float x) {
 }
 
 // FP64 helpers that keep a*b+c rounded twice, as the reference's x86-64
+// Position loads of the pair loops.  A kernel that runs several steps reads
+// positions that other blocks wrote earlier in the same launch: COH makes
+// them plain loads (ordered by the grid barrier) instead of read-only ones.
+template <bool COH>
+__device__ __forceinline__ int4 ld_pos(const int4 *p) {
+  if (!COH) return __ldg(p);
+  int4 v;
+  asm volatile("ld.global.v4.s32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+template <bool COH>
+__device__ __forceinline__ double4 ld_pos(const double4 *p) {
+  // one 32-byte load: a gather of 32-byte records by two 16-byte loads takes
+  // a fifth more passes through the L1 data banks
+  double4 v;
+  if (COH)
+    asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
+                 : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  else
+    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];"
+        : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
+
 // build computes them; used wherever a comparison must be bit-exact.
 __device__ __forceinline__ double dsq3(double a, double b, double c) {
   return __dadd_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)), __dmul_rn(c, c));

@@ -33,6 +33,7 @@ struct EAMDev {
   // embedding rows [c0..c6 -], density and pair rows [c3 c4 c5 c6 c0 c1 c2 -]
   double *frho = nullptr, *rhor = nullptr, *z2r = nullptr;
   float *frho_f = nullptr, *rhor_f = nullptr, *z2r_f = nullptr;
+  double *fz = nullptr;   // one element, as fz_f
   float *fz_f = nullptr;  // one element: [z2 c3..c6 | rho' c0..c2 | 0] per knot
   int type2frho[MD_MAXTYPES + 1];
   int type2rhor[(MD_MAXTYPES + 1) * (MD_MAXTYPES + 1)];
@@ -130,6 +131,7 @@ struct b200_ctx {
   int out_next = 0;
   double *rho = nullptr, *fp = nullptr;
   float *fpf = nullptr;
+  double4 *xf = nullptr;  // one element: position and F' records (EamArgs::xf)
   // split EAM compute (b200_eam_density, then b200_eam_force): the eflag /
   // vflag of the density call and its per-atom embedding energies
   int eam_split_eflag = -1, eam_split_vflag = -1;

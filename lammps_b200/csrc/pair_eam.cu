@@ -26,7 +26,14 @@
 // rho' coefficients as one 32-byte record (fz_f) and forms the z2
 // derivative from the value coefficients, (3 c3 p^2 + 2 c4 p + c5) / dr,
 // the relation PairEAM::interpolate (:723-751) builds the stored derivative
-// coefficients from.
+// coefficients from; the FP64 form does the same with 64-byte records.
+// FP64 pair terms are long dependent chains, so that form is branch-free (an
+// entry past the cutoff reads row 0 and adds nothing) and loads positions and
+// knots 32 bytes at a time: at 252,933 copper atoms, 2 lanes, a step's two
+// passes went from 411 to 290 us.  The mixed form keeps the branch: its chains
+// are short, and branch-free it was 3 % slower at 32,000 atoms.  With one
+// element the density pass leaves position and F' in one record per atom, so
+// the force pass gathers once per neighbor (3.5 % of the FP64 run).
 #include "md_state.h"
 
 namespace {
@@ -40,10 +47,15 @@ struct EamArgs {
   double rdr, rdrho, rhomax, cutforcesq;
   const double *frho, *rhor, *z2r;
   const float *rhor_f, *z2r_f;
-  const float *fz_f;  // one element: per knot [z2 c3 c4 c5 c6 | rho' c0 c1 c2 | 0]
+  const double *fz;   // one element: per knot [z2 c3 c4 c5 c6 | rho' c0 c1 c2 | 0]
+  const float *fz_f;  // the same in FP32
   const int *t2frho, *t2rhor, *t2z2r;  // device copies of the type maps
   double *rho, *fp;
   float *fpf;
+  // one element: position and F' of each atom in one record (double4, or int4
+  // with F' as FP32 bits in the mixed form), written by the density pass, so
+  // that the force pass gathers one record per neighbor
+  double4 *xf;
   double *f;
   double *partial;
   unsigned int *counter;
@@ -90,6 +102,18 @@ __device__ __forceinline__ void embed(const EamArgs &a, int itype_frho, double r
   if (rho > a.rhomax) phi += fp * (rho - a.rhomax);
 }
 
+template <bool MIXED>
+__device__ __forceinline__ void store_xf(double4 *xf, int i, const double4 *x4, const int4 *xq,
+                                         double fp) {
+  if (MIXED) {
+    const int4 q = xq[i];
+    reinterpret_cast<int4 *>(xf)[i] = make_int4(q.x, q.y, q.z, __float_as_int((float)fp));
+  } else {
+    const double4 p = x4[i];
+    xf[i] = make_double4(p.x, p.y, p.z, fp);
+  }
+}
+
 template <int TPA, bool EV, bool ATOM, bool MIXED, bool SINGLE>
 __global__ void __launch_bounds__(128) k_eam_rho(EamArgs a, const double4 *__restrict__ x4,
                                                  const int4 *__restrict__ xq) {
@@ -121,32 +145,35 @@ __global__ void __launch_bounds__(128) k_eam_rho(EamArgs a, const double4 *__res
       // four entries ee of this lane (walk_list); the first mm lie before the
       // atom's count
       auto four = [&](const unsigned (&ee)[4], int mm) {
-        double4 xq[4];
+        // branch-free, so that the four entries' chains and table loads
+        // overlap; an entry past mm or past the cutoff reads row 0 (one
+        // address for all of them) and adds nothing
+        double4 xj[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) xq[u] = x4[u < mm ? md_entry_j(ee[u]) : i];
+        for (int u = 0; u < 4; u++) xj[u] = ld_pos<false>(&x4[u < mm ? md_entry_j(ee[u]) : i]);
+        double val[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-          if (u >= mm) break;
           int j, dx, dy, dz;
           decode(ee[u], j, dx, dy, dz);
-          const double4 xj = xq[u];
-          const double delx = __dsub_rn(xi.x, __dadd_rn(xj.x, pick(sx, dx)));
-          const double dely = __dsub_rn(xi.y, __dadd_rn(xj.y, pick(sy, dy)));
-          const double delz = __dsub_rn(xi.z, __dadd_rn(xj.z, pick(sz, dz)));
+          const double delx = __dsub_rn(xi.x, __dadd_rn(xj[u].x, pick(sx, dx)));
+          const double dely = __dsub_rn(xi.y, __dadd_rn(xj[u].y, pick(sy, dy)));
+          const double delz = __dsub_rn(xi.z, __dadd_rn(xj[u].z, pick(sz, dz)));
           const double rsq = dsq3(delx, dely, delz);
-          if (rsq < a.cutforcesq) {
-            int m;
-            double p;
-            knot_d(__dadd_rn(__dmul_rn(sqrt(rsq), a.rdr), 1.0), a.nr - 1, m, p);
-            const double *row =
-                SINGLE ? rrow : a.rhor + (size_t)s_t2rhor[(int)xj.w * a.ntp1 + ti] * (a.nr + 1) * 8;
-            // knot layout [c3 c4 c5 c6 | c0 c1 c2 -]: the value coefficients
-            // are two 16-byte loads
-            const double2 v01 = __ldg(reinterpret_cast<const double2 *>(row + (size_t)m * 8));
-            const double2 v23 = __ldg(reinterpret_cast<const double2 *>(row + (size_t)m * 8 + 2));
-            rho += ((v01.x * p + v01.y) * p + v23.x) * p + v23.y;
-          }
+          const bool in = u < mm && rsq < a.cutforcesq;
+          int m;
+          double p;
+          knot_d(__dadd_rn(__dmul_rn(sqrt(in ? rsq : 0.0), a.rdr), 1.0), a.nr - 1, m, p);
+          const double *row =
+              SINGLE ? rrow
+                     : a.rhor + (size_t)s_t2rhor[(int)xj[u].w * a.ntp1 + ti] * (a.nr + 1) * 8;
+          // knot layout [c3 c4 c5 c6 | c0 c1 c2 -]: the value coefficients
+          // are one 32-byte load
+          const double4 c = ld_pos<false>(reinterpret_cast<const double4 *>(row + (size_t)m * 8));
+          val[u] = in ? ((c.x * p + c.y) * p + c.z) * p + c.w : 0.0;
         }
+#pragma unroll
+        for (int u = 0; u < 4; u++) rho += val[u];
       };
       walk_list<TPA>(a.nlist, a.stride, i, num, lane, four);
     } else {
@@ -198,6 +225,7 @@ __global__ void __launch_bounds__(128) k_eam_rho(EamArgs a, const double4 *__res
     a.rho[i] = rho;
     a.fp[i] = fpi;
     if (MIXED) a.fpf[i] = (float)fpi;
+    if (SINGLE) store_xf<MIXED>(a.xf, i, x4, xq, fpi);
     if (EV) {
       acc[0] = phi;
       if (ATOM && a.eatom) a.eatom[a.orig[i]] = phi;
@@ -237,74 +265,78 @@ __global__ void __launch_bounds__(128) k_eam_force(EamArgs a, const double4 *__r
       const Shift3 sx = shifts(cx, a.box.ncell[0], a.box.prd[0]);
       const Shift3 sy = shifts(cy, a.box.ncell[1], a.box.prd[1]);
       const Shift3 sz = shifts(cz, a.box.ncell[2], a.box.prd[2]);
-      // one element: the density and pair spline rows of every pair
-      const double *rrow1 =
-          SINGLE ? a.rhor + (size_t)s_t2rhor[a.ntp1 + 1] * (a.nr + 1) * 8 : nullptr;
-      const double *zrow1 = SINGLE ? a.z2r + (size_t)s_t2z2r[a.ntp1 + 1] * (a.nr + 1) * 8 : nullptr;
       // four entries ee of this lane (walk_list); the first mm lie before the
       // atom's count
       auto four = [&](const unsigned (&ee)[4], int mm) {
-       double4 xq[4];
+       // branch-free as the density pass
+       double4 xj[4];
        double fpq[4];
 #pragma unroll
        for (int u = 0; u < 4; u++) {
          const int jj = u < mm ? md_entry_j(ee[u]) : i;
-         xq[u] = x4[jj];
-         fpq[u] = a.fp[jj];
+         xj[u] = ld_pos<false>(&(SINGLE ? a.xf : x4)[jj]);
+         fpq[u] = SINGLE ? xj[u].w : a.fp[jj];
        }
 #pragma unroll
        for (int u = 0; u < 4; u++) {
-        if (u >= mm) break;
         int j, dx, dy, dz;
         decode(ee[u], j, dx, dy, dz);
-        const double4 xj = xq[u];
-        const double delx = __dsub_rn(xi.x, __dadd_rn(xj.x, pick(sx, dx)));
-        const double dely = __dsub_rn(xi.y, __dadd_rn(xj.y, pick(sy, dy)));
-        const double delz = __dsub_rn(xi.z, __dadd_rn(xj.z, pick(sz, dz)));
+        const double delx = __dsub_rn(xi.x, __dadd_rn(xj[u].x, pick(sx, dx)));
+        const double dely = __dsub_rn(xi.y, __dadd_rn(xj[u].y, pick(sy, dy)));
+        const double delz = __dsub_rn(xi.z, __dadd_rn(xj[u].z, pick(sz, dz)));
         const double rsq = dsq3(delx, dely, delz);
-        if (rsq < a.cutforcesq) {
-          const int tj = (int)xj.w;
-          const double r = sqrt(rsq);
-          int m;
-          double p;
-          knot_d(__dadd_rn(__dmul_rn(r, a.rdr), 1.0), a.nr - 1, m, p);
-          const size_t o8 = (size_t)m * 8;
+        const bool in = u < mm && rsq < a.cutforcesq;
+        const int tj = SINGLE ? 1 : (int)xj[u].w;
+        const double r = sqrt(in ? rsq : 1.0);
+        int m;
+        double p;
+        knot_d(__dadd_rn(__dmul_rn(r, a.rdr), 1.0), a.nr - 1, m, p);
+        const size_t o8 = in ? (size_t)m * 8 : 0;
+        double rhoip, rhojp, z2, z2p;
+        if (SINGLE) {
+          // one element: the pair value and density derivative of a knot in
+          // one 64-byte record; the pair derivative from the value's
+          // coefficients, (3 c3 p^2 + 2 c4 p + c5) / dr
+          const double4 z = ld_pos<false>(reinterpret_cast<const double4 *>(a.fz + o8));
+          const double4 d = ld_pos<false>(reinterpret_cast<const double4 *>(a.fz + o8 + 4));
+          rhoip = (d.x * p + d.y) * p + d.z;
+          rhojp = rhoip;
+          z2 = ((z.x * p + z.y) * p + z.z) * p + z.w;
+          z2p = (fma(3.0 * z.x, p, 2.0 * z.y) * p + z.z) * a.rdr;
+        } else {
           // knot layout [c3 c4 c5 c6 | c0 c1 c2 -]
-          const double *ci =
-              (SINGLE ? rrow1 : a.rhor + (size_t)s_t2rhor[ti * a.ntp1 + tj] * (a.nr + 1) * 8) + o8;
-          const double2 d01 = __ldg(reinterpret_cast<const double2 *>(ci + 4));
-          const double rhoip = (d01.x * p + d01.y) * p + __ldg(ci + 6);
-          double rhojp = rhoip;
-          if (!SINGLE && !a.rhor_sym) {
-            const double *cj = a.rhor + ((size_t)s_t2rhor[tj * a.ntp1 + ti] * (a.nr + 1) + m) * 8;
-            const double2 e01 = __ldg(reinterpret_cast<const double2 *>(cj + 4));
-            rhojp = (e01.x * p + e01.y) * p + __ldg(cj + 6);
+          const double4 d = ld_pos<false>(reinterpret_cast<const double4 *>(
+              a.rhor + (size_t)s_t2rhor[ti * a.ntp1 + tj] * (a.nr + 1) * 8 + o8 + 4));
+          rhoip = (d.x * p + d.y) * p + d.z;
+          rhojp = rhoip;
+          if (!a.rhor_sym) {
+            const double4 e = ld_pos<false>(reinterpret_cast<const double4 *>(
+                a.rhor + (size_t)s_t2rhor[tj * a.ntp1 + ti] * (a.nr + 1) * 8 + o8 + 4));
+            rhojp = (e.x * p + e.y) * p + e.z;
           }
-          const double *cz2 =
-              (SINGLE ? zrow1 : a.z2r + (size_t)s_t2z2r[ti * a.ntp1 + tj] * (a.nr + 1) * 8) + o8;
-          const double2 z01 = __ldg(reinterpret_cast<const double2 *>(cz2));
-          const double2 z23 = __ldg(reinterpret_cast<const double2 *>(cz2 + 2));
-          const double2 zd01 = __ldg(reinterpret_cast<const double2 *>(cz2 + 4));
-          const double z2p = (zd01.x * p + zd01.y) * p + __ldg(cz2 + 6);
-          const double z2 = ((z01.x * p + z01.y) * p + z23.x) * p + z23.y;
-          const double recip = rcp_nr(r);
-          const double phi = z2 * recip;
-          const double phip = z2p * recip - phi * recip;
-          const double psip = fpi * rhojp + fpq[u] * rhoip + phip;
-          const double fpair = -psip * recip;
-          fx += delx * fpair;
-          fy += dely * fpair;
-          fz += delz * fpair;
-          if (EV) {
-            acc[0] += 0.5 * phi;
-            const double hf = 0.5 * fpair;
-            acc[1] += delx * delx * hf;
-            acc[2] += dely * dely * hf;
-            acc[3] += delz * delz * hf;
-            acc[4] += delx * dely * hf;
-            acc[5] += delx * delz * hf;
-            acc[6] += dely * delz * hf;
-          }
+          const double *cz = a.z2r + (size_t)s_t2z2r[ti * a.ntp1 + tj] * (a.nr + 1) * 8 + o8;
+          const double4 z = ld_pos<false>(reinterpret_cast<const double4 *>(cz));
+          const double4 zd = ld_pos<false>(reinterpret_cast<const double4 *>(cz + 4));
+          z2p = (zd.x * p + zd.y) * p + zd.z;
+          z2 = ((z.x * p + z.y) * p + z.z) * p + z.w;
+        }
+        const double recip = rcp_nr(r);
+        const double phi = in ? z2 * recip : 0.0;
+        const double phip = z2p * recip - phi * recip;
+        const double psip = fpi * rhojp + fpq[u] * rhoip + phip;
+        const double fpair = in ? -psip * recip : 0.0;
+        fx += delx * fpair;
+        fy += dely * fpair;
+        fz += delz * fpair;
+        if (EV) {
+          acc[0] += 0.5 * phi;
+          const double hf = 0.5 * fpair;
+          acc[1] += delx * delx * hf;
+          acc[2] += dely * dely * hf;
+          acc[3] += delz * delz * hf;
+          acc[4] += delx * dely * hf;
+          acc[5] += delx * delz * hf;
+          acc[6] += dely * delz * hf;
         }
        }
       };
@@ -328,8 +360,8 @@ __global__ void __launch_bounds__(128) k_eam_force(EamArgs a, const double4 *__r
 #pragma unroll
        for (int u = 0; u < 4; u++) {
          const int jj = md_entry_j(ee[u]);
-         xs[u] = xq[jj];
-         fpq[u] = a.fpf[jj];
+         xs[u] = SINGLE ? __ldg(reinterpret_cast<const int4 *>(a.xf) + jj) : xq[jj];
+         fpq[u] = SINGLE ? __int_as_float(xs[u].w) : a.fpf[jj];
        }
        // FP32 sum of the slab's pair forces, added to the FP64 accumulator
        float cfx = 0.f, cfy = 0.f, cfz = 0.f;
@@ -343,7 +375,7 @@ __global__ void __launch_bounds__(128) k_eam_force(EamArgs a, const double4 *__r
         const float delz = md_qlen(md_qdiff(xi.z, xj.z), qz, qzl);
         const float rsq = delx * delx + dely * dely + delz * delz;
         if (rsq < cutf && rsq > 0.f) {
-          const int tj = xj.w;
+          const int tj = SINGLE ? 1 : xj.w;
           const float recip = rsqrtf(rsq);
           const float r = rsq * recip;
           int m;
@@ -533,6 +565,15 @@ __global__ void k_fp_unpack(int m, int n, const int *__restrict__ idx,
   if (fpf) fpf[k] = (float)buf[i];
 }
 
+// the position and F' records again, before a force pass that runs by itself
+// (ghosts have received their F' since the density pass)
+template <bool MIXED>
+__global__ void k_eam_xf(int n, const double4 *__restrict__ x4, const int4 *__restrict__ xq,
+                         const double *__restrict__ fp, double4 *__restrict__ xf) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) store_xf<MIXED>(xf, i, x4, xq, fp[i]);
+}
+
 }  // namespace
 
 cudaError_t md_eam_fp_halo(b200_ctx *c, int m, const int *idx, double *buf, bool pack) {
@@ -570,6 +611,7 @@ static EamArgs eam_args(b200_ctx *c, double *eatom, double *vatom) {
   a.z2r = c->eam.z2r;
   a.rhor_f = c->eam.rhor_f;
   a.z2r_f = c->eam.z2r_f;
+  a.fz = c->eam.fz;
   a.fz_f = c->eam.fz_f;
   // type maps live right after the TAB_* tables in tables_dev (as ints)
   const int *maps = reinterpret_cast<const int *>(c->tables_dev + TAB_COUNT * TABSZ);
@@ -579,6 +621,7 @@ static EamArgs eam_args(b200_ctx *c, double *eatom, double *vatom) {
   a.rho = c->rho;
   a.fp = c->fp;
   a.fpf = c->fpf;
+  a.xf = c->xf;
   a.f = c->f;
   a.partial = c->partial;
   a.counter = c->counter;
@@ -591,6 +634,14 @@ static EamArgs eam_args(b200_ctx *c, double *eatom, double *vatom) {
 cudaError_t md_eam_compute(b200_ctx *c, bool ev, bool atom_ev, double *eatom, double *vatom,
                            cudaEvent_t mid, int stage) {
   EamArgs a = eam_args(c, eatom, vatom);
+  if (stage == EAM_FORCE && c->ntypes == 1) {
+    const int B = 256, grid = md_blocks(c->n, B);
+    if (c->prec == B200_PREC_MIXED)
+      k_eam_xf<true><<<grid, B, 0, c->stream>>>(c->n, c->x4, c->xq, c->fp, c->xf);
+    else
+      k_eam_xf<false><<<grid, B, 0, c->stream>>>(c->n, c->x4, c->xq, c->fp, c->xf);
+    c->launches++;
+  }
   switch (c->tpa) {
     case 1: launch_tpa<1>(c, a, ev, atom_ev, mid, stage); break;
     case 2: launch_tpa<2>(c, a, ev, atom_ev, mid, stage); break;
