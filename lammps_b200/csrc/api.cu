@@ -484,6 +484,8 @@ int status_errors(b200_ctx *c) {
   if (c->status_host[ST_LOST])
     return set_err(c, B200_ERR_LOST_ATOMS,
                    "Lost atoms: a coordinate is not finite or moved beyond one box length");
+  if (c->status_host[ST_BARRIER])
+    return set_err(c, B200_ERR_CUDA, "a grid barrier of a multi-step launch timed out");
   if (c->status_host[ST_OVERFLOW])
     return set_err(c, B200_ERR_NEIGH_OVERFLOW,
                    "Neighbor list overflow, boost neigh_modify one (need %d, have %d)",
@@ -521,6 +523,22 @@ int rebuild_sync(b200_ctx *c) {
   return set_err(c, B200_ERR_NEIGH_OVERFLOW, "Neighbor list overflow, boost neigh_modify one");
 }
 
+// `nsteps` MD steps in one launch
+// (md_lj_multi), from `ago` steps since the build, under the given schedule;
+// the barrier words' other set becomes current
+int launch_multi(b200_ctx *c, const MultiPlan &plan, int nsteps, int ago, double dtv, double dtf, int every,
+                 int check) {
+  MultiArgs m;
+  m.nsteps = nsteps;
+  m.ago = ago;
+  m.bar = c->bar + c->bar_set * MD_BAR_WORDS;
+  m.bar_next = c->bar + (c->bar_set ^ 1) * MD_BAR_WORDS;
+  m.bar_words = MD_BAR_WORDS;
+  CK(md_lj_multi(c, plan, dtv, dtf, m, every, check));
+  c->bar_set ^= 1;
+  return B200_OK;
+}
+
 // Launch-shape search of a box that steps through the one-launch step kernel
 // (md_lj_step / md_eam_step): the step kernel itself is timed, for 1, 2, 4
 // and 8 threads per atom, since its best shape can differ from the two-kernel
@@ -541,16 +559,25 @@ int autotune_step(b200_ctx *c) {
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   const int cand[4] = {1, 2, 4, 8};
+  // eight lanes never win on a box that fills the chip many times over
+  const int ncand = c->n >= 200000 ? 3 : 4;
   float tmin[4] = {1e30f, 1e30f, 1e30f, 1e30f};
   auto step = [&]() -> cudaError_t {
     cudaError_t e = lj ? md_lj_step(c, 0.0, 0.0, false) : md_eam_step(c, 0.0, 0.0, false);
     md_swap_positions(c);
     return e;
   };
-  // one timed block of `reps` steps at the current shape
+  // one timed block of `reps` steps at the current shape, in the form the
+  // run will use at it: one launch of several steps, or a launch each
   auto block = [&](int reps, float &ms) -> cudaError_t {
+    const MultiPlan plan = c->use_graphs ? md_lj_multi_plan(c) : MultiPlan();
     cudaError_t e = cudaEventRecord(e0, c->stream);
-    for (int r = 0; r < reps && e == cudaSuccess; r++) e = step();
+    if (plan.blocks > 0 && e == cudaSuccess) {
+      if (launch_multi(c, plan, reps, 0, 0.0, 0.0, 1 << 30, 0)) e = cudaErrorLaunchFailure;
+      else if (reps & 1) md_swap_positions(c);
+    } else {
+      for (int r = 0; r < reps && e == cudaSuccess; r++) e = step();
+    }
     if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
     if (e == cudaSuccess) e = cudaEventSynchronize(e1);
     if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
@@ -568,7 +595,7 @@ int autotune_step(b200_ctx *c) {
   if (e == cudaSuccess) reps = std::max(5, std::min(40, (int)ceilf(20.0f / std::max(ms, 1e-3f))));
   else rc = set_err(c, B200_ERR_CUDA, "launch-shape search: %s", cudaGetErrorString(e));
   for (int round = 0; round < 3 && !rc; round++)
-    for (int k = 0; k < 4 && !rc; k++) {
+    for (int k = 0; k < ncand && !rc; k++) {
       c->tpa = cand[k];
       e = step();
       if (e == cudaSuccess) e = block(reps, ms);
@@ -856,7 +883,7 @@ int capture_piece(b200_ctx *c, int kind, double dtv, double dtf) {
 // that takes longer than 0.2 s, read the status word after a stream
 // synchronize instead (which also reports a CUDA error) and take the
 // device's count as the host's.
-int wait_decision(b200_ctx *c, bool *rebuild) {
+int wait_decision(b200_ctx *c, bool *rebuild, int *ago = nullptr) {
   volatile int *m = c->mail_host;
   const int want = (int)c->decisions;
   const auto t0 = std::chrono::steady_clock::now();
@@ -864,6 +891,7 @@ int wait_decision(b200_ctx *c, bool *rebuild) {
     if (m[1] == want) {
       std::atomic_thread_fence(std::memory_order_acquire);
       *rebuild = m[0] != 0;
+      if (ago) *ago = m[2];
       return B200_OK;
     }
     if ((it & 4095u) == 0u &&
@@ -871,11 +899,33 @@ int wait_decision(b200_ctx *c, bool *rebuild) {
       break;
   }
   int dc = 0;
-  int rc1 = small_read(c, &c->status_host[ST_REBUILD], c->status + ST_REBUILD, sizeof(int));
+  int rc1 = read_status(c);
   if (!rc1) rc1 = small_read(c, &dc, c->dec_count, sizeof(int));
   if (rc1) return rc1;
+  if (c->status_host[ST_BARRIER]) return status_errors(c);
   c->decisions = (unsigned int)dc;
   *rebuild = c->status_host[ST_REBUILD] != 0;
+  if (ago) *ago = c->status_host[ST_AGO];
+  return B200_OK;
+}
+
+// `nsteps` fused non-output steps in one launch; with the distance criterion
+// it may end early.  *done: steps run; *rebuild: the decision for the step
+// after them.
+int run_multi(b200_ctx *c, const MultiPlan &plan, int nsteps, int ago, double dtv, double dtf,
+              int *done, bool *rebuild) {
+  int rc = launch_multi(c, plan, nsteps, ago, dtv, dtf, c->every, c->check);
+  if (rc) return rc;
+  *done = nsteps;
+  *rebuild = false;
+  if (c->check) {
+    int now = ago + nsteps;
+    c->decisions++;
+    rc = wait_decision(c, rebuild, &now);
+    if (rc) return rc;
+    *done = now - ago;
+  }
+  if (*done & 1) md_swap_positions(c);
   return B200_OK;
 }
 
@@ -1026,6 +1076,8 @@ int b200_create(int device, int precision, b200_ctx **out) {
   }
   if (e == cudaSuccess) e = cudaHostAlloc((void **)&c->bounce_host, kBounceBytes, cudaHostAllocMapped);
   if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&c->bounce_dev, c->bounce_host, 0);
+  if (e == cudaSuccess) e = cudaMalloc((void **)&c->bar, 2 * MD_BAR_WORDS * sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMemset(c->bar, 0, 2 * MD_BAR_WORDS * sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMalloc((void **)&c->dec_count, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(c->dec_count, 0, sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc((void **)&c->ev, 8 * sizeof(double));
@@ -1082,6 +1134,7 @@ int b200_destroy(b200_ctx *c) {
   if (c->mail_host) cudaFreeHost(c->mail_host);
   if (c->bounce_host) cudaFreeHost(c->bounce_host);
   dfree(c->dec_count);
+  dfree(c->bar);
   if (c->s_aux) cudaStreamDestroy(c->s_aux);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
@@ -1236,7 +1289,7 @@ int b200_set_eam(b200_ctx *c, int ntypes, int nrho, double drho, int nr, double 
   if (rc) return rc;
   if (ntypes == 1) {
     // one element: the z2 value and rho' coefficients of each knot in one
-    // 32-byte record for the mixed force kernel
+    // record for the force kernels (64 bytes, or 32 in the mixed form)
     const size_t ri = (size_t)E.type2rhor[ntp1 + 1], zi = (size_t)E.type2z2r[ntp1 + 1];
     std::vector<double> fz((size_t)(nr + 1) * 8, 0.0);
     for (size_t m = 0; m <= (size_t)nr; m++) {
@@ -1295,6 +1348,7 @@ int b200_upload_atoms(b200_ctx *c, int n, const double *x, const double *v, cons
     CK(dalloc(&c->rho, stride));
     CK(dalloc(&c->fp, stride));
     CK(dalloc(&c->fpf, stride));
+    CK(dalloc(&c->xf, stride));
     CK(dalloc(&c->slot, stride));
     CK(dalloc(&c->perm, stride));
     CK(dalloc(&c->cell_tmp, stride));
@@ -1346,7 +1400,6 @@ int b200_upload_atoms(b200_ctx *c, int n, const double *x, const double *v, cons
   c->sorted_once = false;
   return B200_OK;
 }
-    CK(dalloc(&c->xf, stride));
 
 int b200_natoms(const b200_ctx *c) { return c ? c->n : 0; }
 
@@ -1790,6 +1843,8 @@ int b200_run(b200_ctx *c, int nsteps, double dt, double ftm2v, int thermo_every,
     int rc = ensure_graphs(c, dtv, dtf, ftm2v);
     if (rc) return rc;
   }
+  CK(cudaMemsetAsync(c->bar, 0, 2 * MD_BAR_WORDS * sizeof(unsigned), c->stream));
+  CK(cudaMemsetAsync(c->status + ST_BARRIER, 0, sizeof(int), c->stream));
   CK(cudaMemsetAsync(c->status + ST_ROW, 0, sizeof(int), c->stream));
   CK(cudaMemsetAsync(c->status + ST_OVERFLOW, 0, sizeof(int), c->stream));
   CK(cudaMemsetAsync(c->status + ST_MAXNEIGH, 0, sizeof(int), c->stream));
@@ -1836,6 +1891,10 @@ int b200_run(b200_ctx *c, int nsteps, double dt, double ftm2v, int thermo_every,
     // starts with its own initial half-step, so snapshots and replays see
     // whole steps.
     bool pre_done = false;
+    // the decision of the coming step, when a multi-step launch has posted it
+    bool told = false, told_rebuild = false;
+    const MultiPlan multi = c->timing || c->timing_pieces || !c->use_graphs ? MultiPlan()
+                                                                           : md_lj_multi_plan(c);
     if (c->timing_pieces) std::fill(piece_kind.begin(), piece_kind.end(), (signed char)-1);
     for (long long t = s; t <= s_end; t++) {
       cudaEvent_t *ev = c->timing ? &c->ev_pool[(size_t)(t - s) * (MD_NPHASE + 1)] : nullptr;
@@ -1863,17 +1922,40 @@ int b200_run(b200_ctx *c, int nsteps, double dt, double ftm2v, int thermo_every,
         } else {
           // distance criterion: the decision the device just made (it
           // posts to the mailbox exactly on these steps)
-          c->decisions++;
-          rc = wait_decision(c, &rebuild);
-          if (rc) return rc;
+          if (told) {
+            rebuild = told_rebuild;
+          } else {
+            c->decisions++;
+            rc = wait_decision(c, &rebuild);
+            if (rc) return rc;
+          }
         }
       }
+      told = false;
       if (rebuild) {
         rc = piece(1, PIECE_REBUILD, nullptr);
         if (rc) return rc;
         ago = 0;
       }
       const bool fuse = !c->timing && t < s_end;
+      if (multi.blocks > 0 && fuse && !is_out(t)) {
+        // the fused steps up to the next output step, the chunk's last step
+        // or, without the distance criterion, the next rebuild
+        int k = 1;
+        while (t + k < s_end && !is_out(t + k) &&
+               (c->check || ago + k < c->delay || (ago + k) % c->every != 0))
+          k++;
+        if (k > 1) {
+          int done = 0;
+          rc = run_multi(c, multi, k, ago, dtv, dtf, &done, &told_rebuild);
+          if (rc) return rc;
+          told = c->check != 0;
+          ago += done - 1;
+          t += done - 1;
+          pre_done = true;
+          continue;
+        }
+      }
       const int post = fuse ? (is_out(t) ? PIECE_FUSED_OUT : PIECE_FUSED)
                             : (is_out(t) ? PIECE_POST_OUT : PIECE_POST);
       rc = piece(2, post, ev ? ev + 2 : nullptr);

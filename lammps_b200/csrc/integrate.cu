@@ -221,6 +221,29 @@ cudaError_t md_ke(b200_ctx *c) {
   return cudaGetLastError();
 }
 
+int md_sms(const b200_ctx *c) {
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) {
+    cudaGetLastError();
+    return 1;
+  }
+  return sms;
+}
+
+int md_coop_blocks(const b200_ctx *c, const void *k, int threads, size_t smem, int groups) {
+  int per_sm = 0;
+  cudaError_t e = cudaSuccess;
+  if (smem > 48 * 1024)
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return groups <= per_sm * md_sms(c) ? groups : 0;
+}
+
 cudaError_t md_decide(b200_ctx *c) {
   k_decide<<<1, 1, 0, c->stream>>>(c->status, c->every, c->delay, c->check, c->dec_count,
                                    c->mail_dev);

@@ -42,6 +42,7 @@ enum {
   ST_MAXSTAGE = 12,     // most shared memory (16-byte units) one builder tile needed
   ST_HALO_BAD = 13,     // a halo pack/unpack index was outside [0, n)
   ST_BADTYPE = 14,      // 1 + index of an uploaded atom with a type outside [1, ntypes]
+  ST_BARRIER = 15,      // a grid barrier of a multi-step launch gave up
   ST_COUNT = 16
 };
 
@@ -197,7 +198,6 @@ __device__ __forceinline__ float rcp_approx_f32(float x) {
   return y;
 }
 
-// FP64 helpers that keep a*b+c rounded twice, as the reference's x86-64
 // Position loads of the pair loops.  A kernel that runs several steps reads
 // positions that other blocks wrote earlier in the same launch: COH makes
 // them plain loads (ordered by the grid barrier) instead of read-only ones.
@@ -223,6 +223,7 @@ __device__ __forceinline__ double4 ld_pos(const double4 *p) {
   return v;
 }
 
+// FP64 helpers that keep a*b+c rounded twice, as the reference's x86-64
 // build computes them; used wherever a comparison must be bit-exact.
 __device__ __forceinline__ double dsq3(double a, double b, double c) {
   return __dadd_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)), __dmul_rn(c, c));
@@ -493,6 +494,81 @@ __device__ __forceinline__ bool md_nve_fused_atom(int i, int stride, double dtv,
                                                   double triggersq, double &ke) {
   return md_nve_step_atom<KE>(i, stride, dtv, dtf, mass, x4, x4, v, f[i], f[stride + i],
                               f[2 * stride + i], xq, box, xhold, triggersq, ke);
+}
+
+// ---- several MD steps in one launch (k_lj_multi, k_eam_multi) ---------------
+
+// Barrier of all co-resident blocks of a cooperative launch, with the OR of
+// `flag` over their threads.  `slot` is a zeroed word used once: arrivals in
+// the low half, blocks with the flag in the high half, so the word that
+// completes the barrier also carries the result.  wait = false: arrive only.
+// After about a second (kBarrierPolls) it gives up and returns -1, which ends
+// the block; the host finds ST_BARRIER set.
+constexpr unsigned kBarrierPolls = 1u << 22;
+__device__ __forceinline__ int md_grid_barrier(unsigned *slot, bool flag, bool wait, int *status) {
+  __shared__ int s_or;
+  const int any = __syncthreads_or(flag ? 1 : 0);
+  if (threadIdx.x == 0) {
+    const unsigned add = any ? 0x10001u : 1u;
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(slot), "r"(add) : "memory");
+    int r = any;
+    if (wait) {
+      unsigned v = 0, polls = 0;
+      do {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(slot) : "memory");
+      } while ((v & 0xffffu) != gridDim.x && ++polls < kBarrierPolls);
+      r = (v >> 16) != 0u;
+      if ((v & 0xffffu) != gridDim.x) {
+        atomicExch(&status[ST_BARRIER], 1);
+        r = -1;
+      }
+    }
+    s_or = r;
+  }
+  __syncthreads();
+  return s_or;
+}
+
+// What a launch of several steps needs beside StepArgs.  Host and device
+// agree on `ago` (steps since the last build, at the launch).
+struct MultiArgs {
+  int nsteps;      // steps to run unless the distance criterion wants a rebuild before
+  int ago;
+  unsigned *bar;   // barrier words of this launch, zeroed
+  unsigned *bar_next;  // words of the next launch, zeroed by this one
+  int bar_words;
+  int slots;           // list entries per thread kept in shared memory
+};
+// words of one launch: two barriers a step, at most a run chunk's steps
+#define MD_BAR_WORDS 512
+
+// The schedule after step j of the launch (0-based): Neighbor::decide for the
+// step that follows (src/neighbor.cpp:1294-1309).
+__device__ __forceinline__ bool md_candidate(int every, int delay, int ago) {
+  return ago >= delay && ago % every == 0;
+}
+
+// The end of a launch of `done` steps, by one thread: the counters that
+// md_decide_dev would have advanced step by step, and with the distance
+// criterion the mailbox post (flag, steps since the build, count).
+__device__ __forceinline__ void md_multi_end(int *status, int done, int ago, bool rebuild,
+                                             int every, int delay, int check, int *dcount,
+                                             volatile int *mail) {
+  status[ST_AGO] = ago;
+  status[ST_MOVED] = 0;
+  status[ST_REBUILD] = rebuild ? 1 : 0;
+  const unsigned lo = (unsigned)status[ST_STEP_LO], now = lo + (unsigned)done;
+  if (now < lo) status[ST_STEP_HI] += 1;
+  status[ST_STEP_LO] = (int)now;
+  if (check) {
+    if (rebuild && ago == (every > delay ? every : delay)) status[ST_NDANGER] += 1;
+    const int k = *dcount + 1;
+    *dcount = k;
+    mail[0] = rebuild ? 1 : 0;
+    mail[2] = ago;
+    __threadfence_system();
+    mail[1] = k;
+  }
 }
 
 // ---- one-launch MD steps (k_lj_step, k_eam_force with STEP) ---------------

@@ -184,6 +184,9 @@ struct b200_ctx {
   int *bounce_host = nullptr, *bounce_dev = nullptr;
   int *dec_count = nullptr;
   unsigned int decisions = 0;
+  // barrier words of multi-step launches, two sets used in turn
+  unsigned *bar = nullptr;
+  int bar_set = 0;
   double *rows = nullptr;        // device thermo rows (9 doubles each)
   int rows_cap = 0;
 
@@ -283,6 +286,20 @@ cudaError_t md_rep_step(b200_ctx *c, double dtv, double dtf);
 bool md_lj_step_ok(const b200_ctx *c);
 cudaError_t md_lj_step(b200_ctx *c, double dtv, double dtf, bool out);
 void md_swap_positions(b200_ctx *c);
+// several such steps in one cooperative launch (non-output steps)
+struct MultiPlan {
+  const void *kernel = nullptr;
+  int blocks = 0;  // 0: the context does not run in this form
+  int threads = 0, slots = 0;
+  size_t smem = 0;
+};
+MultiPlan md_lj_multi_plan(const b200_ctx *c);
+cudaError_t md_lj_multi(b200_ctx *c, const MultiPlan &p, double dtv, double dtf, MultiArgs m,
+                        int every, int check);
+int md_sms(const b200_ctx *c);
+// blocks of a cooperative launch of kernel k for `groups` blocks' worth of
+// atoms, or 0 when they are not all resident at once
+int md_coop_blocks(const b200_ctx *c, const void *k, int threads, size_t smem, int groups);
 // the same for eam: the density pass, then the force pass with the half-steps
 bool md_eam_step_ok(const b200_ctx *c);
 cudaError_t md_eam_step(b200_ctx *c, double dtv, double dtf, bool out);
