@@ -524,8 +524,12 @@ int rebuild_sync(b200_ctx *c) {
 }
 
 // `nsteps` MD steps in one launch
-// (md_lj_multi), from `ago` steps since the build, under the given schedule;
+// (md_lj_multi, md_eam_multi), from `ago` steps since the build, under the given schedule;
 // the barrier words' other set becomes current
+MultiPlan multi_plan(const b200_ctx *c) {
+  return c->pstyle == B200_PAIR_LJ_CUT ? md_lj_multi_plan(c) : md_eam_multi_plan(c);
+}
+
 int launch_multi(b200_ctx *c, const MultiPlan &plan, int nsteps, int ago, double dtv, double dtf, int every,
                  int check) {
   MultiArgs m;
@@ -534,7 +538,8 @@ int launch_multi(b200_ctx *c, const MultiPlan &plan, int nsteps, int ago, double
   m.bar = c->bar + c->bar_set * MD_BAR_WORDS;
   m.bar_next = c->bar + (c->bar_set ^ 1) * MD_BAR_WORDS;
   m.bar_words = MD_BAR_WORDS;
-  CK(md_lj_multi(c, plan, dtv, dtf, m, every, check));
+  CK(c->pstyle == B200_PAIR_LJ_CUT ? md_lj_multi(c, plan, dtv, dtf, m, every, check)
+                                   : md_eam_multi(c, plan, dtv, dtf, m, every, check));
   c->bar_set ^= 1;
   return B200_OK;
 }
@@ -570,7 +575,7 @@ int autotune_step(b200_ctx *c) {
   // one timed block of `reps` steps at the current shape, in the form the
   // run will use at it: one launch of several steps, or a launch each
   auto block = [&](int reps, float &ms) -> cudaError_t {
-    const MultiPlan plan = c->use_graphs ? md_lj_multi_plan(c) : MultiPlan();
+    const MultiPlan plan = c->use_graphs ? multi_plan(c) : MultiPlan();
     cudaError_t e = cudaEventRecord(e0, c->stream);
     if (plan.blocks > 0 && e == cudaSuccess) {
       if (launch_multi(c, plan, reps, 0, 0.0, 0.0, 1 << 30, 0)) e = cudaErrorLaunchFailure;
@@ -1894,7 +1899,7 @@ int b200_run(b200_ctx *c, int nsteps, double dt, double ftm2v, int thermo_every,
     // the decision of the coming step, when a multi-step launch has posted it
     bool told = false, told_rebuild = false;
     const MultiPlan multi = c->timing || c->timing_pieces || !c->use_graphs ? MultiPlan()
-                                                                           : md_lj_multi_plan(c);
+                                                                           : multi_plan(c);
     if (c->timing_pieces) std::fill(piece_kind.begin(), piece_kind.end(), (signed char)-1);
     for (long long t = s; t <= s_end; t++) {
       cudaEvent_t *ev = c->timing ? &c->ev_pool[(size_t)(t - s) * (MD_NPHASE + 1)] : nullptr;

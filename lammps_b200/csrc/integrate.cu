@@ -230,18 +230,37 @@ int md_sms(const b200_ctx *c) {
   return sms;
 }
 
-int md_coop_blocks(const b200_ctx *c, const void *k, int threads, size_t smem, int groups) {
-  int per_sm = 0;
+// The multi-step launch at the current threads per atom; blocks 0 when the box
+// does not run in that form: all of its atoms must be resident at once.  Up to
+// two blocks per SM a thread may use 128 registers and gathers two groups of
+// neighbours at once (kernel `deep`); above, 64 and one (`lean`).
+MultiPlan md_multi_shape(const b200_ctx *c, const void *lean, const void *deep) {
+  MultiPlan p;
+  const int sms = md_sms(c);
+  const int groups = md_blocks((long long)c->n * c->tpa, kMultiThreads);
+  const int per_sm = (groups + sms - 1) / sms;
+  if (per_sm > 4) return p;  // launch bounds of the lean form
+  p.kernel = per_sm <= 2 ? deep : lean;
+  p.threads = kMultiThreads;
+  // list entries kept per thread: the mean and some more, as far as they fit
+  const double rc = c->cutneighmax, vol = c->box.prd[0] * c->box.prd[1] * c->box.prd[2];
+  const double mean = 4.18879 * rc * rc * rc * c->n / vol;
+  const size_t most = (size_t)216 * 1024 / per_sm - 7 * 1024;
+  p.slots = (int)(1.25 * mean / c->tpa) + 4;
+  while (p.slots > 0 && md_multi_smem(c->tpa, p.slots) > most) p.slots--;
+  p.smem = md_multi_smem(c->tpa, p.slots);
+  int fit = 0;
   cudaError_t e = cudaSuccess;
-  if (smem > 48 * 1024)
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (p.smem > 40 * 1024)
+    e = cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
   if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, p.kernel, p.threads, p.smem);
   if (e != cudaSuccess) {
     cudaGetLastError();
-    return 0;
+    return MultiPlan();
   }
-  return groups <= per_sm * md_sms(c) ? groups : 0;
+  if (groups <= fit * sms) p.blocks = groups;
+  return p;
 }
 
 cudaError_t md_decide(b200_ctx *c) {

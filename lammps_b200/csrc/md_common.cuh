@@ -669,3 +669,131 @@ __device__ __forceinline__ void md_step_tail(const StepArgs &s, bool moved, cons
     *counter = 0u;
   }
 }
+
+// ---- pieces of the multi-step kernels ---------------------------------------
+
+constexpr int kMultiThreads = 256;
+// doubles of an atom's state: x, y, z, v, dtf / mass, x, y, z at the last build
+constexpr int kMultiState = 10;
+inline size_t md_multi_smem(int tpa, int slots) {
+  return (size_t)kMultiState * (kMultiThreads / tpa) * sizeof(double) +
+         (size_t)slots * kMultiThreads * sizeof(int);
+}
+
+// a value of the atom's first lane to all its lanes
+template <int TPA, class T>
+__device__ __forceinline__ T from_first(T v) {
+  return TPA == 1 ? v : __shfl_sync(0xffffffffu, v, 0, TPA);
+}
+
+// loads of data that other blocks wrote earlier in the launch
+__device__ __forceinline__ double ld_plain(const double *p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_plain(const float *p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+
+// This lane's entries (lane, lane + TPA, ... of the atom's list), the first
+// `slots` of them in shared memory.
+template <int TPA>
+struct MultiList {
+  const int *nlist;
+  int *mine;
+  int stride, i, lane, slots, cnt;
+  __device__ __forceinline__ MultiList(const int *nl, int stride_, int i_, int num, int lane_,
+                                       int slots_, int *s_list)
+      : nlist(nl), mine(s_list + threadIdx.x), stride(stride_), i(i_), lane(lane_), slots(slots_),
+        cnt(num > lane_ ? (num - lane_ + TPA - 1) / TPA : 0) {
+    for (int k = 0; k < cnt && k < slots; k++) mine[k * kMultiThreads] = fetch(k);
+  }
+  __device__ __forceinline__ int fetch(int k) const {
+    return nlist[md_slab(lane + TPA * k, i, stride)];
+  }
+  __device__ __forceinline__ unsigned entry(int k) const {
+    return (unsigned)(k < slots ? mine[k * kMultiThreads] : fetch(k));
+  }
+};
+
+// The atom's state in shared memory (field k at p[k * AB]), used by its first
+// lane.
+template <int TPA>
+struct MultiState {
+  static constexpr int AB = kMultiThreads / TPA;
+  double *p;
+  __device__ __forceinline__ explicit MultiState(double *s_state)
+      : p(s_state + threadIdx.x / TPA) {}
+  __device__ __forceinline__ void load(const StepArgs &s, int i, int stride, const double4 &x) {
+    p[0] = x.x;
+    p[AB] = x.y;
+    p[2 * AB] = x.z;
+    p[3 * AB] = s.v[i];
+    p[4 * AB] = s.v[stride + i];
+    p[5 * AB] = s.v[2 * stride + i];
+    p[6 * AB] = s.dtf / s.mass[(int)x.w];
+    if (s.xhold) {
+      const double4 h = s.xhold[i];
+      p[7 * AB] = h.x;
+      p[8 * AB] = h.y;
+      p[9 * AB] = h.z;
+    }
+  }
+  // final half-step of this step, initial half-step of the next (the rounded
+  // operations of md_nve_step_atom); the new position, with type w
+  __device__ __forceinline__ double4 step(const StepArgs &s, double fx, double fy, double fz,
+                                          double w, bool &moved) {
+    const double dtfm = p[6 * AB];
+    double vx = __dadd_rn(p[3 * AB], __dmul_rn(dtfm, fx));
+    double vy = __dadd_rn(p[4 * AB], __dmul_rn(dtfm, fy));
+    double vz = __dadd_rn(p[5 * AB], __dmul_rn(dtfm, fz));
+    vx = __dadd_rn(vx, __dmul_rn(dtfm, fx));
+    vy = __dadd_rn(vy, __dmul_rn(dtfm, fy));
+    vz = __dadd_rn(vz, __dmul_rn(dtfm, fz));
+    const double4 x = make_double4(__dadd_rn(p[0], __dmul_rn(s.dtv, vx)),
+                                   __dadd_rn(p[AB], __dmul_rn(s.dtv, vy)),
+                                   __dadd_rn(p[2 * AB], __dmul_rn(s.dtv, vz)), w);
+    p[0] = x.x;
+    p[AB] = x.y;
+    p[2 * AB] = x.z;
+    p[3 * AB] = vx;
+    p[4 * AB] = vy;
+    p[5 * AB] = vz;
+    moved = s.xhold && dsq3(__dsub_rn(x.x, p[7 * AB]), __dsub_rn(x.y, p[8 * AB]),
+                            __dsub_rn(x.z, p[9 * AB])) > s.triggersq;
+    return x;
+  }
+  // back to memory; the FP64 positions only in the mixed form (the FP64 form
+  // wrote them to the position buffers)
+  __device__ __forceinline__ void store(const StepArgs &s, int i, int stride, bool mixed,
+                                        double w) const {
+    if (mixed) s.x4[i] = make_double4(p[0], p[AB], p[2 * AB], w);
+    s.v[i] = p[3 * AB];
+    s.v[stride + i] = p[4 * AB];
+    s.v[2 * stride + i] = p[5 * AB];
+  }
+};
+
+// After step j of a launch (every thread of the block): advances `ago`, waits
+// for the other blocks' positions and returns 1 to go on, 0 at the end of the
+// launch (block 0 has posted it), -1 when the barrier gave up.
+__device__ __forceinline__ int md_multi_next(const StepArgs &s, const MultiArgs &m, int j, int word,
+                                             int &ago, bool moved) {
+  ago++;
+  const bool last = j + 1 == m.nsteps;
+  const bool cand = md_candidate(s.every, s.delay, ago);
+  bool rebuild = !s.check && cand;
+  if (!last || (s.check && cand)) {
+    // after the last step only the block that posts the decision waits
+    const int r = md_grid_barrier(m.bar + word, moved, !last || blockIdx.x == 0, s.status);
+    if (r < 0) return -1;
+    if (s.check && cand) rebuild = r != 0;
+  }
+  if (!last && !rebuild) return 1;
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    md_multi_end(s.status, j + 1, ago, rebuild, s.every, s.delay, s.check, s.dcount, s.mail);
+  return 0;
+}

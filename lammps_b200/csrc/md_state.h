@@ -296,10 +296,12 @@ struct MultiPlan {
 MultiPlan md_lj_multi_plan(const b200_ctx *c);
 cudaError_t md_lj_multi(b200_ctx *c, const MultiPlan &p, double dtv, double dtf, MultiArgs m,
                         int every, int check);
+MultiPlan md_eam_multi_plan(const b200_ctx *c);
+cudaError_t md_eam_multi(b200_ctx *c, const MultiPlan &p, double dtv, double dtf, MultiArgs m,
+                         int every, int check);
+MultiPlan md_multi_shape(const b200_ctx *c, const void *lean, const void *deep);
 int md_sms(const b200_ctx *c);
-// blocks of a cooperative launch of kernel k for `groups` blocks' worth of
-// atoms, or 0 when they are not all resident at once
-int md_coop_blocks(const b200_ctx *c, const void *k, int threads, size_t smem, int groups);
+StepArgs md_step_args(b200_ctx *c, double dtv, double dtf);
 // the same for eam: the density pass, then the force pass with the half-steps
 bool md_eam_step_ok(const b200_ctx *c);
 cudaError_t md_eam_step(b200_ctx *c, double dtv, double dtf, bool out);

@@ -102,6 +102,247 @@ __device__ __forceinline__ void embed(const EamArgs &a, int itype_frho, double r
   if (rho > a.rhomax) phi += fp * (rho - a.rhomax);
 }
 
+// Atom i's side of its pairs: FP64 position and periodic shifts, or
+// fixed-point position and unit lengths.
+template <bool MIXED, bool SINGLE>
+struct EamSide {
+  double4 xi;
+  int4 qi;
+  int ti;
+  Shift3 sx, sy, sz;
+  float qx, qy, qz, qxl, qyl, qzl;
+  __device__ __forceinline__ void init(const EamArgs &a, int cell) {
+    if (MIXED) {
+      qx = a.box.qs[0], qy = a.box.qs[1], qz = a.box.qs[2];
+      qxl = a.box.qs_lo[0], qyl = a.box.qs_lo[1], qzl = a.box.qs_lo[2];
+    } else {
+      int cx, cy, cz;
+      md_cell_unpack(cell, cx, cy, cz);
+      sx = shifts(cx, a.box.ncell[0], a.box.prd[0]);
+      sy = shifts(cy, a.box.ncell[1], a.box.prd[1]);
+      sz = shifts(cz, a.box.ncell[2], a.box.prd[2]);
+    }
+  }
+  // FP64 separation of entry e at xj
+  __device__ __forceinline__ void sep(unsigned e, const double4 &xj, double &delx, double &dely,
+                                      double &delz) const {
+    int j, dx, dy, dz;
+    decode(e, j, dx, dy, dz);
+    delx = __dsub_rn(xi.x, __dadd_rn(xj.x, pick(sx, dx)));
+    dely = __dsub_rn(xi.y, __dadd_rn(xj.y, pick(sy, dy)));
+    delz = __dsub_rn(xi.z, __dadd_rn(xj.z, pick(sz, dz)));
+  }
+  // minimum-image separation from the fixed-point coordinates
+  __device__ __forceinline__ void sep(const int4 &xj, float &delx, float &dely,
+                                      float &delz) const {
+    delx = md_qlen(md_qdiff(qi.x, xj.x), qx, qxl);
+    dely = md_qlen(md_qdiff(qi.y, xj.y), qy, qyl);
+    delz = md_qlen(md_qdiff(qi.z, xj.z), qz, qzl);
+  }
+};
+
+// Density terms of four entries ee with their positions; the first mm lie
+// before the atom's count.  Branch-free, so that the four entries' chains and
+// table loads overlap; an entry past mm or past the cutoff reads row 0 (one
+// address for all of them) and adds nothing.
+template <bool SINGLE>
+__device__ __forceinline__ void rho_four(const EamArgs &a, const EamSide<false, SINGLE> &me,
+                                         const int *t2rhor, const unsigned (&ee)[4],
+                                         const double4 (&xj)[4], int mm, double &rho) {
+  // one element: the density spline row of every pair
+  const double *rrow = SINGLE ? a.rhor + (size_t)t2rhor[a.ntp1 + 1] * (a.nr + 1) * 8 : nullptr;
+  double val[4];
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    double delx, dely, delz;
+    me.sep(ee[u], xj[u], delx, dely, delz);
+    const double rsq = dsq3(delx, dely, delz);
+    const bool in = u < mm && rsq < a.cutforcesq;
+    int m;
+    double p;
+    knot_d(__dadd_rn(__dmul_rn(sqrt(in ? rsq : 0.0), a.rdr), 1.0), a.nr - 1, m, p);
+    const double *row =
+        SINGLE ? rrow
+               : a.rhor + (size_t)t2rhor[(int)xj[u].w * a.ntp1 + me.ti] * (a.nr + 1) * 8;
+    // knot layout [c3 c4 c5 c6 | c0 c1 c2 -]: the value coefficients
+    // are one 32-byte load
+    const double4 c = ld_pos<false>(reinterpret_cast<const double4 *>(row + (size_t)m * 8));
+    val[u] = in ? ((c.x * p + c.y) * p + c.z) * p + c.w : 0.0;
+  }
+#pragma unroll
+  for (int u = 0; u < 4; u++) rho += val[u];
+}
+// The same in the mixed form.  Pad entries name the atom itself (zero
+// separation), which the r^2 > 0 test rejects.
+template <bool SINGLE>
+__device__ __forceinline__ void rho_four(const EamArgs &a, const EamSide<true, SINGLE> &me,
+                                         const int *t2rhor, const int4 (&xs)[4], double &rho) {
+  const float cutf = (float)a.cutforcesq, rdrf = (float)a.rdr;
+  const float *rrow = SINGLE ? a.rhor_f + (size_t)t2rhor[a.ntp1 + 1] * (a.nr + 1) * 8 : nullptr;
+  float crho = 0.f;  // FP32 slab sum, added to the FP64 density
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    float delx, dely, delz;
+    me.sep(xs[u], delx, dely, delz);
+    const float rsq = delx * delx + dely * dely + delz * delz;
+    if (rsq < cutf && rsq > 0.f) {
+      int m;
+      float p;
+      knot_f(rsq * rsqrtf(rsq) * rdrf + 1.0f, a.nr - 1, m, p);
+      const float *row = SINGLE ? rrow
+                                : a.rhor_f + (size_t)t2rhor[xs[u].w * a.ntp1 + me.ti] *
+                                                 (a.nr + 1) * 8;
+      const float4 c = __ldg(reinterpret_cast<const float4 *>(row + (size_t)m * 8));
+      crho += ((c.x * p + c.y) * p + c.z) * p + c.w;
+    }
+  }
+  rho += (double)crho;
+}
+
+// Force terms (and, with EV, energy and virial) of four entries; fpq their F'.
+template <bool EV, bool SINGLE>
+__device__ __forceinline__ void force_four(const EamArgs &a, const EamSide<false, SINGLE> &me,
+                                           const int *t2rhor, const int *t2z2r, double fpi,
+                                           const unsigned (&ee)[4], const double4 (&xj)[4],
+                                           const double (&fpq)[4], int mm, double &fx, double &fy,
+                                           double &fz, double (&acc)[7]) {
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+   double delx, dely, delz;
+   me.sep(ee[u], xj[u], delx, dely, delz);
+   const double rsq = dsq3(delx, dely, delz);
+   const bool in = u < mm && rsq < a.cutforcesq;
+   const int tj = SINGLE ? 1 : (int)xj[u].w;
+   const double r = sqrt(in ? rsq : 1.0);
+   int m;
+   double p;
+   knot_d(__dadd_rn(__dmul_rn(r, a.rdr), 1.0), a.nr - 1, m, p);
+   const size_t o8 = in ? (size_t)m * 8 : 0;
+   double rhoip, rhojp, z2, z2p;
+   if (SINGLE) {
+     // one element: the pair value and density derivative of a knot in
+     // one 64-byte record; the pair derivative from the value's
+     // coefficients, (3 c3 p^2 + 2 c4 p + c5) / dr
+     const double4 z = ld_pos<false>(reinterpret_cast<const double4 *>(a.fz + o8));
+     const double4 d = ld_pos<false>(reinterpret_cast<const double4 *>(a.fz + o8 + 4));
+     rhoip = (d.x * p + d.y) * p + d.z;
+     rhojp = rhoip;
+     z2 = ((z.x * p + z.y) * p + z.z) * p + z.w;
+     z2p = (fma(3.0 * z.x, p, 2.0 * z.y) * p + z.z) * a.rdr;
+   } else {
+     // knot layout [c3 c4 c5 c6 | c0 c1 c2 -]
+     const double4 d = ld_pos<false>(reinterpret_cast<const double4 *>(
+         a.rhor + (size_t)t2rhor[me.ti * a.ntp1 + tj] * (a.nr + 1) * 8 + o8 + 4));
+     rhoip = (d.x * p + d.y) * p + d.z;
+     rhojp = rhoip;
+     if (!a.rhor_sym) {
+       const double4 e = ld_pos<false>(reinterpret_cast<const double4 *>(
+           a.rhor + (size_t)t2rhor[tj * a.ntp1 + me.ti] * (a.nr + 1) * 8 + o8 + 4));
+       rhojp = (e.x * p + e.y) * p + e.z;
+     }
+     const double *cz = a.z2r + (size_t)t2z2r[me.ti * a.ntp1 + tj] * (a.nr + 1) * 8 + o8;
+     const double4 z = ld_pos<false>(reinterpret_cast<const double4 *>(cz));
+     const double4 zd = ld_pos<false>(reinterpret_cast<const double4 *>(cz + 4));
+     z2p = (zd.x * p + zd.y) * p + zd.z;
+     z2 = ((z.x * p + z.y) * p + z.z) * p + z.w;
+   }
+   const double recip = rcp_nr(r);
+   const double phi = in ? z2 * recip : 0.0;
+   const double phip = z2p * recip - phi * recip;
+   const double psip = fpi * rhojp + fpq[u] * rhoip + phip;
+   const double fpair = in ? -psip * recip : 0.0;
+   fx += delx * fpair;
+   fy += dely * fpair;
+   fz += delz * fpair;
+   if (EV) {
+     acc[0] += 0.5 * phi;
+     const double hf = 0.5 * fpair;
+     acc[1] += delx * delx * hf;
+     acc[2] += dely * dely * hf;
+     acc[3] += delz * delz * hf;
+     acc[4] += delx * dely * hf;
+     acc[5] += delx * delz * hf;
+     acc[6] += dely * delz * hf;
+   }
+  }
+}
+template <bool EV, bool SINGLE>
+__device__ __forceinline__ void force_four(const EamArgs &a, const EamSide<true, SINGLE> &me,
+                                           const int *t2rhor, const int *t2z2r, float fpi,
+                                           const int4 (&xs)[4], const float (&fpq)[4], double &fx,
+                                           double &fy, double &fz, double (&acc)[7]) {
+  const float cutf = (float)a.cutforcesq, rdrf = (float)a.rdr;
+  // one element: the density-derivative and pair spline rows of every pair
+  const float *drow1 = SINGLE ? a.fz_f + 4 : nullptr;
+  const float *zrow1 = SINGLE ? a.fz_f : nullptr;
+  // FP32 sum of the slab's pair forces, added to the FP64 accumulator
+  float cfx = 0.f, cfy = 0.f, cfz = 0.f;
+  float ce[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // EV: the slab's FP32 sums
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+   float delx, dely, delz;
+   me.sep(xs[u], delx, dely, delz);
+   const float rsq = delx * delx + dely * dely + delz * delz;
+   if (rsq < cutf && rsq > 0.f) {
+     const int tj = SINGLE ? 1 : xs[u].w;
+     const float recip = rsqrtf(rsq);
+     const float r = rsq * recip;
+     int m;
+     float p;
+     knot_f(r * rdrf + 1.0f, a.nr - 1, m, p);
+     const size_t o8 = (size_t)m * 8;
+     const float *drow =
+         SINGLE ? drow1 : a.rhor_f + (size_t)t2rhor[me.ti * a.ntp1 + tj] * (a.nr + 1) * 8 + 4;
+     const float4 ci = __ldg(reinterpret_cast<const float4 *>(drow + o8));
+     const float rhoip = (ci.x * p + ci.y) * p + ci.z;
+     float rhojp = rhoip;
+     if (!SINGLE && !a.rhor_sym) {
+       const float4 cj = __ldg(reinterpret_cast<const float4 *>(
+           a.rhor_f + ((size_t)t2rhor[tj * a.ntp1 + me.ti] * (a.nr + 1) + m) * 8 + 4));
+       rhojp = (cj.x * p + cj.y) * p + cj.z;
+     }
+     const float *zb =
+         (SINGLE ? zrow1 : a.z2r_f + (size_t)t2z2r[me.ti * a.ntp1 + tj] * (a.nr + 1) * 8) + o8;
+     const float4 zv = __ldg(reinterpret_cast<const float4 *>(zb));
+     float z2p;
+     if (SINGLE) {
+       // the z2 derivative from the value coefficients:
+       // (3 c3 p^2 + 2 c4 p + c5) / dr, as PairEAM::interpolate stores it
+       z2p = (fmaf(3.0f * zv.x, p, 2.0f * zv.y) * p + zv.z) * rdrf;
+     } else {
+       const float4 zd = __ldg(reinterpret_cast<const float4 *>(zb + 4));
+       z2p = (zd.x * p + zd.y) * p + zd.z;
+     }
+     const float z2 = ((zv.x * p + zv.y) * p + zv.z) * p + zv.w;
+     const float phi = z2 * recip;
+     const float phip = z2p * recip - phi * recip;
+     const float psip = fpi * rhojp + fpq[u] * rhoip + phip;
+     const float fpair = -psip * recip;
+     cfx += delx * fpair;
+     cfy += dely * fpair;
+     cfz += delz * fpair;
+     if (EV) {
+       ce[0] = fmaf(0.5f, phi, ce[0]);
+       const float hf = 0.5f * fpair;
+       ce[1] = fmaf(delx * delx, hf, ce[1]);
+       ce[2] = fmaf(dely * dely, hf, ce[2]);
+       ce[3] = fmaf(delz * delz, hf, ce[3]);
+       ce[4] = fmaf(delx * dely, hf, ce[4]);
+       ce[5] = fmaf(delx * delz, hf, ce[5]);
+       ce[6] = fmaf(dely * delz, hf, ce[6]);
+     }
+   }
+  }
+  fx += (double)cfx;
+  fy += (double)cfy;
+  fz += (double)cfz;
+  // the energy and virial terms join the FP64 sums once per slab, as the
+  // forces do
+  if (EV)
+#pragma unroll
+    for (int k = 0; k < 7; k++) acc[k] += (double)ce[k];
+}
+
 template <bool MIXED>
 __device__ __forceinline__ void store_xf(double4 *xf, int i, const double4 *x4, const int4 *xq,
                                          double fp) {
@@ -131,91 +372,26 @@ __global__ void __launch_bounds__(128) k_eam_rho(EamArgs a, const double4 *__res
   int ti = 1;
   if (active) {
     const int num = a.numneigh[i];
-    if (!MIXED) {
-      const double4 xi = x4[i];
-      ti = (int)xi.w;
-      int cx, cy, cz;
-      md_cell_unpack(a.cell[i], cx, cy, cz);
-      const Shift3 sx = shifts(cx, a.box.ncell[0], a.box.prd[0]);
-      const Shift3 sy = shifts(cy, a.box.ncell[1], a.box.prd[1]);
-      const Shift3 sz = shifts(cz, a.box.ncell[2], a.box.prd[2]);
-      // one element: the density spline row of every pair
-      const double *rrow =
-          SINGLE ? a.rhor + (size_t)s_t2rhor[a.ntp1 + 1] * (a.nr + 1) * 8 : nullptr;
-      // four entries ee of this lane (walk_list); the first mm lie before the
-      // atom's count
-      auto four = [&](const unsigned (&ee)[4], int mm) {
-        // branch-free, so that the four entries' chains and table loads
-        // overlap; an entry past mm or past the cutoff reads row 0 (one
-        // address for all of them) and adds nothing
+    EamSide<MIXED, SINGLE> me;
+    me.init(a, MIXED ? 0 : a.cell[i]);
+    // four entries ee of this lane (walk_list); the first mm lie before the
+    // atom's count
+    auto four = [&](const unsigned (&ee)[4], int mm) {
+      if constexpr (!MIXED) {
         double4 xj[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) xj[u] = ld_pos<false>(&x4[u < mm ? md_entry_j(ee[u]) : i]);
-        double val[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          int j, dx, dy, dz;
-          decode(ee[u], j, dx, dy, dz);
-          const double delx = __dsub_rn(xi.x, __dadd_rn(xj[u].x, pick(sx, dx)));
-          const double dely = __dsub_rn(xi.y, __dadd_rn(xj[u].y, pick(sy, dy)));
-          const double delz = __dsub_rn(xi.z, __dadd_rn(xj[u].z, pick(sz, dz)));
-          const double rsq = dsq3(delx, dely, delz);
-          const bool in = u < mm && rsq < a.cutforcesq;
-          int m;
-          double p;
-          knot_d(__dadd_rn(__dmul_rn(sqrt(in ? rsq : 0.0), a.rdr), 1.0), a.nr - 1, m, p);
-          const double *row =
-              SINGLE ? rrow
-                     : a.rhor + (size_t)s_t2rhor[(int)xj[u].w * a.ntp1 + ti] * (a.nr + 1) * 8;
-          // knot layout [c3 c4 c5 c6 | c0 c1 c2 -]: the value coefficients
-          // are one 32-byte load
-          const double4 c = ld_pos<false>(reinterpret_cast<const double4 *>(row + (size_t)m * 8));
-          val[u] = in ? ((c.x * p + c.y) * p + c.z) * p + c.w : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) rho += val[u];
-      };
-      walk_list<TPA>(a.nlist, a.stride, i, num, lane, four);
-    } else {
-      const int4 xi = xq[i];
-      ti = xi.w;
-      const float qx = a.box.qs[0], qy = a.box.qs[1], qz = a.box.qs[2];
-      const float qxl = a.box.qs_lo[0], qyl = a.box.qs_lo[1], qzl = a.box.qs_lo[2];
-      const float cutf = (float)a.cutforcesq, rdrf = (float)a.rdr;
-      // one element: the density spline row of every pair
-      const float *rrow =
-          SINGLE ? a.rhor_f + (size_t)s_t2rhor[a.ntp1 + 1] * (a.nr + 1) * 8 : nullptr;
-      // four entries ee of this lane (walk_list)
-      auto four = [&](const unsigned (&ee)[4], int) {
-        // whole slabs: pad entries in the last slab name the atom itself
-        // (zero separation), which the r^2 > 0 test rejects
+        rho_four<SINGLE>(a, me, s_t2rhor, ee, xj, mm, rho);
+      } else {
         int4 xs[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) xs[u] = xq[md_entry_j(ee[u])];
-        float crho = 0.f;  // FP32 slab sum, added to the FP64 density
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int4 xj = xs[u];
-          // minimum-image separation from the fixed-point coordinates
-          const float delx = md_qlen(md_qdiff(xi.x, xj.x), qx, qxl);
-          const float dely = md_qlen(md_qdiff(xi.y, xj.y), qy, qyl);
-          const float delz = md_qlen(md_qdiff(xi.z, xj.z), qz, qzl);
-          const float rsq = delx * delx + dely * dely + delz * delz;
-          if (rsq < cutf && rsq > 0.f) {
-            int m;
-            float p;
-            knot_f(rsq * rsqrtf(rsq) * rdrf + 1.0f, a.nr - 1, m, p);
-            const float *row = SINGLE ? rrow
-                                      : a.rhor_f + (size_t)s_t2rhor[xj.w * a.ntp1 + ti] *
-                                                       (a.nr + 1) * 8;
-            const float4 c = __ldg(reinterpret_cast<const float4 *>(row + (size_t)m * 8));
-            crho += ((c.x * p + c.y) * p + c.z) * p + c.w;
-          }
-        }
-        rho += (double)crho;
-      };
-      walk_list<TPA>(a.nlist, a.stride, i, num, lane, four);
-    }
+        rho_four<SINGLE>(a, me, s_t2rhor, xs, rho);
+      }
+    };
+    if (MIXED) me.qi = xq[i], ti = me.ti = me.qi.w;
+    else me.xi = x4[i], ti = me.ti = (int)me.xi.w;
+    walk_list<TPA>(a.nlist, a.stride, i, num, lane, four);
   }
   rho = lane_sum<TPA>(rho);
   double acc[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -256,185 +432,38 @@ __global__ void __launch_bounds__(128) k_eam_force(EamArgs a, const double4 *__r
   double acc[7] = {0, 0, 0, 0, 0, 0, 0};
   if (active) {
     const int num = a.numneigh[i];
-    if (!MIXED) {
-      const double4 xi = x4[i];
-      const int ti = (int)xi.w;
-      const double fpi = a.fp[i];
-      int cx, cy, cz;
-      md_cell_unpack(a.cell[i], cx, cy, cz);
-      const Shift3 sx = shifts(cx, a.box.ncell[0], a.box.prd[0]);
-      const Shift3 sy = shifts(cy, a.box.ncell[1], a.box.prd[1]);
-      const Shift3 sz = shifts(cz, a.box.ncell[2], a.box.prd[2]);
-      // four entries ee of this lane (walk_list); the first mm lie before the
-      // atom's count
-      auto four = [&](const unsigned (&ee)[4], int mm) {
-       // branch-free as the density pass
-       double4 xj[4];
-       double fpq[4];
+    EamSide<MIXED, SINGLE> me;
+    me.init(a, MIXED ? 0 : a.cell[i]);
+    if (MIXED) me.qi = xq[i], me.ti = me.qi.w;
+    else me.xi = x4[i], me.ti = (int)me.xi.w;
+    const double fpd = MIXED ? 0.0 : a.fp[i];
+    const float fpf = MIXED ? a.fpf[i] : 0.f;
+    // four entries ee of this lane (walk_list); the first mm lie before the
+    // atom's count
+    auto four = [&](const unsigned (&ee)[4], int mm) {
+      if constexpr (!MIXED) {
+        double4 xj[4];
+        double fpq[4];
 #pragma unroll
-       for (int u = 0; u < 4; u++) {
-         const int jj = u < mm ? md_entry_j(ee[u]) : i;
-         xj[u] = ld_pos<false>(&(SINGLE ? a.xf : x4)[jj]);
-         fpq[u] = SINGLE ? xj[u].w : a.fp[jj];
-       }
-#pragma unroll
-       for (int u = 0; u < 4; u++) {
-        int j, dx, dy, dz;
-        decode(ee[u], j, dx, dy, dz);
-        const double delx = __dsub_rn(xi.x, __dadd_rn(xj[u].x, pick(sx, dx)));
-        const double dely = __dsub_rn(xi.y, __dadd_rn(xj[u].y, pick(sy, dy)));
-        const double delz = __dsub_rn(xi.z, __dadd_rn(xj[u].z, pick(sz, dz)));
-        const double rsq = dsq3(delx, dely, delz);
-        const bool in = u < mm && rsq < a.cutforcesq;
-        const int tj = SINGLE ? 1 : (int)xj[u].w;
-        const double r = sqrt(in ? rsq : 1.0);
-        int m;
-        double p;
-        knot_d(__dadd_rn(__dmul_rn(r, a.rdr), 1.0), a.nr - 1, m, p);
-        const size_t o8 = in ? (size_t)m * 8 : 0;
-        double rhoip, rhojp, z2, z2p;
-        if (SINGLE) {
-          // one element: the pair value and density derivative of a knot in
-          // one 64-byte record; the pair derivative from the value's
-          // coefficients, (3 c3 p^2 + 2 c4 p + c5) / dr
-          const double4 z = ld_pos<false>(reinterpret_cast<const double4 *>(a.fz + o8));
-          const double4 d = ld_pos<false>(reinterpret_cast<const double4 *>(a.fz + o8 + 4));
-          rhoip = (d.x * p + d.y) * p + d.z;
-          rhojp = rhoip;
-          z2 = ((z.x * p + z.y) * p + z.z) * p + z.w;
-          z2p = (fma(3.0 * z.x, p, 2.0 * z.y) * p + z.z) * a.rdr;
-        } else {
-          // knot layout [c3 c4 c5 c6 | c0 c1 c2 -]
-          const double4 d = ld_pos<false>(reinterpret_cast<const double4 *>(
-              a.rhor + (size_t)s_t2rhor[ti * a.ntp1 + tj] * (a.nr + 1) * 8 + o8 + 4));
-          rhoip = (d.x * p + d.y) * p + d.z;
-          rhojp = rhoip;
-          if (!a.rhor_sym) {
-            const double4 e = ld_pos<false>(reinterpret_cast<const double4 *>(
-                a.rhor + (size_t)s_t2rhor[tj * a.ntp1 + ti] * (a.nr + 1) * 8 + o8 + 4));
-            rhojp = (e.x * p + e.y) * p + e.z;
-          }
-          const double *cz = a.z2r + (size_t)s_t2z2r[ti * a.ntp1 + tj] * (a.nr + 1) * 8 + o8;
-          const double4 z = ld_pos<false>(reinterpret_cast<const double4 *>(cz));
-          const double4 zd = ld_pos<false>(reinterpret_cast<const double4 *>(cz + 4));
-          z2p = (zd.x * p + zd.y) * p + zd.z;
-          z2 = ((z.x * p + z.y) * p + z.z) * p + z.w;
+        for (int u = 0; u < 4; u++) {
+          const int jj = u < mm ? md_entry_j(ee[u]) : i;
+          xj[u] = ld_pos<false>(&(SINGLE ? a.xf : x4)[jj]);
+          fpq[u] = SINGLE ? xj[u].w : a.fp[jj];
         }
-        const double recip = rcp_nr(r);
-        const double phi = in ? z2 * recip : 0.0;
-        const double phip = z2p * recip - phi * recip;
-        const double psip = fpi * rhojp + fpq[u] * rhoip + phip;
-        const double fpair = in ? -psip * recip : 0.0;
-        fx += delx * fpair;
-        fy += dely * fpair;
-        fz += delz * fpair;
-        if (EV) {
-          acc[0] += 0.5 * phi;
-          const double hf = 0.5 * fpair;
-          acc[1] += delx * delx * hf;
-          acc[2] += dely * dely * hf;
-          acc[3] += delz * delz * hf;
-          acc[4] += delx * dely * hf;
-          acc[5] += delx * delz * hf;
-          acc[6] += dely * delz * hf;
+        force_four<EV, SINGLE>(a, me, s_t2rhor, s_t2z2r, fpd, ee, xj, fpq, mm, fx, fy, fz, acc);
+      } else {
+        int4 xs[4];
+        float fpq[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int jj = md_entry_j(ee[u]);
+          xs[u] = SINGLE ? __ldg(reinterpret_cast<const int4 *>(a.xf) + jj) : xq[jj];
+          fpq[u] = SINGLE ? __int_as_float(xs[u].w) : a.fpf[jj];
         }
-       }
-      };
-      walk_list<TPA>(a.nlist, a.stride, i, num, lane, four);
-    } else {
-      const int4 xi = xq[i];
-      const int ti = xi.w;
-      const float fpi = a.fpf[i];
-      const float qx = a.box.qs[0], qy = a.box.qs[1], qz = a.box.qs[2];
-      const float qxl = a.box.qs_lo[0], qyl = a.box.qs_lo[1], qzl = a.box.qs_lo[2];
-      const float cutf = (float)a.cutforcesq, rdrf = (float)a.rdr;
-      // one element: the density-derivative and pair spline rows of every pair
-      const float *drow1 = SINGLE ? a.fz_f + 4 : nullptr;
-      const float *zrow1 = SINGLE ? a.fz_f : nullptr;
-      // four entries ee of this lane (walk_list)
-      auto four = [&](const unsigned (&ee)[4], int) {
-       // whole slabs: pad entries in the last slab name the atom itself
-       // (zero separation), which the r^2 > 0 test rejects
-       int4 xs[4];
-       float fpq[4];
-#pragma unroll
-       for (int u = 0; u < 4; u++) {
-         const int jj = md_entry_j(ee[u]);
-         xs[u] = SINGLE ? __ldg(reinterpret_cast<const int4 *>(a.xf) + jj) : xq[jj];
-         fpq[u] = SINGLE ? __int_as_float(xs[u].w) : a.fpf[jj];
-       }
-       // FP32 sum of the slab's pair forces, added to the FP64 accumulator
-       float cfx = 0.f, cfy = 0.f, cfz = 0.f;
-       float ce[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // EV: the slab's FP32 sums
-#pragma unroll
-       for (int u = 0; u < 4; u++) {
-        const int4 xj = xs[u];
-        // minimum-image separation from the fixed-point coordinates
-        const float delx = md_qlen(md_qdiff(xi.x, xj.x), qx, qxl);
-        const float dely = md_qlen(md_qdiff(xi.y, xj.y), qy, qyl);
-        const float delz = md_qlen(md_qdiff(xi.z, xj.z), qz, qzl);
-        const float rsq = delx * delx + dely * dely + delz * delz;
-        if (rsq < cutf && rsq > 0.f) {
-          const int tj = SINGLE ? 1 : xj.w;
-          const float recip = rsqrtf(rsq);
-          const float r = rsq * recip;
-          int m;
-          float p;
-          knot_f(r * rdrf + 1.0f, a.nr - 1, m, p);
-          const size_t o8 = (size_t)m * 8;
-          const float *drow =
-              SINGLE ? drow1 : a.rhor_f + (size_t)s_t2rhor[ti * a.ntp1 + tj] * (a.nr + 1) * 8 + 4;
-          const float4 ci = __ldg(reinterpret_cast<const float4 *>(drow + o8));
-          const float rhoip = (ci.x * p + ci.y) * p + ci.z;
-          float rhojp = rhoip;
-          if (!SINGLE && !a.rhor_sym) {
-            const float4 cj = __ldg(reinterpret_cast<const float4 *>(
-                a.rhor_f + ((size_t)s_t2rhor[tj * a.ntp1 + ti] * (a.nr + 1) + m) * 8 + 4));
-            rhojp = (cj.x * p + cj.y) * p + cj.z;
-          }
-          const float *zb =
-              (SINGLE ? zrow1 : a.z2r_f + (size_t)s_t2z2r[ti * a.ntp1 + tj] * (a.nr + 1) * 8) + o8;
-          const float4 zv = __ldg(reinterpret_cast<const float4 *>(zb));
-          float z2p;
-          if (SINGLE) {
-            // the z2 derivative from the value coefficients:
-            // (3 c3 p^2 + 2 c4 p + c5) / dr, as PairEAM::interpolate stores it
-            z2p = (fmaf(3.0f * zv.x, p, 2.0f * zv.y) * p + zv.z) * rdrf;
-          } else {
-            const float4 zd = __ldg(reinterpret_cast<const float4 *>(zb + 4));
-            z2p = (zd.x * p + zd.y) * p + zd.z;
-          }
-          const float z2 = ((zv.x * p + zv.y) * p + zv.z) * p + zv.w;
-          const float phi = z2 * recip;
-          const float phip = z2p * recip - phi * recip;
-          const float psip = fpi * rhojp + fpq[u] * rhoip + phip;
-          const float fpair = -psip * recip;
-          cfx += delx * fpair;
-          cfy += dely * fpair;
-          cfz += delz * fpair;
-          if (EV) {
-            ce[0] = fmaf(0.5f, phi, ce[0]);
-            const float hf = 0.5f * fpair;
-            ce[1] = fmaf(delx * delx, hf, ce[1]);
-            ce[2] = fmaf(dely * dely, hf, ce[2]);
-            ce[3] = fmaf(delz * delz, hf, ce[3]);
-            ce[4] = fmaf(delx * dely, hf, ce[4]);
-            ce[5] = fmaf(delx * delz, hf, ce[5]);
-            ce[6] = fmaf(dely * delz, hf, ce[6]);
-          }
-        }
-       }
-       fx += (double)cfx;
-       fy += (double)cfy;
-       fz += (double)cfz;
-       // the energy and virial terms join the FP64 sums once per slab, as the
-       // forces do
-       if (EV)
-#pragma unroll
-         for (int k = 0; k < 7; k++) acc[k] += (double)ce[k];
-      };
-      walk_list<TPA>(a.nlist, a.stride, i, num, lane, four);
-    }
+        force_four<EV, SINGLE>(a, me, s_t2rhor, s_t2z2r, fpf, xs, fpq, fx, fy, fz, acc);
+      }
+    };
+    walk_list<TPA>(a.nlist, a.stride, i, num, lane, four);
   }
   fx = lane_sum<TPA>(fx);
   fy = lane_sum<TPA>(fy);
@@ -468,6 +497,164 @@ __global__ void __launch_bounds__(128) k_eam_force(EamArgs a, const double4 *__r
     }
     block_partials_finish<7>(acc, red, a.partial, a.counter, a.ev, true);
   }
+}
+
+// Several MD steps of eam in one cooperative launch, as k_lj_multi: a thread
+// keeps its atom, its list entries and (first lane) the atom's state for the
+// whole launch.  A step is the density pass, a grid barrier (every F' is
+// written), the force pass with the half-steps, and a barrier (every position
+// is written), whose word carries the distance criterion.
+template <int TPA, bool MIXED, bool SINGLE, int DEPTH>
+__global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
+    k_eam_multi(EamArgs a, MultiArgs m) {
+  constexpr int AB = kMultiThreads / TPA;  // atoms of a block
+  extern __shared__ double s_state[];
+  __shared__ int s_t2rhor[TABSZ];
+  __shared__ int s_t2z2r[TABSZ];
+  __shared__ int s_t2frho[MD_MAXTYPES + 1];
+  int *s_list = reinterpret_cast<int *>(s_state + kMultiState * AB);
+  StepArgs &s = a.step;
+  for (int k = threadIdx.x; k < a.ntp1 * a.ntp1; k += blockDim.x) {
+    s_t2rhor[k] = a.t2rhor[k];
+    s_t2z2r[k] = a.t2z2r[k];
+  }
+  for (int k = threadIdx.x; k < a.ntp1; k += blockDim.x) s_t2frho[k] = a.t2frho[k];
+  if (blockIdx.x == 0)
+    for (int k = threadIdx.x; k < m.bar_words; k += blockDim.x) m.bar_next[k] = 0u;
+  const int i = (blockIdx.x * kMultiThreads + threadIdx.x) / TPA;
+  const int lane = threadIdx.x % TPA;
+  const bool active = i < a.n;
+  const MultiList<TPA> list(a.nlist, a.stride, active ? i : 0, active ? a.numneigh[i] : 0, lane,
+                            m.slots, s_list);
+  MultiState<TPA> st(s_state);
+  EamSide<MIXED, SINGLE> me;
+  me.ti = 1;
+  me.xi = make_double4(0, 0, 0, 1);
+  me.qi = make_int4(0, 0, 0, 1);
+  me.init(a, !MIXED && active ? a.cell[i] : 0);
+  if (active) {
+    if (MIXED) me.qi = static_cast<const int4 *>(s.cur)[i], me.ti = me.qi.w;
+    else me.xi = static_cast<const double4 *>(s.cur)[i], me.ti = (int)me.xi.w;
+    if (lane == 0) st.load(s, i, a.stride, MIXED ? s.x4[i] : me.xi);
+  }
+  __syncthreads();
+  int ago = m.ago;
+  for (int j = 0;; j++) {
+    // density and embedding
+    double rho = 0.0;
+    for (int k = 0; k < list.cnt; k += 4 * DEPTH) {
+      unsigned ee[DEPTH][4];
+      double4 xj[DEPTH][4];
+      int4 xs[DEPTH][4];
+#pragma unroll
+      for (int d = 0; d < DEPTH; d++)
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int e = k + 4 * d + u;
+          ee[d][u] = e < list.cnt ? list.entry(e) : 0u;
+          if (MIXED)  // past the end: the atom itself
+            xs[d][u] = e < list.cnt
+                           ? ld_pos<true>(static_cast<const int4 *>(s.cur) + md_entry_j(ee[d][u]))
+                           : me.qi;
+          else
+            xj[d][u] = e < list.cnt ? ld_pos<true>(static_cast<const double4 *>(s.cur) +
+                                                   md_entry_j(ee[d][u]))
+                                    : me.xi;
+        }
+#pragma unroll
+      for (int d = 0; d < DEPTH; d++) {
+        if (d > 0 && k + 4 * d >= list.cnt) break;
+        if constexpr (MIXED) rho_four<SINGLE>(a, me, s_t2rhor, xs[d], rho);
+        else rho_four<SINGLE>(a, me, s_t2rhor, ee[d], xj[d], list.cnt - k - 4 * d, rho);
+      }
+    }
+    rho = lane_sum<TPA>(rho);
+    double fpi = 0.0;
+    if (active && lane == 0) {
+      double phi;
+      embed(a, s_t2frho[me.ti], rho, fpi, phi);
+      if (SINGLE) {
+        if (MIXED)
+          reinterpret_cast<int4 *>(a.xf)[i] =
+              make_int4(me.qi.x, me.qi.y, me.qi.z, __float_as_int((float)fpi));
+        else a.xf[i] = make_double4(me.xi.x, me.xi.y, me.xi.z, fpi);
+      } else if (MIXED) a.fpf[i] = (float)fpi;
+      else a.fp[i] = fpi;
+    }
+    if (md_grid_barrier(m.bar + 2 * j, false, true, s.status) < 0) return;
+    fpi = from_first<TPA>(fpi);
+    // forces
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    double acc[7] = {0, 0, 0, 0, 0, 0, 0};
+    for (int k = 0; k < list.cnt; k += 4 * DEPTH) {
+      unsigned ee[DEPTH][4];
+      double4 xj[DEPTH][4];
+      int4 xs[DEPTH][4];
+      double fpd[DEPTH][4];
+      float fpf[DEPTH][4];
+#pragma unroll
+      for (int d = 0; d < DEPTH; d++)
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int e = k + 4 * d + u;
+          const bool have = e < list.cnt;
+          ee[d][u] = have ? list.entry(e) : 0u;
+          const int jj = md_entry_j(ee[d][u]);
+          if (MIXED) {
+            const int4 *base = SINGLE ? reinterpret_cast<const int4 *>(a.xf)
+                                      : static_cast<const int4 *>(s.cur);
+            xs[d][u] = have ? ld_pos<true>(base + jj) : me.qi;
+            fpf[d][u] = SINGLE ? __int_as_float(xs[d][u].w) : have ? ld_plain(a.fpf + jj) : 0.f;
+            if (SINGLE && !have) fpf[d][u] = 0.f;
+          } else {
+            const double4 *base = SINGLE ? a.xf : static_cast<const double4 *>(s.cur);
+            xj[d][u] = have ? ld_pos<true>(base + jj) : me.xi;
+            fpd[d][u] = SINGLE ? xj[d][u].w : have ? ld_plain(a.fp + jj) : 0.0;
+          }
+        }
+#pragma unroll
+      for (int d = 0; d < DEPTH; d++) {
+        if (d > 0 && k + 4 * d >= list.cnt) break;
+        if constexpr (MIXED)
+          force_four<false, SINGLE>(a, me, s_t2rhor, s_t2z2r, (float)fpi, xs[d], fpf[d], fx, fy,
+                                    fz, acc);
+        else
+          force_four<false, SINGLE>(a, me, s_t2rhor, s_t2z2r, fpi, ee[d], xj[d], fpd[d],
+                                    list.cnt - k - 4 * d, fx, fy, fz, acc);
+      }
+    }
+    fx = lane_sum<TPA>(fx);
+    fy = lane_sum<TPA>(fy);
+    fz = lane_sum<TPA>(fz);
+    bool moved = false;
+    if (active && lane == 0) {
+      const double4 p = st.step(s, fx, fy, fz, MIXED ? (double)me.qi.w : me.xi.w, moved);
+      if (MIXED) {
+        me.qi = md_xq(p, a.box);
+        static_cast<int4 *>(s.nxt)[i] = me.qi;
+      } else {
+        me.xi = p;
+        static_cast<double4 *>(s.nxt)[i] = p;
+      }
+    }
+    void *t = const_cast<void *>(s.cur);
+    s.cur = s.nxt;
+    s.nxt = t;
+    const int go = md_multi_next(s, m, j, 2 * j + 1, ago, moved);
+    if (go < 0) return;
+    if (go == 0) break;
+    if (MIXED) {
+      me.qi.x = from_first<TPA>(me.qi.x);
+      me.qi.y = from_first<TPA>(me.qi.y);
+      me.qi.z = from_first<TPA>(me.qi.z);
+    } else {
+      me.xi.x = from_first<TPA>(me.xi.x);
+      me.xi.y = from_first<TPA>(me.xi.y);
+      me.xi.z = from_first<TPA>(me.xi.z);
+    }
+  }
+  if (active && lane == 0)
+    st.store(s, i, a.stride, MIXED, MIXED ? (double)me.qi.w : me.xi.w);
 }
 
 // phase event between the two passes: an event-record node when the stream
@@ -668,6 +855,45 @@ void launch_step_tpa(b200_ctx *c, const EamArgs &a, bool out) {
 }
 }  // namespace
 
+namespace {
+template <int TPA, int DEPTH>
+const void *eam_multi_kernel(const b200_ctx *c) {
+  const bool single = c->ntypes == 1;
+  if (c->prec == B200_PREC_MIXED)
+    return single ? (const void *)k_eam_multi<TPA, true, true, DEPTH>
+                  : (const void *)k_eam_multi<TPA, true, false, DEPTH>;
+  return single ? (const void *)k_eam_multi<TPA, false, true, DEPTH>
+                : (const void *)k_eam_multi<TPA, false, false, DEPTH>;
+}
+template <int DEPTH>
+const void *eam_multi_kernel(const b200_ctx *c) {
+  return c->tpa == 1   ? eam_multi_kernel<1, DEPTH>(c)
+         : c->tpa == 2 ? eam_multi_kernel<2, DEPTH>(c)
+         : c->tpa == 4 ? eam_multi_kernel<4, DEPTH>(c)
+                       : eam_multi_kernel<8, DEPTH>(c);
+}
+}  // namespace
+
+MultiPlan md_eam_multi_plan(const b200_ctx *c) {
+  if (!md_eam_step_ok(c)) return MultiPlan();
+  return md_multi_shape(c, eam_multi_kernel<1>(c), eam_multi_kernel<2>(c));
+}
+
+cudaError_t md_eam_multi(b200_ctx *c, const MultiPlan &p, double dtv, double dtf, MultiArgs m,
+                         int every, int check) {
+  EamArgs a = eam_args(c, nullptr, nullptr);
+  a.step = md_step_args(c, dtv, dtf);
+  a.step.every = every;
+  a.step.check = check;
+  if (!check) a.step.xhold = nullptr;
+  m.slots = p.slots;
+  void *args[2] = {&a, &m};
+  cudaError_t e = cudaLaunchCooperativeKernel(p.kernel, dim3(p.blocks), dim3(p.threads), args,
+                                              p.smem, c->stream);
+  c->launches++;
+  return e;
+}
+
 bool md_eam_step_ok(const b200_ctx *c) {
   return c->pstyle == B200_PAIR_EAM && c->tpa >= 1 && c->tpa <= 8 && c->nrep == 0 &&
          !c->ghosts_on;
@@ -675,29 +901,7 @@ bool md_eam_step_ok(const b200_ctx *c) {
 
 cudaError_t md_eam_step(b200_ctx *c, double dtv, double dtf, bool out) {
   EamArgs a = eam_args(c, nullptr, nullptr);
-  StepArgs &s = a.step;
-  s.dtv = dtv;
-  s.dtf = dtf;
-  s.triggersq = 0.25 * c->skin * c->skin;  // src/neighbor.cpp:239
-  s.mass = c->mass_dev;
-  s.x4 = c->x4;
-  if (c->prec == B200_PREC_MIXED) {
-    s.cur = c->xq;
-    s.nxt = c->xqb;
-  } else {
-    s.cur = c->x4;
-    s.nxt = c->x4b;
-  }
-  s.v = c->v;
-  s.xhold = c->check ? c->xhold : nullptr;
-  s.status = c->status;
-  s.dcount = c->dec_count;
-  s.mail = c->mail_dev;
-  s.rows = c->rows;
-  s.rows_cap = c->rows_cap;
-  s.every = c->every;
-  s.delay = c->delay;
-  s.check = c->check;
+  a.step = md_step_args(c, dtv, dtf);
   switch (c->tpa) {
     case 1: launch_step_tpa<1>(c, a, out); break;
     case 2: launch_step_tpa<2>(c, a, out); break;

@@ -465,23 +465,6 @@ __global__ void __launch_bounds__(128) k_lj_step(PairArgs a, StepArgs s) {
 // lanes, 15.7 -> 9.0; 32,000 FP64 25 -> 18.  Of the 9.0, 2.5 to 3 are the
 // barrier and the half-steps, the rest the gathers (each SM's L1 starts cold
 // after every barrier).
-constexpr int kMultiThreads = 256;
-// doubles of an atom's state: x, y, z, v, dtf / mass, x, y, z at the last build
-constexpr int kMultiState = 10;
-inline size_t multi_smem(int tpa, int slots) {
-  return (size_t)kMultiState * (kMultiThreads / tpa) * sizeof(double) +
-         (size_t)slots * kMultiThreads * sizeof(int);
-}
-// one 32-bit word of the atom's first lane to all its lanes
-template <int TPA>
-__device__ __forceinline__ int from_first(int v) {
-  return TPA == 1 ? v : __shfl_sync(0xffffffffu, v, 0, TPA);
-}
-template <int TPA>
-__device__ __forceinline__ double from_first(double v) {
-  return TPA == 1 ? v : __shfl_sync(0xffffffffu, v, 0, TPA);
-}
-
 template <int TPA, bool SINGLE, bool MIXED, int DEPTH>
 __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
     k_lj_multi(PairArgs a, StepArgs s, MultiArgs m) {
@@ -504,39 +487,17 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
   const int i = (blockIdx.x * kMultiThreads + threadIdx.x) / TPA;
   const int lane = threadIdx.x % TPA;
   const bool active = i < a.n;
-  double *st = s_state + threadIdx.x / TPA;  // field k at st[k * AB]
-  // this lane's entries: lane, lane + TPA, ... of the atom's list
-  const int num = active ? a.numneigh[i] : 0;
-  const int cnt = num > lane ? (num - lane + TPA - 1) / TPA : 0;
-  auto fetch = [&](int k) {
-    const int e = lane + TPA * k;
-    return a.nlist[md_slab(e, i, a.stride)];
-  };
-  for (int k = 0; k < cnt && k < m.slots; k++) s_list[k * kMultiThreads + threadIdx.x] = fetch(k);
-  auto entry = [&](int k) {
-    return (unsigned)(k < m.slots ? s_list[k * kMultiThreads + threadIdx.x] : fetch(k));
-  };
+  const MultiList<TPA> list(a.nlist, a.stride, active ? i : 0, active ? a.numneigh[i] : 0, lane,
+                            m.slots, s_list);
+  const int cnt = list.cnt;
+  auto entry = [&](int k) { return list.entry(k); };
+  MultiState<TPA> st(s_state);
   double4 xi = make_double4(0, 0, 0, 1);  // FP64: this atom's position
   int4 qi = make_int4(0, 0, 0, 1);        // mixed: the same in fixed point
   if (active) {
     if (MIXED) qi = static_cast<const int4 *>(s.cur)[i];
     else xi = static_cast<const double4 *>(s.cur)[i];
-    if (lane == 0) {
-      const double4 p = MIXED ? s.x4[i] : xi;
-      st[0] = p.x;
-      st[AB] = p.y;
-      st[2 * AB] = p.z;
-      st[3 * AB] = s.v[i];
-      st[4 * AB] = s.v[a.stride + i];
-      st[5 * AB] = s.v[2 * a.stride + i];
-      st[6 * AB] = s.dtf / s.mass[(int)p.w];
-      if (s.xhold) {
-        const double4 h = s.xhold[i];
-        st[7 * AB] = h.x;
-        st[8 * AB] = h.y;
-        st[9 * AB] = h.z;
-      }
-    }
+    if (lane == 0) st.load(s, i, a.stride, MIXED ? s.x4[i] : xi);
   }
   __syncthreads();
   const MixedPairs<false, SINGLE, true> mp(a, a.box, tabf, nt2);
@@ -585,19 +546,7 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
     fz = lane_sum<TPA>(fz);
     bool moved = false;
     if (active && lane == 0) {
-      // final half-step of this step, initial half-step of the next: the
-      // rounded operations of md_nve_step_atom
-      const double dtfm = st[6 * AB];
-      double vx = __dadd_rn(st[3 * AB], __dmul_rn(dtfm, fx));
-      double vy = __dadd_rn(st[4 * AB], __dmul_rn(dtfm, fy));
-      double vz = __dadd_rn(st[5 * AB], __dmul_rn(dtfm, fz));
-      vx = __dadd_rn(vx, __dmul_rn(dtfm, fx));
-      vy = __dadd_rn(vy, __dmul_rn(dtfm, fy));
-      vz = __dadd_rn(vz, __dmul_rn(dtfm, fz));
-      const double4 p = make_double4(__dadd_rn(st[0], __dmul_rn(s.dtv, vx)),
-                                     __dadd_rn(st[AB], __dmul_rn(s.dtv, vy)),
-                                     __dadd_rn(st[2 * AB], __dmul_rn(s.dtv, vz)),
-                                     MIXED ? (double)qi.w : xi.w);
+      const double4 p = st.step(s, fx, fy, fz, MIXED ? (double)qi.w : xi.w, moved);
       if (MIXED) {
         qi = md_xq(p, a.box);
         static_cast<int4 *>(s.nxt)[i] = qi;
@@ -605,34 +554,13 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
         xi = p;
         static_cast<double4 *>(s.nxt)[i] = p;
       }
-      st[0] = p.x;
-      st[AB] = p.y;
-      st[2 * AB] = p.z;
-      st[3 * AB] = vx;
-      st[4 * AB] = vy;
-      st[5 * AB] = vz;
-      if (s.xhold)
-        moved = dsq3(__dsub_rn(p.x, st[7 * AB]), __dsub_rn(p.y, st[8 * AB]),
-                     __dsub_rn(p.z, st[9 * AB])) > s.triggersq;
     }
     void *t = const_cast<void *>(s.cur);
     s.cur = s.nxt;
     s.nxt = t;
-    ago++;
-    const bool last = j + 1 == m.nsteps;
-    const bool cand = md_candidate(s.every, s.delay, ago);
-    bool rebuild = !s.check && cand;
-    if (!last || (s.check && cand)) {
-      // after the last step only the block that posts the decision waits
-      const int r = md_grid_barrier(m.bar + j, moved, !last || blockIdx.x == 0, s.status);
-      if (r < 0) return;
-      if (s.check && cand) rebuild = r != 0;
-    }
-    if (last || rebuild) {
-      if (blockIdx.x == 0 && threadIdx.x == 0)
-        md_multi_end(s.status, j + 1, ago, rebuild, s.every, s.delay, s.check, s.dcount, s.mail);
-      break;
-    }
+    const int go = md_multi_next(s, m, j, j, ago, moved);
+    if (go < 0) return;
+    if (go == 0) break;
     if (MIXED) {
       qi.x = from_first<TPA>(qi.x);
       qi.y = from_first<TPA>(qi.y);
@@ -643,12 +571,7 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
       xi.z = from_first<TPA>(xi.z);
     }
   }
-  if (active && lane == 0) {
-    if (MIXED) s.x4[i] = make_double4(st[0], st[AB], st[2 * AB], (double)qi.w);
-    s.v[i] = st[3 * AB];
-    s.v[a.stride + i] = st[4 * AB];
-    s.v[2 * a.stride + i] = st[5 * AB];
-  }
+  if (active && lane == 0) st.store(s, i, a.stride, MIXED, MIXED ? (double)qi.w : xi.w);
 }
 
 // One MD step of every replica of a batched context in one launch.  Cluster g
@@ -986,7 +909,7 @@ bool md_lj_step_ok(const b200_ctx *c) {
          (c->prec != B200_PREC_MIXED || md_q_iso(c)) && c->nrep == 0 && !c->ghosts_on;
 }
 
-static StepArgs step_args(b200_ctx *c, double dtv, double dtf) {
+StepArgs md_step_args(b200_ctx *c, double dtv, double dtf) {
   StepArgs s;
   s.dtv = dtv;
   s.dtf = dtf;
@@ -1015,7 +938,7 @@ static StepArgs step_args(b200_ctx *c, double dtv, double dtf) {
 
 cudaError_t md_lj_step(b200_ctx *c, double dtv, double dtf, bool out) {
   const PairArgs a = pair_args(c, nullptr, nullptr);
-  const StepArgs s = step_args(c, dtv, dtf);
+  const StepArgs s = md_step_args(c, dtv, dtf);
   switch (c->tpa) {
     case 1: launch_step_tpa<1>(c, a, s, out); break;
     case 2: launch_step_tpa<2>(c, a, s, out); break;
@@ -1048,32 +971,15 @@ const void *multi_kernel(const b200_ctx *c) {
 }
 }  // namespace
 
-// The multi-step launch at the current shape; blocks 0 when the box does not
-// run in that form: all of its atoms must be resident at once.  Up to two
-// blocks per SM, a thread may use 128 registers and gathers two groups of
-// neighbours at once; above, 64 and one.
 MultiPlan md_lj_multi_plan(const b200_ctx *c) {
-  MultiPlan p;
-  if (!md_lj_step_ok(c)) return p;
-  const int groups = md_blocks((long long)c->n * c->tpa, kMultiThreads);
-  p.kernel = groups <= 2 * md_sms(c) ? multi_kernel<2>(c) : multi_kernel<1>(c);
-  p.threads = kMultiThreads;
-  // list entries kept per thread: the mean and some more, as far as they fit
-  const double rc = c->cutneighmax, vol = c->box.prd[0] * c->box.prd[1] * c->box.prd[2];
-  const double mean = 4.18879 * rc * rc * rc * c->n / vol;
-  const int per_sm = (groups + md_sms(c) - 1) / md_sms(c);
-  const size_t most = (size_t)216 * 1024 / (per_sm > 0 ? per_sm : 1) - 7 * 1024;
-  p.slots = (int)(1.25 * mean / c->tpa) + 4;
-  while (p.slots > 0 && multi_smem(c->tpa, p.slots) > most) p.slots--;
-  p.smem = multi_smem(c->tpa, p.slots);
-  p.blocks = md_coop_blocks(c, p.kernel, p.threads, p.smem, groups);
-  return p;
+  if (!md_lj_step_ok(c)) return MultiPlan();
+  return md_multi_shape(c, multi_kernel<1>(c), multi_kernel<2>(c));
 }
 
 cudaError_t md_lj_multi(b200_ctx *c, const MultiPlan &p, double dtv, double dtf, MultiArgs m,
                         int every, int check) {
   PairArgs a = pair_args(c, nullptr, nullptr);
-  StepArgs s = step_args(c, dtv, dtf);
+  StepArgs s = md_step_args(c, dtv, dtf);
   s.every = every;
   s.check = check;
   if (!check) s.xhold = nullptr;

@@ -59,6 +59,8 @@ CASES = [
     ("lj", 1, (6, 6, 6), 0, (1, 3, True), 60, 25),
     ("lj", 3, (8, 8, 8), 3, (5, 0, True), 47, 10),
     ("lj", 1, (12, 12, 12), 0, (7, 0, False), 40, 0),
+    ("eam", 1, (5, 6, 5), 1, (1, 5, True), 45, 20),
+    ("eam", 1, (10, 10, 10), 0, (10, 0, False), 33, 0),
 ]
 
 
