@@ -364,6 +364,11 @@ int b200_replica_thermo(b200_ctx *ctx, double *rows);
 
    Replace the positions (device array) and rebuild the list. */
 int b200_adj_set_positions(b200_ctx *ctx, const double *x);
+/* *held = 1 when x (device, 3n doubles, caller order) is, bit for bit, what
+   the last b200_adj_set_positions was given and no call has changed the
+   context's atoms, lists or settings since: a backward pass then needs no
+   second upload and build. */
+int b200_adj_positions_held(b200_ctx *ctx, const double *x, int *held);
 /* F_i = sum_j phi(r_ij) (x_i - x_j), phi = (lj1 r^-6 - lj2) r^-8 inside
    cutsq (PairLJCut::compute's pair force, src/pair_lj_cut.cpp:100-113);
    FP32 pair math with FP64 sums for a B200_PREC_MIXED context, FP64

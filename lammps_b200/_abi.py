@@ -79,6 +79,7 @@ SIGNATURES = {
     "b200_replica_count": (C.c_int, [_vp]),
     "b200_replica_thermo": (C.c_int, [_vp, _dp]),
     "b200_adj_set_positions": (C.c_int, [_vp, _vp]),
+    "b200_adj_positions_held": (C.c_int, [_vp, _vp, C.POINTER(C.c_int)]),
     "b200_adj_forces": (C.c_int, [_vp, _dp, _dp, _dp, _vp]),
     "b200_adj_backward": (C.c_int, [_vp, _dp, _dp, _dp, _vp, _vp, _dp, _dp]),
     "b200_kinetic_sum_noalloc": (C.c_int, [C.c_int, _vp, _vp, _vp, C.c_int, _vp, _vp]),

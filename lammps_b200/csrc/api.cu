@@ -51,6 +51,7 @@ void dfree(T *&p) {
 }
 
 void invalidate_graphs(b200_ctx *c) {
+  c->adj_held = false;
   for (int k = 0; k < MD_NGRAPHS; k++) {
     if (c->step_exec[k]) cudaGraphExecDestroy(c->step_exec[k]);
     if (c->step_graph[k]) cudaGraphDestroy(c->step_graph[k]);
@@ -393,6 +394,12 @@ int upload_tables(b200_ctx *c) {
     maps[(MD_MAXTYPES + 1) + k] = c->eam.type2rhor[k];
     maps[(MD_MAXTYPES + 1) + TABSZ + k] = c->eam.type2z2r[k];
   }
+  std::vector<double> m(MD_MAXTYPES + 1, 1.0);
+  for (int t = 1; t <= c->ntypes; t++) m[t] = c->mass[t];
+  // the device already holds these values
+  if (c->tables_dev && c->mass_dev && tab == c->tab_up && maps == c->maps_up && m == c->mass_up)
+    return B200_OK;
+  c->tab_up.clear();
   if (!c->tables_dev) {
     size_t bytes = TAB_COUNT * TABSZ * sizeof(double) + maps.size() * sizeof(int);
     CK(cudaMalloc((void **)&c->tables_dev, bytes));
@@ -402,12 +409,13 @@ int upload_tables(b200_ctx *c) {
                      cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->tables_dev + TAB_COUNT * TABSZ, maps.data(), maps.size() * sizeof(int),
                      cudaMemcpyHostToDevice, c->stream));
-  std::vector<double> m(MD_MAXTYPES + 1, 1.0);
-  for (int t = 1; t <= c->ntypes; t++) m[t] = c->mass[t];
   if (!c->mass_dev) CK(cudaMalloc((void **)&c->mass_dev, (MD_MAXTYPES + 1) * sizeof(double)));
   CK(cudaMemcpyAsync(c->mass_dev, m.data(), m.size() * sizeof(double), cudaMemcpyHostToDevice,
                      c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  c->tab_up = tab;
+  c->maps_up = maps;
+  c->mass_up = m;
   return B200_OK;
 }
 
@@ -1123,7 +1131,7 @@ int b200_destroy(b200_ctx *c) {
   dfree(c->cell_count); dfree(c->cell_start); dfree(c->scan_tmp);
   dfree(c->slot); dfree(c->perm); dfree(c->cell_tmp);
   dfree(c->nlist); dfree(c->numneigh); dfree(c->partial); dfree(c->counter); dfree(c->ev);
-  dfree(c->adj_gs); dfree(c->adj_gtab);
+  dfree(c->adj_gs); dfree(c->adj_gtab); dfree(c->adj_x);
   dfree(c->d_rep_box); dfree(c->d_rep_of_atom); dfree(c->d_rep_cell_base); dfree(c->d_tile_rep);
   dfree(c->d_rep_tile_base); 
   dfree(c->status); dfree(c->rows); dfree(c->tables_dev);
@@ -1317,6 +1325,7 @@ int b200_upload_atoms(b200_ctx *c, int n, const double *x, const double *v, cons
                       const int *tag) {
   (void)tag;
   if (!c || n < 1 || !x || !type) return set_err(c, B200_ERR_ARG, "Illegal atoms");
+  c->adj_held = false;
   if (n > MD_MAX_ATOMS) return set_err(c, B200_ERR_ARG, "too many atoms (%d > %d)", n, MD_MAX_ATOMS);
   if (c->ntypes < 1) return set_err(c, B200_ERR_STATE, "set masses or a pair style before atoms");
   CK(cudaSetDevice(c->device));
@@ -1447,6 +1456,7 @@ int b200_gather(b200_ctx *c, int fields, int m, const int *idx, double *out) {
 
 int b200_update_positions(b200_ctx *c, const double *x) {
   if (!c || !x) return B200_ERR_ARG;
+  c->adj_held = false;
   if (!c->sorted_once) return set_err(c, B200_ERR_STATE, "neighbor list not built");
   CK(cudaSetDevice(c->device));
   const size_t bytes = 3 * (size_t)c->n * sizeof(double);
@@ -1542,6 +1552,7 @@ int b200_stage_atoms(b200_ctx *c, int n, const double *x, const double *v, const
 
 int b200_set_staged_atoms(b200_ctx *c) {
   if (!c) return B200_ERR_ARG;
+  c->adj_held = false;
   if (c->in_count == 0) return set_err(c, B200_ERR_STATE, "no staged atom set");
   CK(cudaSetDevice(c->device));
   b200_ctx::XferSlot &s = c->in_slot[c->in_head];
@@ -1624,6 +1635,7 @@ static int prepare(b200_ctx *c) {
 
 int b200_neigh_build(b200_ctx *c) {
   if (!c) return B200_ERR_ARG;
+  c->adj_held = false;
   int rc = prepare(c);
   if (rc) return rc;
   rc = rebuild_sync(c);
@@ -1753,6 +1765,7 @@ int b200_eam_force(b200_ctx *c, int eflag, int vflag, double *eng, double virial
 
 int b200_nve_initial(b200_ctx *c, double dtv, double dtf) {
   if (!c) return B200_ERR_ARG;
+  c->adj_held = false;
   if (!c->sorted_once) return set_err(c, B200_ERR_STATE, "neighbor list not built");
   CK(cudaSetDevice(c->device));
   CK(md_nve_initial(c, dtv, dtf));
@@ -1771,6 +1784,7 @@ int b200_nve_final(b200_ctx *c, double dtf) {
 
 int b200_setup(b200_ctx *c, double *row) {
   if (!c) return B200_ERR_ARG;
+  c->adj_held = false;
   int rc = prepare(c);
   if (rc) return rc;
   CK(cudaMemsetAsync(c->status, 0, ST_COUNT * sizeof(int), c->stream));
@@ -1815,6 +1829,7 @@ int b200_setup(b200_ctx *c, double *row) {
 int b200_run(b200_ctx *c, int nsteps, double dt, double ftm2v, int thermo_every, double *rows,
              int maxrows, int *nrows) {
   if (!c || nsteps < 0) return B200_ERR_ARG;
+  c->adj_held = false;
   if (!c->sorted_once) return set_err(c, B200_ERR_STATE, "b200_setup not called");
   if (c->ghosts_on)
     return set_err(c, B200_ERR_STATE,
@@ -2216,12 +2231,32 @@ int b200_adj_set_positions(b200_ctx *c, const double *x) {
   if (!c || !x) return B200_ERR_ARG;
   if (!c->have_atoms) return set_err(c, B200_ERR_STATE, "no atoms uploaded");
   CK(cudaSetDevice(c->device));
+  c->adj_held = false;
+  if (c->adj_x_n < c->n) {
+    CK(dalloc(&c->adj_x, 3 * (size_t)c->stride));
+    c->adj_x_n = c->stride;
+  }
   CK(md_adj_positions(c, x));
   int rc = prepare(c);
   if (rc) return rc;
   rc = rebuild_sync(c);
   if (rc) return rc;
   c->sorted_once = true;
+  c->adj_held = true;
+  return B200_OK;
+}
+
+int b200_adj_positions_held(b200_ctx *c, const double *x, int *held) {
+  if (!c || !x || !held) return B200_ERR_ARG;
+  *held = 0;
+  if (!c->adj_held) return B200_OK;
+  CK(cudaSetDevice(c->device));
+  CK(cudaMemsetAsync(c->status + ST_HALO_BAD, 0, sizeof(int), c->stream));
+  CK(md_adj_compare(c, x, c->status + ST_HALO_BAD));
+  int diff = 0;
+  const int rc = small_read(c, &diff, c->status + ST_HALO_BAD, sizeof(int));
+  if (rc) return rc;
+  *held = diff == 0;
   return B200_OK;
 }
 
@@ -2296,6 +2331,7 @@ int b200_neigh_check(b200_ctx *c, int *moved) {
 
 static int halo_call(b200_ctx *c, int m, const int *idx, const double *buf, bool pack) {
   if (!c || m < 0 || (m > 0 && (!idx || !buf))) return B200_ERR_ARG;
+  c->adj_held = false;
   if (!c->sorted_once) return set_err(c, B200_ERR_STATE, "neighbor list not built");
   CK(cudaSetDevice(c->device));
   if (m == 0) return B200_OK;

@@ -93,6 +93,9 @@ struct b200_ctx {
   // device copy of the per-type tables, TAB_* blocks of (ntypes+1)^2 doubles
   double *tables_dev = nullptr;
   double *cutneighsq_dev = nullptr;  // = tables_dev + TAB_CUTNEIGHSQ*TABSZ
+  // what tables_dev and mass_dev hold
+  std::vector<double> tab_up, mass_up;
+  std::vector<int> maps_up;
 
   // atoms (device, cell-sorted order)
   int n = 0, nalloc = 0, stride = 0;
@@ -168,6 +171,9 @@ struct b200_ctx {
   double *adj_gs = nullptr;    // force-matching scratch: G in the sorted order
   double *adj_gtab = nullptr;  // force-matching parameter gradients
   int adj_n = 0;
+  double *adj_x = nullptr;     // the positions b200_adj_set_positions was given
+  int adj_x_n = 0;
+  bool adj_held = false;       // nothing has changed atoms, lists or settings since
   double *ev = nullptr;          // [0] eng, [1..6] virial, [7] sum m v^2
   int *status = nullptr;         // ST_* words
   int *status_host = nullptr;    // pinned mirror
@@ -329,6 +335,8 @@ cudaError_t md_adj_backward(b200_ctx *c, const double *lj1, const double *lj2,
                             const double *cutsq, const double *g, double *gx, double *gs,
                             double *gtab);
 cudaError_t md_adj_positions(b200_ctx *c, const double *x);
+// *diff (device) = 1 when x is not, bit for bit, what md_adj_positions was given
+cudaError_t md_adj_compare(b200_ctx *c, const double *x, int *diff);
 
 // ---- replicas (replica.cu) ------------------------------------------------------
 // per-replica thermo rows {natoms, sum m v^2, eng_vdwl, virial[6]} from the

@@ -48,26 +48,26 @@ def lj_tables(eps, sigma, cut_factor: float = 2.5):
     return lj1.reshape(-1), lj2.reshape(-1), cutsq
 
 
+_pair_index = {}  # ntypes -> entry of [0, values...] at each matrix element (numpy)
+
+
 def pair_matrix(values, ntypes: int):
     """Symmetric (ntypes+1)^2 tensor from the upper-triangle values
     (1,1), (1,2), ..., (1,n), (2,2), ... (torch, differentiable)."""
     import torch
 
-    m = torch.zeros((ntypes + 1, ntypes + 1), dtype=values.dtype, device=values.device)
-    k = 0
-    rows, cols = [], []
-    for i in range(1, ntypes + 1):
-        for j in range(i, ntypes + 1):
-            rows.append(i)
-            cols.append(j)
-            k += 1
+    k = ntypes * (ntypes + 1) // 2
     if values.numel() != k:
         raise ValueError(f"expected {k} pair values for {ntypes} types, got {values.numel()}")
-    r = torch.tensor(rows)
-    c = torch.tensor(cols)
-    m = m.index_put((r, c), values)
-    m = m.index_put((c, r), values)
-    return m
+    index = _pair_index.get(ntypes)
+    if index is None:
+        m = np.zeros((ntypes + 1, ntypes + 1), np.int64)
+        r, c = np.triu_indices(ntypes)
+        m[r + 1, c + 1] = m[c + 1, r + 1] = 1 + np.arange(k)
+        index = _pair_index[ntypes] = m.ravel()
+    flat = torch.cat([values.new_zeros(1), values.reshape(-1)])
+    index = torch.from_numpy(index).to(values.device)
+    return flat.index_select(0, index).reshape(ntypes + 1, ntypes + 1)
 
 
 class LJForceField:
@@ -123,6 +123,16 @@ class LJForceField:
         self.sys._ck(self._L.b200_adj_set_positions(self.sys._h, C.c_void_p(xc.data_ptr())))
         self._x_ptr = xc
 
+    def _holds(self, x):
+        """Whether the context still holds the positions x and their list
+        (the device compares all of x); torch's work on x must be done."""
+        if tuple(x.shape) != (self.n, 3):
+            return False
+        held = C.c_int(0)
+        self.sys._ck(self._L.b200_adj_positions_held(self.sys._h, C.c_void_p(x.data_ptr()),
+                                                     C.byref(held)))
+        return bool(held.value)
+
     def _check_cutsq(self, cutsq):
         if np.any(cutsq > self.max_cutsq * (1 + 1e-12)):
             raise ValueError("a cutoff exceeds the max_cut the force field was built for")
@@ -157,11 +167,12 @@ def _make_function():
     class LJForces(torch.autograd.Function):
         @staticmethod
         def forward(ctx, x, lj1, lj2, ff, cutsq):
+            # allocated before set_positions, whose wait for torch's work also
+            # settles a block that torch's allocator has just handed out
+            f = torch.empty((ff.n, 3), dtype=torch.float64, device=x.device)
             ff.set_positions(x)
             l1 = np.ascontiguousarray(lj1.detach().cpu().numpy(), dtype=np.float64)
             l2 = np.ascontiguousarray(lj2.detach().cpu().numpy(), dtype=np.float64)
-            f = torch.empty((ff.n, 3), dtype=torch.float64, device=x.device)
-            torch.cuda.synchronize(x.device)
             ff.forces_raw(l1, l2, cutsq, f)
             ctx.save_for_backward(x, lj1, lj2)
             ctx.ff, ctx.cutsq, ctx.l1, ctx.l2 = ff, cutsq, l1, l2
@@ -171,10 +182,13 @@ def _make_function():
         def backward(ctx, gf):
             x, lj1, lj2 = ctx.saved_tensors
             ff = ctx.ff
-            ff.set_positions(x)
             g = gf.detach().to(torch.float64).contiguous()
             gx = torch.empty((ff.n, 3), dtype=torch.float64, device=x.device)
+            xc = x.detach().to(torch.float64).contiguous()
             torch.cuda.synchronize(x.device)
+            # the forward pass's list serves unless something came between
+            if not ff._holds(xc):
+                ff.set_positions(x)
             glj1, glj2 = ff.backward_raw(ctx.l1, ctx.l2, ctx.cutsq, g, gx)
             t1 = torch.from_numpy(glj1).to(dtype=lj1.dtype, device=lj1.device)
             t2 = torch.from_numpy(glj2).to(dtype=lj2.dtype, device=lj2.device)
