@@ -492,8 +492,11 @@ int status_errors(b200_ctx *c) {
   if (c->status_host[ST_LOST])
     return set_err(c, B200_ERR_LOST_ATOMS,
                    "Lost atoms: a coordinate is not finite or moved beyond one box length");
-  if (c->status_host[ST_BARRIER])
-    return set_err(c, B200_ERR_CUDA, "a grid barrier of a multi-step launch timed out");
+  if (c->status_host[ST_BARRIER]) {
+    cudaMemsetAsync(c->bar, 0, (2 * MD_BAR_WORDS + 4) * sizeof(unsigned), c->stream);
+    cudaMemsetAsync(c->status + ST_BARRIER, 0, sizeof(int), c->stream);
+    return set_err(c, B200_ERR_CUDA, "a grid barrier of a cooperative launch timed out");
+  }
   if (c->status_host[ST_OVERFLOW])
     return set_err(c, B200_ERR_NEIGH_OVERFLOW,
                    "Neighbor list overflow, boost neigh_modify one (need %d, have %d)",
@@ -517,7 +520,7 @@ int rebuild_sync(b200_ctx *c) {
     CK(md_rebuild(c, nullptr));
     int rc = read_status(c);
     if (rc) return rc;
-    if (c->status_host[ST_LOST]) return status_errors(c);
+    if (c->status_host[ST_LOST] || c->status_host[ST_BARRIER]) return status_errors(c);
     if (md_stage_feedback(c, c->status_host[ST_MAXSTAGE])) invalidate_graphs(c);
     if (!c->status_host[ST_OVERFLOW]) return B200_OK;
     if (c->one_user > 0) return status_errors(c);
@@ -1089,8 +1092,8 @@ int b200_create(int device, int precision, b200_ctx **out) {
   }
   if (e == cudaSuccess) e = cudaHostAlloc((void **)&c->bounce_host, kBounceBytes, cudaHostAllocMapped);
   if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&c->bounce_dev, c->bounce_host, 0);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&c->bar, 2 * MD_BAR_WORDS * sizeof(unsigned));
-  if (e == cudaSuccess) e = cudaMemset(c->bar, 0, 2 * MD_BAR_WORDS * sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMalloc((void **)&c->bar, (2 * MD_BAR_WORDS + 4) * sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMemset(c->bar, 0, (2 * MD_BAR_WORDS + 4) * sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMalloc((void **)&c->dec_count, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(c->dec_count, 0, sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc((void **)&c->ev, 8 * sizeof(double));
@@ -1863,7 +1866,7 @@ int b200_run(b200_ctx *c, int nsteps, double dt, double ftm2v, int thermo_every,
     int rc = ensure_graphs(c, dtv, dtf, ftm2v);
     if (rc) return rc;
   }
-  CK(cudaMemsetAsync(c->bar, 0, 2 * MD_BAR_WORDS * sizeof(unsigned), c->stream));
+  CK(cudaMemsetAsync(c->bar, 0, (2 * MD_BAR_WORDS + 4) * sizeof(unsigned), c->stream));
   CK(cudaMemsetAsync(c->status + ST_BARRIER, 0, sizeof(int), c->stream));
   CK(cudaMemsetAsync(c->status + ST_ROW, 0, sizeof(int), c->stream));
   CK(cudaMemsetAsync(c->status + ST_OVERFLOW, 0, sizeof(int), c->stream));
@@ -1984,7 +1987,7 @@ int b200_run(b200_ctx *c, int nsteps, double dt, double ftm2v, int thermo_every,
     }
     rc = read_status(c);
     if (rc) return rc;
-    if (c->status_host[ST_LOST]) return status_errors(c);
+    if (c->status_host[ST_LOST] || c->status_host[ST_BARRIER]) return status_errors(c);
     if (md_stage_feedback(c, c->status_host[ST_MAXSTAGE])) {
       // a builder tile staged more atoms than its shared memory held (it
       // took the slower global-memory path): larger staging from now on
