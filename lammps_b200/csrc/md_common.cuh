@@ -672,7 +672,7 @@ __device__ __forceinline__ void md_step_tail(const StepArgs &s, bool moved, cons
 
 // ---- pieces of the multi-step kernels ---------------------------------------
 
-constexpr int kMultiThreads = 256;
+constexpr int kMultiThreads = 256;  // threads of a block, at most
 // doubles of an atom's state: x, y, z, v, dtf / mass, x, y, z at the last build
 constexpr int kMultiState = 10;
 inline size_t md_multi_smem(int tpa, int slots) {
@@ -698,21 +698,64 @@ __device__ __forceinline__ float ld_plain(const float *p) {
   return v;
 }
 
+// Periodic shifts of an atom's neighbours in the FP64 form.  With two or more
+// cells per edge a cell has at most one wrapping neighbour per dimension, so
+// an entry's cell-offset code reduces to one bit per dimension (shifted or
+// not), made once when the entry is fetched.
+struct MultiShift {
+  double v[3];
+  int code[3];
+  bool any;
+  __device__ __forceinline__ MultiShift(int cell, const BoxGeom &box) {
+    int c[3];
+    md_cell_unpack(cell, c[0], c[1], c[2]);
+    any = false;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const bool lo = c[d] == 0, hi = c[d] + 1 >= box.ncell[d];
+      v[d] = lo ? -box.prd[d] : hi ? box.prd[d] : 0.0;
+      code[d] = lo ? 0 : hi ? 2 : 3;  // 3: no entry
+      any |= lo || hi;
+    }
+  }
+  // bits 0..2: shifted in x, y, z; bits 6.. the neighbour
+  __device__ __forceinline__ int encode(int e) const {
+    return (e & ~63) | ((e & 3) == code[0] ? 1 : 0) | (((e >> 2) & 3) == code[1] ? 2 : 0) |
+           (((e >> 4) & 3) == code[2] ? 4 : 0);
+  }
+  // x_i - (x_j + shift): x_j + 0.0 is x_j exactly
+  template <bool WRAP>
+  __device__ __forceinline__ void sep(unsigned e, const double4 &xi, const double4 &xj,
+                                      double &dx, double &dy, double &dz) const {
+    if (WRAP) {
+      dx = __dsub_rn(xi.x, __dadd_rn(xj.x, (e & 1u) ? v[0] : 0.0));
+      dy = __dsub_rn(xi.y, __dadd_rn(xj.y, (e & 2u) ? v[1] : 0.0));
+      dz = __dsub_rn(xi.z, __dadd_rn(xj.z, (e & 4u) ? v[2] : 0.0));
+    } else {
+      dx = __dsub_rn(xi.x, xj.x);
+      dy = __dsub_rn(xi.y, xj.y);
+      dz = __dsub_rn(xi.z, xj.z);
+    }
+  }
+};
+
 // This lane's entries (lane, lane + TPA, ... of the atom's list), the first
-// `slots` of them in shared memory.
-template <int TPA>
+// `slots` of them in shared memory; ENCODE: with MultiShift's bits.
+template <int TPA, bool ENCODE>
 struct MultiList {
+  const MultiShift *shift;
   const int *nlist;
   int *mine;
   int stride, i, lane, slots, cnt;
   __device__ __forceinline__ MultiList(const int *nl, int stride_, int i_, int num, int lane_,
-                                       int slots_, int *s_list)
-      : nlist(nl), mine(s_list + threadIdx.x), stride(stride_), i(i_), lane(lane_), slots(slots_),
+                                       int slots_, int *s_list, const MultiShift *shift_)
+      : shift(shift_), nlist(nl), mine(s_list + threadIdx.x), stride(stride_), i(i_), lane(lane_), slots(slots_),
         cnt(num > lane_ ? (num - lane_ + TPA - 1) / TPA : 0) {
     for (int k = 0; k < cnt && k < slots; k++) mine[k * kMultiThreads] = fetch(k);
   }
   __device__ __forceinline__ int fetch(int k) const {
-    return nlist[md_slab(lane + TPA * k, i, stride)];
+    const int e = nlist[md_slab(lane + TPA * k, i, stride)];
+    return ENCODE ? shift->encode(e) : e;
   }
   __device__ __forceinline__ unsigned entry(int k) const {
     return (unsigned)(k < slots ? mine[k * kMultiThreads] : fetch(k));

@@ -123,14 +123,17 @@ struct EamSide {
       sz = shifts(cz, a.box.ncell[2], a.box.prd[2]);
     }
   }
-  // FP64 separation of entry e at xj
-  __device__ __forceinline__ void sep(unsigned e, const double4 &xj, double &delx, double &dely,
-                                      double &delz) const {
+  // FP64 separation x - (x_j + shift) of entry e (WRAP as in MultiShift; the
+  // periodic shift is always formed: one path without it for interior atoms
+  // measured no gain here)
+  template <bool WRAP>
+  __device__ __forceinline__ void sep(unsigned e, const double4 &x, const double4 &xj,
+                                      double &delx, double &dely, double &delz) const {
     int j, dx, dy, dz;
     decode(e, j, dx, dy, dz);
-    delx = __dsub_rn(xi.x, __dadd_rn(xj.x, pick(sx, dx)));
-    dely = __dsub_rn(xi.y, __dadd_rn(xj.y, pick(sy, dy)));
-    delz = __dsub_rn(xi.z, __dadd_rn(xj.z, pick(sz, dz)));
+    delx = __dsub_rn(x.x, __dadd_rn(xj.x, pick(sx, dx)));
+    dely = __dsub_rn(x.y, __dadd_rn(xj.y, pick(sy, dy)));
+    delz = __dsub_rn(x.z, __dadd_rn(xj.z, pick(sz, dz)));
   }
   // minimum-image separation from the fixed-point coordinates
   __device__ __forceinline__ void sep(const int4 &xj, float &delx, float &dely,
@@ -145,9 +148,10 @@ struct EamSide {
 // before the atom's count.  Branch-free, so that the four entries' chains and
 // table loads overlap; an entry past mm or past the cutoff reads row 0 (one
 // address for all of them) and adds nothing.
-template <bool SINGLE>
-__device__ __forceinline__ void rho_four(const EamArgs &a, const EamSide<false, SINGLE> &me,
-                                         const int *t2rhor, const unsigned (&ee)[4],
+// `of` forms the separations (the atom's side, or MultiShift).
+template <bool SINGLE, class S>
+__device__ __forceinline__ void rho_four(const EamArgs &a, const S &of,
+                                         const EamSide<false, SINGLE> &me, const int *t2rhor, const unsigned (&ee)[4],
                                          const double4 (&xj)[4], int mm, double &rho) {
   // one element: the density spline row of every pair
   const double *rrow = SINGLE ? a.rhor + (size_t)t2rhor[a.ntp1 + 1] * (a.nr + 1) * 8 : nullptr;
@@ -155,7 +159,7 @@ __device__ __forceinline__ void rho_four(const EamArgs &a, const EamSide<false, 
 #pragma unroll
   for (int u = 0; u < 4; u++) {
     double delx, dely, delz;
-    me.sep(ee[u], xj[u], delx, dely, delz);
+    of.template sep<true>(ee[u], me.xi, xj[u], delx, dely, delz);
     const double rsq = dsq3(delx, dely, delz);
     const bool in = u < mm && rsq < a.cutforcesq;
     int m;
@@ -200,8 +204,9 @@ __device__ __forceinline__ void rho_four(const EamArgs &a, const EamSide<true, S
 }
 
 // Force terms (and, with EV, energy and virial) of four entries; fpq their F'.
-template <bool EV, bool SINGLE>
-__device__ __forceinline__ void force_four(const EamArgs &a, const EamSide<false, SINGLE> &me,
+template <bool EV, bool SINGLE, class S>
+__device__ __forceinline__ void force_four(const EamArgs &a, const S &of,
+                                           const EamSide<false, SINGLE> &me,
                                            const int *t2rhor, const int *t2z2r, double fpi,
                                            const unsigned (&ee)[4], const double4 (&xj)[4],
                                            const double (&fpq)[4], int mm, double &fx, double &fy,
@@ -209,7 +214,7 @@ __device__ __forceinline__ void force_four(const EamArgs &a, const EamSide<false
 #pragma unroll
   for (int u = 0; u < 4; u++) {
    double delx, dely, delz;
-   me.sep(ee[u], xj[u], delx, dely, delz);
+   of.template sep<true>(ee[u], me.xi, xj[u], delx, dely, delz);
    const double rsq = dsq3(delx, dely, delz);
    const bool in = u < mm && rsq < a.cutforcesq;
    const int tj = SINGLE ? 1 : (int)xj[u].w;
@@ -374,24 +379,23 @@ __global__ void __launch_bounds__(128) k_eam_rho(EamArgs a, const double4 *__res
     const int num = a.numneigh[i];
     EamSide<MIXED, SINGLE> me;
     me.init(a, MIXED ? 0 : a.cell[i]);
+    if (MIXED) me.qi = xq[i], ti = me.ti = me.qi.w;
+    else me.xi = x4[i], ti = me.ti = (int)me.xi.w;
     // four entries ee of this lane (walk_list); the first mm lie before the
     // atom's count
-    auto four = [&](const unsigned (&ee)[4], int mm) {
+    walk_list<TPA>(a.nlist, a.stride, i, num, lane, [&](const unsigned (&ee)[4], int mm) {
       if constexpr (!MIXED) {
         double4 xj[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) xj[u] = ld_pos<false>(&x4[u < mm ? md_entry_j(ee[u]) : i]);
-        rho_four<SINGLE>(a, me, s_t2rhor, ee, xj, mm, rho);
+        rho_four<SINGLE>(a, me, me, s_t2rhor, ee, xj, mm, rho);
       } else {
         int4 xs[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) xs[u] = xq[md_entry_j(ee[u])];
         rho_four<SINGLE>(a, me, s_t2rhor, xs, rho);
       }
-    };
-    if (MIXED) me.qi = xq[i], ti = me.ti = me.qi.w;
-    else me.xi = x4[i], ti = me.ti = (int)me.xi.w;
-    walk_list<TPA>(a.nlist, a.stride, i, num, lane, four);
+    });
   }
   rho = lane_sum<TPA>(rho);
   double acc[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -440,7 +444,7 @@ __global__ void __launch_bounds__(128) k_eam_force(EamArgs a, const double4 *__r
     const float fpf = MIXED ? a.fpf[i] : 0.f;
     // four entries ee of this lane (walk_list); the first mm lie before the
     // atom's count
-    auto four = [&](const unsigned (&ee)[4], int mm) {
+    walk_list<TPA>(a.nlist, a.stride, i, num, lane, [&](const unsigned (&ee)[4], int mm) {
       if constexpr (!MIXED) {
         double4 xj[4];
         double fpq[4];
@@ -450,7 +454,8 @@ __global__ void __launch_bounds__(128) k_eam_force(EamArgs a, const double4 *__r
           xj[u] = ld_pos<false>(&(SINGLE ? a.xf : x4)[jj]);
           fpq[u] = SINGLE ? xj[u].w : a.fp[jj];
         }
-        force_four<EV, SINGLE>(a, me, s_t2rhor, s_t2z2r, fpd, ee, xj, fpq, mm, fx, fy, fz, acc);
+        force_four<EV, SINGLE>(a, me, me, s_t2rhor, s_t2z2r, fpd, ee, xj, fpq, mm, fx, fy,
+                                     fz, acc);
       } else {
         int4 xs[4];
         float fpq[4];
@@ -462,8 +467,7 @@ __global__ void __launch_bounds__(128) k_eam_force(EamArgs a, const double4 *__r
         }
         force_four<EV, SINGLE>(a, me, s_t2rhor, s_t2z2r, fpf, xs, fpq, fx, fy, fz, acc);
       }
-    };
-    walk_list<TPA>(a.nlist, a.stride, i, num, lane, four);
+    });
   }
   fx = lane_sum<TPA>(fx);
   fy = lane_sum<TPA>(fy);
@@ -521,11 +525,12 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
   for (int k = threadIdx.x; k < a.ntp1; k += blockDim.x) s_t2frho[k] = a.t2frho[k];
   if (blockIdx.x == 0)
     for (int k = threadIdx.x; k < m.bar_words; k += blockDim.x) m.bar_next[k] = 0u;
-  const int i = (blockIdx.x * kMultiThreads + threadIdx.x) / TPA;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / TPA;
   const int lane = threadIdx.x % TPA;
   const bool active = i < a.n;
-  const MultiList<TPA> list(a.nlist, a.stride, active ? i : 0, active ? a.numneigh[i] : 0, lane,
-                            m.slots, s_list);
+  const MultiShift shift(!MIXED && active ? a.cell[i] : md_cell_pack(1, 1, 1), a.box);
+  const MultiList<TPA, !MIXED> list(a.nlist, a.stride, active ? i : 0,
+                                    active ? a.numneigh[i] : 0, lane, m.slots, s_list, &shift);
   MultiState<TPA> st(s_state);
   EamSide<MIXED, SINGLE> me;
   me.ti = 1;
@@ -565,7 +570,7 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
       for (int d = 0; d < DEPTH; d++) {
         if (d > 0 && k + 4 * d >= list.cnt) break;
         if constexpr (MIXED) rho_four<SINGLE>(a, me, s_t2rhor, xs[d], rho);
-        else rho_four<SINGLE>(a, me, s_t2rhor, ee[d], xj[d], list.cnt - k - 4 * d, rho);
+        else rho_four<SINGLE>(a, shift, me, s_t2rhor, ee[d], xj[d], list.cnt - k - 4 * d, rho);
       }
     }
     rho = lane_sum<TPA>(rho);
@@ -619,8 +624,8 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
           force_four<false, SINGLE>(a, me, s_t2rhor, s_t2z2r, (float)fpi, xs[d], fpf[d], fx, fy,
                                     fz, acc);
         else
-          force_four<false, SINGLE>(a, me, s_t2rhor, s_t2z2r, fpi, ee[d], xj[d], fpd[d],
-                                    list.cnt - k - 4 * d, fx, fy, fz, acc);
+          force_four<false, SINGLE>(a, shift, me, s_t2rhor, s_t2z2r, fpi, ee[d], xj[d],
+                                          fpd[d], list.cnt - k - 4 * d, fx, fy, fz, acc);
       }
     }
     fx = lane_sum<TPA>(fx);

@@ -112,9 +112,26 @@ struct Fp64Pairs {
     interior = cx >= 1 && cx + 2 <= box.ncell[0] && cy >= 1 && cy + 2 <= box.ncell[1] &&
                cz >= 1 && cz + 2 <= box.ncell[2];
   }
-  // the first m of four entries ee with their positions xj
+  // x_i - (x_j + shift) of entry e
   template <bool WRAP>
-  __device__ __forceinline__ void four(const double4 &xi, const unsigned (&ee)[4],
+  __device__ __forceinline__ void sep(unsigned e, const double4 &xi, const double4 &xj,
+                                      double &delx, double &dely, double &delz) const {
+    if (WRAP) {
+      int j, dx, dy, dz;
+      decode(e, j, dx, dy, dz);
+      delx = __dsub_rn(xi.x, __dadd_rn(xj.x, pick(sx, dx)));
+      dely = __dsub_rn(xi.y, __dadd_rn(xj.y, pick(sy, dy)));
+      delz = __dsub_rn(xi.z, __dadd_rn(xj.z, pick(sz, dz)));
+    } else {
+      delx = __dsub_rn(xi.x, xj.x);
+      dely = __dsub_rn(xi.y, xj.y);
+      delz = __dsub_rn(xi.z, xj.z);
+    }
+  }
+  // the first m of four entries ee with their positions xj; `of` forms the
+  // separations (this, or MultiShift)
+  template <bool WRAP, class S>
+  __device__ __forceinline__ void four(const S &of, const double4 &xi, const unsigned (&ee)[4],
                                        const double4 (&xj)[4], int m, double &fx, double &fy,
                                        double &fz, double (&acc)[7]) const {
     const int ti = (int)xi.w;
@@ -124,17 +141,7 @@ struct Fp64Pairs {
 #pragma unroll
     for (int u = 0; u < 4; u++) {
       double delx, dely, delz;
-      if (WRAP) {
-        int j, dx, dy, dz;
-        decode(ee[u], j, dx, dy, dz);
-        delx = __dsub_rn(xi.x, __dadd_rn(xj[u].x, pick(sx, dx)));
-        dely = __dsub_rn(xi.y, __dadd_rn(xj[u].y, pick(sy, dy)));
-        delz = __dsub_rn(xi.z, __dadd_rn(xj[u].z, pick(sz, dz)));
-      } else {
-        delx = __dsub_rn(xi.x, xj[u].x);
-        dely = __dsub_rn(xi.y, xj[u].y);
-        delz = __dsub_rn(xi.z, xj[u].z);
-      }
+      of.template sep<WRAP>(ee[u], xi, xj[u], delx, dely, delz);
       const double rsq = dsq3(delx, dely, delz);
       const int tt = ti * ntp1 + (int)xj[u].w;
       const bool in = u < m && rsq < (SINGLE ? cutsq1 : tab[0 * nt2 + tt]);
@@ -184,10 +191,11 @@ __device__ __forceinline__ void lj_atom_fp64(const PairArgs &a, const double4 *_
       double4 xj[4];
 #pragma unroll
       for (int u = 0; u < 4; u++) xj[u] = ld_pos<false>(&x4[u < m ? md_entry_j(ee[u]) : i]);
-      pairs.template four<WRAP>(xi, ee, xj, m, fx, fy, fz, acc);
+      pairs.template four<WRAP>(pairs, xi, ee, xj, m, fx, fy, fz, acc);
     });
   };
-  if (pairs.interior) slabs(std::false_type{});
+  // one path per warp: lanes on either path would run one after the other
+  if (__all_sync(__activemask(), pairs.interior)) slabs(std::false_type{});
   else slabs(std::true_type{});
 }
 
@@ -462,9 +470,12 @@ __global__ void __launch_bounds__(128) k_lj_step(PairArgs a, StepArgs s) {
 // wants a rebuild for; every block knows that from the barrier's word.
 // Microseconds per step, one launch each (with the decision kernel and gaps)
 // against several: 864 atoms mixed, 8 lanes, 11 -> 4.3; 32,000 mixed, 4
-// lanes, 15.7 -> 9.0; 32,000 FP64 25 -> 18.  Of the 9.0, 2.5 to 3 are the
-// barrier and the half-steps, the rest the gathers (each SM's L1 starts cold
-// after every barrier).
+// lanes, 15.7 -> 8.6; 32,000 FP64 25 -> 11; 4,000 FP64 15 -> 4.5.  Of the
+// 8.6, 2.5 to 3 are the barrier and the half-steps, the rest the pair loop.
+// Every warp waits for the slowest one at each step, so the FP64 pair loop is
+// kept even: one path per warp (lanes with and without periodic shifts ran
+// one after the other), and shifts by one bit per dimension (MultiShift);
+// that took the two FP64 cases from 18 and 8 us.
 template <int TPA, bool SINGLE, bool MIXED, int DEPTH>
 __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
     k_lj_multi(PairArgs a, StepArgs s, MultiArgs m) {
@@ -484,11 +495,12 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
     }
   if (blockIdx.x == 0)
     for (int k = threadIdx.x; k < m.bar_words; k += blockDim.x) m.bar_next[k] = 0u;
-  const int i = (blockIdx.x * kMultiThreads + threadIdx.x) / TPA;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / TPA;
   const int lane = threadIdx.x % TPA;
   const bool active = i < a.n;
-  const MultiList<TPA> list(a.nlist, a.stride, active ? i : 0, active ? a.numneigh[i] : 0, lane,
-                            m.slots, s_list);
+  const MultiShift shift(!MIXED && active ? a.cell[i] : md_cell_pack(1, 1, 1), a.box);
+  const MultiList<TPA, !MIXED> list(a.nlist, a.stride, active ? i : 0,
+                                    active ? a.numneigh[i] : 0, lane, m.slots, s_list, &shift);
   const int cnt = list.cnt;
   auto entry = [&](int k) { return list.entry(k); };
   MultiState<TPA> st(s_state);
@@ -501,7 +513,8 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
   }
   __syncthreads();
   const MixedPairs<false, SINGLE, true> mp(a, a.box, tabf, nt2);
-  const Fp64Pairs<false, SINGLE> dp(a, a.box, !MIXED && active ? a.cell[i] : 0, tab, nt2);
+  const Fp64Pairs<false, SINGLE> dp(a, a.box, 0, tab, nt2);
+  const bool wrap = __any_sync(0xffffffffu, !MIXED && active && shift.any);
   int ago = m.ago;
   for (int j = 0;; j++) {
     double fx = 0.0, fy = 0.0, fz = 0.0;
@@ -535,11 +548,11 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
             }
 #pragma unroll
           for (int d = 0; d < DEPTH; d++)
-            dp.template four<WRAP>(xi, ee[d], xs[d], min(G, cnt - k - d * G), fx, fy, fz, acc);
+            dp.template four<WRAP>(shift, xi, ee[d], xs[d], min(G, cnt - k - d * G), fx, fy, fz, acc);
         }
       };
-      if (dp.interior) walk(std::false_type{});
-      else walk(std::true_type{});
+      if (wrap) walk(std::true_type{});
+      else walk(std::false_type{});
     }
     fx = lane_sum<TPA>(fx);
     fy = lane_sum<TPA>(fy);
