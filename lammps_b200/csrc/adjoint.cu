@@ -403,7 +403,8 @@ cudaError_t md_adj_backward(b200_ctx *c, const double *lj1, const double *lj2,
 
 // caller-order device positions -> the context's sorted FP64 positions
 // (types kept, image flags restarted); the next build wraps and re-sorts.
-// `held` keeps them as they came.
+// `held` keeps them as they came (EamArgs::xf's memory: an lj/cut context has no
+// other use for it).
 __global__ void k_adj_positions(int n, const int *__restrict__ orig, const double *__restrict__ x,
                                 double4 *__restrict__ x4, int *__restrict__ image,
                                 double *__restrict__ held) {
@@ -419,8 +420,8 @@ __global__ void k_adj_positions(int n, const int *__restrict__ orig, const doubl
 }
 
 cudaError_t md_adj_positions(b200_ctx *c, const double *x) {
-  k_adj_positions<<<md_blocks(c->n, 256), 256, 0, c->stream>>>(c->n, c->orig, x, c->x4, c->image,
-                                                               c->adj_x);
+  k_adj_positions<<<md_blocks(c->n, 256), 256, 0, c->stream>>>(
+      c->n, c->orig, x, c->x4, c->image, reinterpret_cast<double *>(c->xf));
   c->launches++;
   return cudaGetLastError();
 }
@@ -436,7 +437,7 @@ __global__ void k_adj_compare(int m, const unsigned long long *__restrict__ a,
 cudaError_t md_adj_compare(b200_ctx *c, const double *x, int *diff) {
   k_adj_compare<<<md_blocks(3 * c->n, 256), 256, 0, c->stream>>>(
       3 * c->n, reinterpret_cast<const unsigned long long *>(x),
-      reinterpret_cast<const unsigned long long *>(c->adj_x), diff);
+      reinterpret_cast<const unsigned long long *>(c->xf), diff);
   c->launches++;
   return cudaGetLastError();
 }

@@ -1134,7 +1134,7 @@ int b200_destroy(b200_ctx *c) {
   dfree(c->cell_count); dfree(c->cell_start); dfree(c->scan_tmp);
   dfree(c->slot); dfree(c->perm); dfree(c->cell_tmp);
   dfree(c->nlist); dfree(c->numneigh); dfree(c->partial); dfree(c->counter); dfree(c->ev);
-  dfree(c->adj_gs); dfree(c->adj_gtab); dfree(c->adj_x);
+  dfree(c->adj_gs); dfree(c->adj_gtab);
   dfree(c->d_rep_box); dfree(c->d_rep_of_atom); dfree(c->d_rep_cell_base); dfree(c->d_tile_rep);
   dfree(c->d_rep_tile_base); 
   dfree(c->status); dfree(c->rows); dfree(c->tables_dev);
@@ -2235,10 +2235,6 @@ int b200_adj_set_positions(b200_ctx *c, const double *x) {
   if (!c->have_atoms) return set_err(c, B200_ERR_STATE, "no atoms uploaded");
   CK(cudaSetDevice(c->device));
   c->adj_held = false;
-  if (c->adj_x_n < c->n) {
-    CK(dalloc(&c->adj_x, 3 * (size_t)c->stride));
-    c->adj_x_n = c->stride;
-  }
   CK(md_adj_positions(c, x));
   int rc = prepare(c);
   if (rc) return rc;

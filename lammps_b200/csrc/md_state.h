@@ -134,7 +134,9 @@ struct b200_ctx {
   int out_next = 0;
   double *rho = nullptr, *fp = nullptr;
   float *fpf = nullptr;
-  double4 *xf = nullptr;  // one element: position and F' records (EamArgs::xf)
+  // eam, one element: position and F' records (EamArgs::xf); force matching:
+  // the positions given (adj_held)
+  double4 *xf = nullptr;
   // split EAM compute (b200_eam_density, then b200_eam_force): the eflag /
   // vflag of the density call and its per-atom embedding energies
   int eam_split_eflag = -1, eam_split_vflag = -1;
@@ -171,9 +173,9 @@ struct b200_ctx {
   double *adj_gs = nullptr;    // force-matching scratch: G in the sorted order
   double *adj_gtab = nullptr;  // force-matching parameter gradients
   int adj_n = 0;
-  double *adj_x = nullptr;     // the positions b200_adj_set_positions was given
-  int adj_x_n = 0;
-  bool adj_held = false;       // nothing has changed atoms, lists or settings since
+  // xf holds the positions b200_adj_set_positions was given, and nothing has
+  // changed atoms, lists or settings since
+  bool adj_held = false;
   double *ev = nullptr;          // [0] eng, [1..6] virial, [7] sum m v^2
   int *status = nullptr;         // ST_* words
   int *status_host = nullptr;    // pinned mirror
