@@ -969,9 +969,11 @@ namespace {
 template <int TPA, int DEPTH>
 const void *multi_kernel(const b200_ctx *c) {
   const bool single = c->ntypes == 1;
+  // eight lanes hold about ten entries each: all of them in flight at once
+  constexpr int MD = DEPTH == 2 && TPA == 8 ? 3 : DEPTH;
   if (c->prec == B200_PREC_MIXED)
-    return single ? (const void *)k_lj_multi<TPA, true, true, DEPTH>
-                  : (const void *)k_lj_multi<TPA, false, true, DEPTH>;
+    return single ? (const void *)k_lj_multi<TPA, true, true, MD>
+                  : (const void *)k_lj_multi<TPA, false, true, MD>;
   return single ? (const void *)k_lj_multi<TPA, true, false, DEPTH>
                 : (const void *)k_lj_multi<TPA, false, false, DEPTH>;
 }
