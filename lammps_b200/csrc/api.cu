@@ -1164,7 +1164,7 @@ const char *b200_last_error(const b200_ctx *c) { return c ? c->err.c_str() : "nu
 long long b200_bytes(const b200_ctx *c) {
   if (!c) return 0;
   long long s = (long long)c->stride;
-  long long b = s * (2 * 32 + 2 * 24 + 24 + 5 * 4 + 16 + 32 + 16 + 4) + c->nlist_alloc * 4 +
+  long long b = s * (3 * 32 + 2 * 24 + 24 + 5 * 4 + 16 + 32 + 16 + 4) + c->nlist_alloc * 4 +
                 (long long)c->ncell_alloc * 8;
   return b;
 }

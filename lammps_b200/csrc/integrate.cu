@@ -259,8 +259,10 @@ MultiPlan md_multi_shape(const b200_ctx *c, const void *lean, const void *deep) 
   p.smem = md_multi_smem(c->tpa, p.slots);
   int fit = 0;
   cudaError_t e = cudaSuccess;
+  // the opt-in is the kernel's, not the launch's: the same value from every
+  // context, whatever its own size
   if (p.smem > 40 * 1024)
-    e = cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    e = cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, p.kernel, p.threads, p.smem);
   if (e != cudaSuccess) {

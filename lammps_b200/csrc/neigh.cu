@@ -816,7 +816,7 @@ __global__ void __launch_bounds__(kNeighThreads, 8) k_neigh_tiles(NeighArgs A) {
               if (me < 32u && (info & 0xF0000) == 0x40000) x &= ~(0x80000000u >> me);
               if (!act) x = 0;
             }
-            // words kept of this atom in this round: bits 0, 8, 16, 24
+            // words kept of this atom, these four chunks: bits 0, 8, 16, 24
             const unsigned full = (__ballot_sync(0xffffffffu, x != 0u) >> a) & 0x01010101u;
             if (x) {
               const int k = kept + cols * __popc(full & below);
