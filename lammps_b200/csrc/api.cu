@@ -570,6 +570,7 @@ int autotune_step(b200_ctx *c) {
   if (rc0) return rc0;
   const int mail_save[2] = {c->mail_host[0], c->mail_host[1]};
   const int parity_save = c->pos_parity;
+  const int tpa_was = c->tpa;  // 0: the search at setup
   const bool lj = c->pstyle == B200_PAIR_LJ_CUT;
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
@@ -638,6 +639,11 @@ int autotune_step(b200_ctx *c) {
       best = tmin[k];
       best_tpa = cand[k];
     }
+  // the repeat changes the shape only where that clearly pays: near-ties
+  // would otherwise go either way from run to run, and with them the
+  // summation order
+  for (int k = 0; k < 4; k++)
+    if (tpa_was == cand[k] && best > 0.93f * tmin[k]) best_tpa = tpa_was;
   c->tpa = best_tpa;
   c->tuned = true;
   return B200_OK;
