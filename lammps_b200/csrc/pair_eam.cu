@@ -255,7 +255,8 @@ __device__ __forceinline__ void force_four(const EamArgs &a, const S &of,
    const double phi = in ? z2 * recip : 0.0;
    const double phip = z2p * recip - phi * recip;
    const double psip = fpi * rhojp + fpq[u] * rhoip + phip;
-   const double fpair = in ? -psip * recip : 0.0;
+   const double fpair = -psip * recip;
+   drop_unless(in, delx, dely, delz);
    fx += delx * fpair;
    fy += dely * fpair;
    fz += delz * fpair;

@@ -129,15 +129,17 @@ struct Fp64Pairs {
     }
   }
   // the first m of four entries ee with their positions xj; `of` forms the
-  // separations (this, or MultiShift)
-  template <bool WRAP, class S>
+  // separations (this, or MultiShift).  FINITE: every xj is finite, or the
+  // caller looks at the sums and calls again without it.
+  template <bool WRAP, bool FINITE, class S>
   __device__ __forceinline__ void four(const S &of, const double4 &xi, const unsigned (&ee)[4],
                                        const double4 (&xj)[4], int m, double &fx, double &fy,
                                        double &fz, double (&acc)[7]) const {
     const int ti = (int)xi.w;
     // Branch-free: an FP64 pair term is a chain of about twenty dependent
     // operations, and only without branches do the four entries' chains
-    // overlap.  An entry past m or past the cutoff gets a zero factor.
+    // overlap.  An entry past m or past the cutoff gets a zero separation
+    // (drop_unless) or, with FINITE, a zero factor.
 #pragma unroll
     for (int u = 0; u < 4; u++) {
       double delx, dely, delz;
@@ -150,7 +152,8 @@ struct Fp64Pairs {
       const double r2inv = rcp_nr(in ? rsq : 1.0);
       const double r6inv = r2inv * r2inv * r2inv;
       const double forcelj = r6inv * (c1 * r6inv - c2);
-      const double fpair = in ? forcelj * r2inv : 0.0;
+      const double fpair = !FINITE || in ? forcelj * r2inv : 0.0;
+      if (!FINITE) drop_unless(in, delx, dely, delz);
       fx += delx * fpair;
       fy += dely * fpair;
       fz += delz * fpair;
@@ -191,7 +194,7 @@ __device__ __forceinline__ void lj_atom_fp64(const PairArgs &a, const double4 *_
       double4 xj[4];
 #pragma unroll
       for (int u = 0; u < 4; u++) xj[u] = ld_pos<false>(&x4[u < m ? md_entry_j(ee[u]) : i]);
-      pairs.template four<WRAP>(pairs, xi, ee, xj, m, fx, fy, fz, acc);
+      pairs.template four<WRAP, false>(pairs, xi, ee, xj, m, fx, fy, fz, acc);
     });
   };
   // one path per warp: lanes on either path would run one after the other
@@ -533,8 +536,8 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
       }
     } else {
       const double4 *x4 = static_cast<const double4 *>(s.cur);
-      auto walk = [&](auto wrap_tag) {
-        constexpr bool WRAP = decltype(wrap_tag)::value;
+      auto walk = [&](auto wrap_tag, auto finite_tag) {
+        constexpr bool WRAP = decltype(wrap_tag)::value, FINITE = decltype(finite_tag)::value;
         for (int k = 0; k < cnt; k += G * DEPTH) {
           unsigned ee[DEPTH][G];
           double4 xs[DEPTH][G];
@@ -548,11 +551,19 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
             }
 #pragma unroll
           for (int d = 0; d < DEPTH; d++)
-            dp.template four<WRAP>(shift, xi, ee[d], xs[d], min(G, cnt - k - d * G), fx, fy, fz, acc);
+            dp.template four<WRAP, FINITE>(shift, xi, ee[d], xs[d], min(G, cnt - k - d * G), fx, fy,
+                                           fz, acc);
         }
       };
-      if (wrap) walk(std::true_type{});
-      else walk(std::false_type{});
+      if (wrap) walk(std::true_type{}, std::true_type{});
+      else walk(std::false_type{}, std::true_type{});
+      // a neighbour that is not finite (or a force that is not): once more,
+      // dropping rejected pairs (32,000 atoms: 1,725 us a run with this, 1,720
+      // without, 1,803 with drop_unless in the loop)
+      if (!isfinite(fx + fy + fz)) {
+        fx = fy = fz = 0.0;
+        walk(std::true_type{}, std::false_type{});
+      }
     }
     fx = lane_sum<TPA>(fx);
     fy = lane_sum<TPA>(fy);
