@@ -251,6 +251,12 @@ int b200_set_timing(b200_ctx *ctx, int on);
    that do not want graphs).  Both follow the same host-mirrored rebuild
    schedule and give identical results. */
 int b200_set_graphs(b200_ctx *ctx, int on);
+/* The grid barriers of the cooperative launches (several MD steps, the cell sort
+   of a small box) give up after a few seconds.  The call that finds it returns
+   B200_ERR_TIMEOUT; the context stays usable, but its atoms are gone and have to
+   be uploaded again.  on = 1 makes them give up at once, to test a caller's
+   handling of that error; on = 0 (default) ends it. */
+int b200_expire_waits(b200_ctx *ctx, int on);
 int b200_get_timing(b200_ctx *ctx, double phase_ms[5], long long *steps, int reset);
 /* Device time of every step timed since the last reset (milliseconds, from
    the step's first phase event to its last; timing must be on): *count

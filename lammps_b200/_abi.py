@@ -68,6 +68,7 @@ SIGNATURES = {
     "b200_kernel_launches": (C.c_longlong, [_vp]),
     "b200_set_timing": (C.c_int, [_vp, C.c_int]),
     "b200_set_graphs": (C.c_int, [_vp, C.c_int]),
+    "b200_expire_waits": (C.c_int, [_vp, C.c_int]),
     "b200_get_timing": (C.c_int, [_vp, _dp, C.POINTER(C.c_longlong), C.c_int]),
     "b200_stream": (_vp, [_vp]),
     "b200_get_step_times": (C.c_int, [_vp, _dp, C.c_int, _ip, C.c_int]),

@@ -488,15 +488,25 @@ int small_read(b200_ctx *c, void *host, const void *dev, size_t bytes) {
 
 int read_status(b200_ctx *c) { return small_read(c, c->status_host, c->status, ST_COUNT * sizeof(int)); }
 
+// A barrier gave up: some blocks have gone on and others not, so the atoms are
+// in no defined state.  Clears what the launch left behind (barrier words, cell
+// counts, the status word); the next call has to bring the atoms again.
+int barrier_error(b200_ctx *c) {
+  c->have_atoms = c->sorted_once = c->adj_held = false;
+  c->status_host[ST_BARRIER] = 0;
+  CK(cudaMemsetAsync(c->bar, 0, (2 * MD_BAR_WORDS + 4) * sizeof(unsigned), c->stream));
+  if (c->cell_count)
+    CK(cudaMemsetAsync(c->cell_count, 0, (size_t)c->ncell_alloc * sizeof(int), c->stream));
+  CK(cudaMemsetAsync(c->status + ST_BARRIER, 0, sizeof(int), c->stream));
+  return set_err(c, B200_ERR_TIMEOUT,
+                 "a grid barrier of a cooperative launch timed out: upload the atoms again");
+}
+
 int status_errors(b200_ctx *c) {
+  if (c->status_host[ST_BARRIER]) return barrier_error(c);
   if (c->status_host[ST_LOST])
     return set_err(c, B200_ERR_LOST_ATOMS,
                    "Lost atoms: a coordinate is not finite or moved beyond one box length");
-  if (c->status_host[ST_BARRIER]) {
-    cudaMemsetAsync(c->bar, 0, (2 * MD_BAR_WORDS + 4) * sizeof(unsigned), c->stream);
-    cudaMemsetAsync(c->status + ST_BARRIER, 0, sizeof(int), c->stream);
-    return set_err(c, B200_ERR_CUDA, "a grid barrier of a cooperative launch timed out");
-  }
   if (c->status_host[ST_OVERFLOW])
     return set_err(c, B200_ERR_NEIGH_OVERFLOW,
                    "Neighbor list overflow, boost neigh_modify one (need %d, have %d)",
@@ -534,21 +544,22 @@ int rebuild_sync(b200_ctx *c) {
   return set_err(c, B200_ERR_NEIGH_OVERFLOW, "Neighbor list overflow, boost neigh_modify one");
 }
 
-// `nsteps` MD steps in one launch
-// (md_lj_multi, md_eam_multi), from `ago` steps since the build, under the given schedule;
-// the barrier words' other set becomes current
 MultiPlan multi_plan(const b200_ctx *c) {
   return c->pstyle == B200_PAIR_LJ_CUT ? md_lj_multi_plan(c) : md_eam_multi_plan(c);
 }
 
-int launch_multi(b200_ctx *c, const MultiPlan &plan, int nsteps, int ago, double dtv, double dtf, int every,
-                 int check) {
+// `nsteps` MD steps in one launch (md_lj_multi, md_eam_multi), from `ago` steps
+// since the build, under the given schedule; the barrier words' other set
+// becomes current
+int launch_multi(b200_ctx *c, const MultiPlan &plan, int nsteps, int ago, double dtv, double dtf,
+                 int every, int check) {
   MultiArgs m;
   m.nsteps = nsteps;
   m.ago = ago;
   m.bar = c->bar + c->bar_set * MD_BAR_WORDS;
   m.bar_next = c->bar + (c->bar_set ^ 1) * MD_BAR_WORDS;
   m.bar_words = MD_BAR_WORDS;
+  if (c->expire_waits) CK(cudaMemsetAsync(m.bar, kExpireByte, sizeof(unsigned), c->stream));
   CK(c->pstyle == B200_PAIR_LJ_CUT ? md_lj_multi(c, plan, dtv, dtf, m, every, check)
                                    : md_eam_multi(c, plan, dtv, dtf, m, every, check));
   c->bar_set ^= 1;
@@ -625,13 +636,17 @@ int autotune_step(b200_ctx *c) {
   // back to the buffer the search started from (after a zero-timestep step
   // both buffers hold the same positions)
   if (c->pos_parity != parity_save) md_swap_positions(c);
+  int gave_up = 0;  // a barrier of a trial launch
+  if (!rc) rc = small_read(c, &gave_up, c->status + ST_BARRIER, sizeof(int));
   CK(cudaMemcpyAsync(c->status, status_save, sizeof(status_save), cudaMemcpyHostToDevice,
                      c->stream));
   CK(cudaMemcpyAsync(c->dec_count, &dcount_save, sizeof(int), cudaMemcpyHostToDevice, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   c->mail_host[0] = mail_save[0];
   c->mail_host[1] = mail_save[1];
+  if (rc || gave_up) c->tpa = tpa_was;
   if (rc) return rc;
+  if (gave_up) return barrier_error(c);
   float best = 1e30f;
   int best_tpa = 1;
   for (int k = 0; k < 4; k++)
@@ -924,8 +939,8 @@ int wait_decision(b200_ctx *c, bool *rebuild, int *ago = nullptr) {
   int rc1 = read_status(c);
   if (!rc1) rc1 = small_read(c, &dc, c->dec_count, sizeof(int));
   if (rc1) return rc1;
-  if (c->status_host[ST_BARRIER]) return status_errors(c);
   c->decisions = (unsigned int)dc;
+  if (c->status_host[ST_BARRIER]) return barrier_error(c);
   *rebuild = c->status_host[ST_REBUILD] != 0;
   if (ago) *ago = c->status_host[ST_AGO];
   return B200_OK;
@@ -1015,6 +1030,8 @@ int grow_list(b200_ctx *c, int capacity, bool keep) {
     c->nlist = nl;
     c->nlist_alloc = need;
   }
+  // no entries until the next build, which a barrier's time-out may skip
+  if (!keep) CK(cudaMemsetAsync(c->numneigh, 0, (size_t)c->stride * sizeof(int), c->stream));
   c->capacity = capacity;
   invalidate_graphs(c);
   return B200_OK;
@@ -2185,6 +2202,13 @@ int b200_set_graphs(b200_ctx *c, int on) {
   if (!c) return B200_ERR_ARG;
   c->use_graphs = on != 0;
   invalidate_graphs(c);
+  return B200_OK;
+}
+
+int b200_expire_waits(b200_ctx *c, int on) {
+  if (!c) return B200_ERR_ARG;
+  c->expire_waits = on != 0;
+  invalidate_graphs(c);  // the rebuild's graph holds the sort
   return B200_OK;
 }
 

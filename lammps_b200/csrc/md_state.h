@@ -44,6 +44,9 @@ struct EAMDev {
   bool rhor_sym = false;
 };
 
+// a barrier word filled with this byte holds kBarrierExpired
+constexpr int kExpireByte = 0x80;
+
 // blocks of tables_dev, each TABSZ doubles
 enum { TAB_CUTNEIGHSQ = 0, TAB_CUTSQ, TAB_LJ1, TAB_LJ2, TAB_LJ3, TAB_LJ4, TAB_OFFSET, TAB_COUNT };
 constexpr int TABSZ = (MD_MAXTYPES + 1) * (MD_MAXTYPES + 1);
@@ -192,9 +195,11 @@ struct b200_ctx {
   int *bounce_host = nullptr, *bounce_dev = nullptr;
   int *dec_count = nullptr;
   unsigned int decisions = 0;
-  // barrier words of multi-step launches, two sets used in turn
+  // barrier words of multi-step launches, two sets used in turn, and of the
+  // one-launch sort
   unsigned *bar = nullptr;
   int bar_set = 0;
+  bool expire_waits = false;  // b200_expire_waits
   double *rows = nullptr;        // device thermo rows (9 doubles each)
   int rows_cap = 0;
 

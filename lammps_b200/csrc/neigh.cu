@@ -283,7 +283,9 @@ struct SortArgs {
   double4 *xhold;
   int *status;
   const int *flag;
-  unsigned *bar;  // three barrier words, zero between launches
+  // three barrier words; 0 and 1 are zero between launches, 2 is zeroed after
+  // the first barrier
+  unsigned *bar;
 };
 
 template <bool BATCH>
@@ -291,6 +293,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_sort_all(SortArgs A) {
   if (!rebuild_on(A.flag)) return;
   const int i = blockIdx.x * kSortThreads + threadIdx.x;
   const bool act = i < A.n;
+  const int gave_up = A.status[ST_BARRIER];  // an earlier launch's barrier
   double4 p = make_double4(0, 0, 0, 1);
   double v0 = 0, v1 = 0, v2 = 0;
   int o = 0, img = 0, c = 0, slot = 0, cc[3] = {0, 0, 0};
@@ -306,8 +309,12 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_sort_all(SortArgs A) {
     if (wrap_atom(p, img, cc, box)) atomicExch(&A.status[ST_LOST], 1);
     c = cc[0] + box.ncell[0] * (cc[1] + box.ncell[1] * cc[2]);
     if (BATCH) c += A.reps.cell_base[rep];
-    slot = atomicAdd(&A.cell_count[c], 1);
   }
+  // Looked at before the first change of the cell counts: a launch that gives
+  // up leaves them as they are, and counting on top of them would place atoms
+  // past the arrays.
+  if (__syncthreads_or(gave_up)) return;
+  if (act) slot = atomicAdd(&A.cell_count[c], 1);
   if (md_grid_barrier(A.bar, false, true, A.status) < 0) return;
   if (blockIdx.x == 0) {
     if (threadIdx.x == 0) A.bar[2] = 0u;
@@ -519,6 +526,7 @@ inline int tile_units_of(double per_cell, int tc, bool single) {
 template <int TC, bool SINGLE, bool BATCH>
 __global__ void __launch_bounds__(kNeighThreads, 8) k_neigh_tiles(NeighArgs A) {
   if (!rebuild_on(A.flag)) return;
+  const int gave_up = A.status[ST_BARRIER];  // the sort's barrier
   constexpr int NSX = TC + 2, NST = 9 * NSX;
   constexpr int WPC = kNeighThreads / 32 / TC;  // warps per owned cell
   // batched: this tile's replica, its box and its cells' slice of cell_start
@@ -576,7 +584,8 @@ __global__ void __launch_bounds__(kNeighThreads, 8) k_neigh_tiles(NeighArgs A) {
     s_img[id][2] = (signed char)iz;
     s_start[id + 1] = cnt;
   }
-  __syncthreads();
+  // after a sort that gave up, cell_start may never have been written
+  if (__syncthreads_or(gave_up)) return;
   if (warp == 0) {  // prefix sum of the counts, two per lane
     const int i0 = 2 * lane, i1 = 2 * lane + 1;
     const int c0 = i0 < NST ? s_start[i0 + 1] : 0, c1 = i1 < NST ? s_start[i1 + 1] : 0;
@@ -1208,6 +1217,10 @@ static cudaError_t launch_sort_all(b200_ctx *c, const int *d_flag) {
   A.flag = d_flag;
   A.bar = c->bar + 2 * MD_BAR_WORDS;
   void *args[1] = {&A};
+  if (c->expire_waits) {
+    const cudaError_t e = cudaMemsetAsync(A.bar, kExpireByte, sizeof(unsigned), c->stream);
+    if (e != cudaSuccess) return e;
+  }
   c->launches++;
   return cudaLaunchCooperativeKernel(
       c->nrep ? (const void *)k_sort_all<true> : (const void *)k_sort_all<false>,
