@@ -412,8 +412,9 @@ constexpr int kNeighThreads = 128;
 constexpr int kMaxCols = 384;  // owned atoms of a tile, padded to eight per cell, at most
 // 32-candidate chunks of one cell's nine rows, at most
 constexpr int max_chunks(int tc) { return 192 / tc; }
-// most dynamic shared memory a tile may take (opt-in), in 16-byte units
-constexpr int kStageUnitsMax = 200 * 1024 / 16;
+// most dynamic shared memory a tile may take (opt-in), in 16-byte units: what
+// the kernel's tables (2.8 KB) leave of an SM's 227 KB
+constexpr int kStageUnitsMax = 222 * 1024 / 16;
 
 struct NeighArgs {
   int n, stride, capacity, units, ntp1, pass, units1;
@@ -1047,22 +1048,41 @@ __global__ void k_prefix_ll(int n, const int *__restrict__ cnt, long long *__res
 
 }  // namespace
 
+// Whether a tile of the mean density can be staged (what some atoms more or
+// less then need, the capacity below and its feedback cover).
+static bool mean_tile_fits(const b200_ctx *c, int tc) {
+  const double per_cell = c->ncells > 0 ? (double)c->n / c->ncells : 0.0;
+  const int chunks = 9 * ((int)(3.0 * per_cell / 32.0) + 1), cols = tc * (((int)per_cell + 7) & ~7);
+  return chunks <= max_chunks(tc) && cols <= kMaxCols &&
+         tile_units((int)(9 * (tc + 2) * per_cell), chunks, cols, c->ntypes == 1) <= kStageUnitsMax;
+}
+
 // Cells along x per builder tile.  A tile of two stages 18 cells per owned
-// cell instead of 27, but gives half the CTAs: a 4,000,000-atom run of 60 steps
-// takes 41.1 ms with two and 43.2 with one (four: 41.5), 1,728 cells of copper
-// 3.86 against 3.96, 27 cells 1.35 against 1.32.  Replica boxes are a few
-// cells wide, so half of their two-cell tiles would own one cell (11.78
+// cell instead of 27, but gives half the CTAs and takes more shared memory.
+// One build (sort included), one cell against two per tile:
+//   19 atoms per cell: 1,000 cells 51 and 52 us, 1,331 56 and 52, 5,832 112 and
+//     100, 13,824 226 and 192
+//   27: 1,000 cells 58 and 63 us, 1,331 69 and 65; 32: 8,000 cells 279 and 278
+//   44: 5,832 cells 347 and 331 us; 62: 4,096 cells 444 and 508; 93: 2,744
+//     cells 1,122 and 1,104; from 108 on, where a tile of two no longer fits
+//     (mean_tile_fits), 891 and 7,744
+// so two from seven tiles per SM and up to 50 atoms per cell.  Four cells took
+// 41.5 ms where two take 41.1 (a run of 4,000,000 atoms).  Replica boxes are a
+// few cells wide, so half of their two-cell tiles would own one cell (11.78
 // against 11.66 ms).
 int md_tile_cells(const b200_ctx *c) {
-  return !c->nrep && c->ncells >= 148 * 7 ? 2 : 1;
+  return !c->nrep && c->ncells >= 7 * md_sms(c) && (double)c->n <= 50.0 * c->ncells ? 2 : 1;
 }
 
 // Shared memory of the builder tiles, in 16-byte units: what a tile of the
 // mean density takes, with some room, raised when a build reports a larger
 // tile.  For a batch the mean is the batch's (the common case, at full
 // occupancy); the densest replicas' tiles are built in a second pass with
-// md_stage_cap2.
+// md_stage_cap2.  A box whose mean tile is too crowded to be staged takes the
+// global-memory path everywhere, and none of the memory, which would leave one
+// CTA per SM.
 int md_stage_cap(const b200_ctx *c) {
+  if (!c->nrep && !mean_tile_fits(c, c->tile_cells)) return 0;
   const double per_cell = c->ncells > 0 ? (double)c->n / c->ncells : 0.0;
   int cap = tile_units_of(per_cell, c->tile_cells, c->ntypes == 1);
   if (!c->nrep && c->stage_need > cap) cap = c->stage_need;
@@ -1094,7 +1114,7 @@ bool md_stage_feedback(b200_ctx *c, int staged_max) {
     return cap2 > 0 ? cap2 : md_stage_cap(c);
   };
   const int cap = cap_now();
-  if (staged_max <= cap || cap >= kStageUnitsMax) return false;
+  if (cap == 0 || staged_max <= cap || cap >= kStageUnitsMax) return false;
   c->stage_need = staged_max + staged_max / 10;
   return cap_now() != cap;
 }
