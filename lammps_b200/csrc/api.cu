@@ -525,13 +525,13 @@ int pair_compute_dev(b200_ctx *c, bool ev, bool atom, double *eatom, double *vat
 // rebuild with overflow recovery (host-synchronous; setup and b200_neigh_build)
 int rebuild_sync(b200_ctx *c) {
   for (int attempt = 0; attempt < 3; attempt++) {
-    CK(cudaMemsetAsync(c->status + ST_MAXNEIGH, 0, sizeof(int), c->stream));
-    CK(cudaMemsetAsync(c->status + ST_OVERFLOW, 0, sizeof(int), c->stream));
+    static_assert(ST_OVERFLOW == ST_MAXNEIGH + 1 && ST_MAXSTAGE == ST_MAXNEIGH + 2, "one clear");
+    CK(cudaMemsetAsync(c->status + ST_MAXNEIGH, 0, 3 * sizeof(int), c->stream));
     CK(md_rebuild(c, nullptr));
     int rc = read_status(c);
     if (rc) return rc;
     if (c->status_host[ST_LOST] || c->status_host[ST_BARRIER]) return status_errors(c);
-    if (md_stage_feedback(c, c->status_host[ST_MAXSTAGE])) invalidate_graphs(c);
+    if (md_stage_feedback(c, c->status_host[ST_MAXSTAGE], true)) invalidate_graphs(c);
     if (!c->status_host[ST_OVERFLOW]) return B200_OK;
     if (c->one_user > 0) return status_errors(c);
     int need = c->status_host[ST_MAXNEIGH];
@@ -2011,7 +2011,7 @@ int b200_run(b200_ctx *c, int nsteps, double dt, double ftm2v, int thermo_every,
     rc = read_status(c);
     if (rc) return rc;
     if (c->status_host[ST_LOST] || c->status_host[ST_BARRIER]) return status_errors(c);
-    if (md_stage_feedback(c, c->status_host[ST_MAXSTAGE])) {
+    if (md_stage_feedback(c, c->status_host[ST_MAXSTAGE], false)) {
       // a builder tile staged more atoms than its shared memory held (it
       // took the slower global-memory path): larger staging from now on
       invalidate_graphs(c);

@@ -27,19 +27,20 @@
 
 // status words in device memory (read by the host after a step or a run)
 enum {
+  // the first three are cleared together before a build (rebuild_sync)
   ST_MAXNEIGH = 0,   // largest per-atom full-list count seen at the last build
-  ST_LOST = 1,       // a coordinate was non-finite or beyond one box image
-  ST_MOVED = 2,      // some atom moved more than half the skin (check yes)
+  ST_OVERFLOW = 1,   // a build exceeded the list capacity (sticky)
+  ST_MAXSTAGE = 2,   // most shared memory (16-byte units) one builder tile needed
+  ST_MOVED = 12,     // some atom moved more than half the skin (check yes)
   ST_REBUILD = 3,    // decision of the current step
   ST_AGO = 4,        // steps since the last build (Neighbor::ago)
   ST_NCALLS = 5,     // builds since setup (Neighbor::ncalls)
   ST_NDANGER = 6,    // dangerous builds (Neighbor::ndanger)
-  ST_OVERFLOW = 7,   // a build exceeded the list capacity (sticky)
+  ST_LOST = 7,       // a coordinate was non-finite or beyond one box image
   ST_ROW = 8,        // thermo rows written by the device in this run
   ST_STEP_LO = 9,    // current timestep (low/high 32 bits)
   ST_STEP_HI = 10,
   ST_FORCE_BUILD = 11,  // rebuild on the next step regardless of the schedule
-  ST_MAXSTAGE = 12,     // most shared memory (16-byte units) one builder tile needed
   ST_HALO_BAD = 13,     // a halo pack/unpack index was outside [0, n)
   ST_BADTYPE = 14,      // 1 + index of an uploaded atom with a type outside [1, ntypes]
   ST_BARRIER = 15,      // a grid barrier of a multi-step launch gave up

@@ -263,7 +263,7 @@ inline bool md_q_iso(const b200_ctx *c) {
 cudaError_t md_rebuild(b200_ctx *c, const int *d_flag);
 int md_tile_cells(const b200_ctx *c);
 int md_stage_cap(const b200_ctx *c);
-bool md_stage_feedback(b200_ctx *c, int staged_max);
+bool md_stage_feedback(b200_ctx *c, int staged_max, bool lower);
 // LAMMPS half list derived from the full list; returns entry count via *total
 cudaError_t md_half_list(b200_ctx *c, int *d_num, int *d_jowner, int *d_jimage, long long cap,
                          long long *total);

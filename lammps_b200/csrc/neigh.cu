@@ -513,8 +513,10 @@ __device__ __forceinline__ unsigned candidate_order(unsigned x) {
 // (4 B) and, with several types, types (1 B) with 32 spare slots, and the
 // acceptance words (4 B) with their first slots (2 B)
 __host__ __device__ inline int tile_units(int nstage, int chunks, int cols, bool single) {
-  const int m = nstage + 32, c = chunks * cols;
-  return m + (m + 3) / 4 + (single ? 0 : (m + 15) / 16) + (c + 3) / 4 + (c + 7) / 8;
+  const long long m = (long long)nstage + 32, c = (long long)chunks * cols;
+  const long long u =
+      m + (m + 3) / 4 + (single ? 0 : (m + 15) / 16) + (c + 3) / 4 + (c + 7) / 8;
+  return u < (1 << 30) ? (int)u : 1 << 30;  // (a collapsed cell: 1e5 atoms)
 }
 // the units of a tile of tc cells at a mean of `per_cell` atoms per cell
 inline int tile_units_of(double per_cell, int tc, bool single) {
@@ -631,7 +633,6 @@ __global__ void __launch_bounds__(kNeighThreads, 8) k_neigh_tiles(NeighArgs A) {
   // fit); pass 1: the tiles that fit `units`; pass 2: only the tiles that
   // pass 1 left (more than units1), with more shared memory
   if ((A.pass == 1 && need > A.units) || (A.pass == 2 && need <= A.units1)) return;
-  if (tid == 0) atomicMax(&A.status[ST_MAXSTAGE], need);
   // rb: extent of the owned atoms from the tile centre; a candidate near the
   // cutoff of one lies within ra
   const float fscale = (float)A.scale;
@@ -642,8 +643,11 @@ __global__ void __launch_bounds__(kNeighThreads, 8) k_neigh_tiles(NeighArgs A) {
                     (SINGLE ? 0.f : A.dmax * (1.0f / 2048.0f));
   // cells far wider than the cutoff would overflow FP16 or put every pair
   // inside the band
-  const bool staged = need <= A.units && maxw <= max_chunks(TC) && nstage < 65504 &&
-                      cols <= kMaxCols && ra < 32.f;
+  const bool stageable = need <= kStageUnitsMax && maxw <= max_chunks(TC) && nstage < 65504 &&
+                         cols <= kMaxCols && ra < 32.f;
+  const bool staged = stageable && need <= A.units;
+  // for the next build's capacity: a tile that none can stage does not count
+  if (tid == 0 && stageable) atomicMax(&A.status[ST_MAXSTAGE], need);
   const int a0 = s_src[own0];
   const int nown = s_start[own0 + ow] - s_start[own0];
 
@@ -1106,15 +1110,19 @@ int md_stage_cap2(const b200_ctx *c) {
 }
 
 // After a build: raise the capacity when some tile needed more than the
-// current one holds.  Returns true when the capacity changed (the caller
-// re-captures its graphs).
-bool md_stage_feedback(b200_ctx *c, int staged_max) {
+// current one holds and, with `lower` (staged_max is of a single build of the
+// current atoms), bring it down when no tile needs that much any more: it
+// would cost every later system resident blocks.  Returns true when the
+// capacity changed (the caller re-captures its graphs).
+bool md_stage_feedback(b200_ctx *c, int staged_max, bool lower) {
   auto cap_now = [&] {
     const int cap2 = md_stage_cap2(c);
     return cap2 > 0 ? cap2 : md_stage_cap(c);
   };
   const int cap = cap_now();
-  if (cap == 0 || staged_max <= cap || cap >= kStageUnitsMax) return false;
+  if (cap == 0) return false;
+  const bool raise = staged_max > cap && cap < kStageUnitsMax;
+  if (!raise && !(lower && staged_max + staged_max / 4 < c->stage_need)) return false;
   c->stage_need = staged_max + staged_max / 10;
   return cap_now() != cap;
 }

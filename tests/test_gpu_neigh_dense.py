@@ -12,14 +12,14 @@ from lammps_b200 import PairLJCut, System
 pytestmark = pytest.mark.gpu
 
 
-def box(per_cell, cells, ntypes, clump=0):
+def box(per_cell, cells, ntypes, clump=0, s=None):
     """cells^3 cells of the list cutoff 1, per_cell atoms each on the mean."""
     rng = np.random.default_rng(per_cell + cells)
     edge = np.full(3, cells * 1.0001)
     x = rng.random((per_cell * cells**3, 3)) * edge
     if clump:  # one cell with many more
         x[:clump] = 3.0 + 0.9 * rng.random((clump, 3))
-    s = System("lj", "fp64")
+    s = s or System("lj", "fp64")
     s.set_box(np.zeros(3), edge)
     p = PairLJCut(0.9, ntypes)
     for t in range(1, ntypes + 1):
@@ -59,17 +59,37 @@ def test_list(per_cell, cells, ntypes, clump):
     assert np.array_equal(np.sort(got), np.sort(np.concatenate(want)))
 
 
+def seconds(s, builds=10):
+    best = 1e9
+    for _ in range(builds):
+        t = time.perf_counter()
+        s.neigh_build()
+        best = min(best, time.perf_counter() - t)
+    return best
+
+
 def test_cost_grows_with_the_pairs():
     """A build is bound by its pairs: with four times as many per atom it takes
     about four times as long per atom, and ten times is a path of its own."""
     per_atom = []
     for per_cell in (30, 120):
         s, x, _ = box(per_cell, 12, 1)
-        best = 1e9
-        for _ in range(8):
-            t = time.perf_counter()
-            s.neigh_build()
-            best = min(best, time.perf_counter() - t)
-        per_atom.append(best / len(x))
+        per_atom.append(seconds(s) / len(x))
         s.close()
     assert per_atom[1] < 10 * per_atom[0], per_atom
+
+
+@pytest.mark.parametrize("clump", [200, 600])  # one tile that needs much memory; one past all
+def test_a_clump_costs_no_later_box(clump):
+    """The builder's memory per tile follows the current atoms: a box built
+    after one with a clump takes the time it takes in a context of its own."""
+    s, _, _ = box(20, 20, 1)
+    alone = seconds(s)
+    box(20, 20, 1, clump, s)
+    s.neigh_build()
+    s.neigh_build()
+    box(20, 20, 1, 0, s)
+    s.neigh_build()
+    after = seconds(s)
+    s.close()
+    assert after < 1.2 * alone, (alone, after)
