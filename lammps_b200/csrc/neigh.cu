@@ -546,7 +546,7 @@ __global__ void __launch_bounds__(kNeighThreads, 8) k_neigh_tiles(NeighArgs A) {
   __shared__ int s_nchunk[TC];
   __shared__ unsigned short s_count[kMaxCols];  // neighbors of each owned atom
   __shared__ double cns[SINGLE ? 1 : (MD_MAXTYPES + 1) * (MD_MAXTYPES + 1)];
-  __shared__ __half s_delta[SINGLE ? 1 : MD_MAXTYPES * MD_MAXTYPES];
+  __shared__ __align__(4) __half s_delta[SINGLE ? 1 : MD_MAXTYPES * MD_MAXTYPES];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ncx = box.ncell[0], ncy = box.ncell[1], ncz = box.ncell[2];
   const int tiles_x = (ncx + TC - 1) / TC;
