@@ -1150,21 +1150,25 @@ static cudaError_t launch_tiles(b200_ctx *c, const NeighArgs &A, int tiles, cuda
     const int most = kStageUnitsMax * 16;
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaFuncSetAttribute(k_neigh_tiles<TC, true, false>, attr, most);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_neigh_tiles<TC, true, true>, attr, most);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_neigh_tiles<TC, false, false>, attr, most);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_neigh_tiles<TC, false, true>, attr, most);
+    if constexpr (TC == 1) {
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_neigh_tiles<1, true, true>, attr, most);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_neigh_tiles<1, false, true>, attr, most);
+    }
     if (e != cudaSuccess) return e;
     opt_in.fetch_or(dev_bit);
   }
   const size_t smem = (size_t)A.units * 16;
-  if (c->ntypes == 1 && !c->nrep)
-    k_neigh_tiles<TC, true, false><<<tiles, kNeighThreads, smem, st>>>(A);
-  else if (c->ntypes == 1)
-    k_neigh_tiles<TC, true, true><<<tiles, kNeighThreads, smem, st>>>(A);
-  else if (!c->nrep)
-    k_neigh_tiles<TC, false, false><<<tiles, kNeighThreads, smem, st>>>(A);
-  else
-    k_neigh_tiles<TC, false, true><<<tiles, kNeighThreads, smem, st>>>(A);
+  if constexpr (TC == 1) {  // a batch's tiles own one cell (md_tile_cells)
+    if (c->nrep) {
+      if (c->ntypes == 1) k_neigh_tiles<1, true, true><<<tiles, kNeighThreads, smem, st>>>(A);
+      else k_neigh_tiles<1, false, true><<<tiles, kNeighThreads, smem, st>>>(A);
+      c->launches++;
+      return cudaGetLastError();
+    }
+  }
+  if (c->ntypes == 1) k_neigh_tiles<TC, true, false><<<tiles, kNeighThreads, smem, st>>>(A);
+  else k_neigh_tiles<TC, false, false><<<tiles, kNeighThreads, smem, st>>>(A);
   c->launches++;
   return cudaGetLastError();
 }
