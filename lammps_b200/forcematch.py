@@ -22,6 +22,7 @@ reference form.
 from __future__ import annotations
 
 import ctypes as C
+from functools import lru_cache
 
 import numpy as np
 
@@ -48,7 +49,13 @@ def lj_tables(eps, sigma, cut_factor: float = 2.5):
     return lj1.reshape(-1), lj2.reshape(-1), cutsq
 
 
-_pair_index = {}  # ntypes -> entry of [0, values...] at each matrix element (numpy)
+@lru_cache(maxsize=16)
+def _pair_index(ntypes: int):
+    """Entry of [0, values...] at each element of the matrix (flattened)."""
+    m = np.zeros((ntypes + 1, ntypes + 1), np.int64)
+    r, c = np.triu_indices(ntypes)
+    m[r + 1, c + 1] = m[c + 1, r + 1] = 1 + np.arange(len(r))
+    return m.ravel()
 
 
 def pair_matrix(values, ntypes: int):
@@ -57,16 +64,12 @@ def pair_matrix(values, ntypes: int):
     import torch
 
     k = ntypes * (ntypes + 1) // 2
-    if values.numel() != k:
+    if ntypes < 1 or values.numel() != k:
         raise ValueError(f"expected {k} pair values for {ntypes} types, got {values.numel()}")
-    index = _pair_index.get(ntypes)
-    if index is None:
-        m = np.zeros((ntypes + 1, ntypes + 1), np.int64)
-        r, c = np.triu_indices(ntypes)
-        m[r + 1, c + 1] = m[c + 1, r + 1] = 1 + np.arange(k)
-        index = _pair_index[ntypes] = m.ravel()
+    if values.dim() > 1:
+        raise ValueError(f"pair values of shape {tuple(values.shape)}, not a vector")
     flat = torch.cat([values.new_zeros(1), values.reshape(-1)])
-    index = torch.from_numpy(index).to(values.device)
+    index = torch.from_numpy(_pair_index(ntypes)).to(values.device)
     return flat.index_select(0, index).reshape(ntypes + 1, ntypes + 1)
 
 
