@@ -403,41 +403,49 @@ cudaError_t md_adj_backward(b200_ctx *c, const double *lj1, const double *lj2,
 
 // caller-order device positions -> the context's sorted FP64 positions
 // (types kept, image flags restarted); the next build wraps and re-sorts.
-// `held` keeps them as they came (EamArgs::xf's memory: an lj/cut context has no
-// other use for it).
+// hxy (if given) and hz keep them as they came (b200_ctx::adj_held).
 __global__ void k_adj_positions(int n, const int *__restrict__ orig, const double *__restrict__ x,
                                 double4 *__restrict__ x4, int *__restrict__ image,
-                                double *__restrict__ held) {
+                                double2 *__restrict__ hxy, double *__restrict__ hz) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int o = orig[i];
   const double4 p = x4[i];
-  x4[i] = make_double4(x[3 * o], x[3 * o + 1], x[3 * o + 2], p.w);
-  held[3 * o] = x[3 * o];
-  held[3 * o + 1] = x[3 * o + 1];
-  held[3 * o + 2] = x[3 * o + 2];
+  const double xo = x[3 * o], yo = x[3 * o + 1], zo = x[3 * o + 2];
+  x4[i] = make_double4(xo, yo, zo, p.w);
+  if (hxy) {
+    hxy[o] = make_double2(xo, yo);
+    hz[o] = zo;
+  }
   image[i] = md_img_pack(0, 0, 0);
 }
 
 cudaError_t md_adj_positions(b200_ctx *c, const double *x) {
   k_adj_positions<<<md_blocks(c->n, 256), 256, 0, c->stream>>>(
-      c->n, c->orig, x, c->x4, c->image, reinterpret_cast<double *>(c->xf));
+      c->n, c->orig, x, c->x4, c->image,
+      c->pstyle == B200_PAIR_LJ_CUT ? reinterpret_cast<double2 *>(c->xqb) : nullptr, c->rho);
   c->launches++;
   return cudaGetLastError();
 }
 
-// *diff = 1 when any of m words differs
-__global__ void k_adj_compare(int m, const unsigned long long *__restrict__ a,
-                              const unsigned long long *__restrict__ b, int *diff) {
+// *diff = 1 when a bit of the n positions differs
+__global__ void k_adj_compare(int n, const unsigned long long *__restrict__ x,
+                              const ulonglong2 *__restrict__ hxy,
+                              const unsigned long long *__restrict__ hz, int *diff) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool ne = i < m && a[i] != b[i];
+  bool ne = false;
+  if (i < n) {
+    const ulonglong2 h = hxy[i];
+    ne = x[3 * i] != h.x || x[3 * i + 1] != h.y || x[3 * i + 2] != hz[i];
+  }
   if (__any_sync(0xffffffffu, ne) && (threadIdx.x & 31) == 0) atomicExch(diff, 1);
 }
 
 cudaError_t md_adj_compare(b200_ctx *c, const double *x, int *diff) {
-  k_adj_compare<<<md_blocks(3 * c->n, 256), 256, 0, c->stream>>>(
-      3 * c->n, reinterpret_cast<const unsigned long long *>(x),
-      reinterpret_cast<const unsigned long long *>(c->xf), diff);
+  k_adj_compare<<<md_blocks(c->n, 256), 256, 0, c->stream>>>(
+      c->n, reinterpret_cast<const unsigned long long *>(x),
+      reinterpret_cast<const ulonglong2 *>(c->xqb),
+      reinterpret_cast<const unsigned long long *>(c->rho), diff);
   c->launches++;
   return cudaGetLastError();
 }

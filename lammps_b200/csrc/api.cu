@@ -419,6 +419,19 @@ int upload_tables(b200_ctx *c) {
   return B200_OK;
 }
 
+// The position and F' records of one-element eam: 32 bytes per atom that no
+// other style reads (128 MB at 4,000,000 atoms).  Called wherever the style or
+// the atoms change.
+int alloc_xf(b200_ctx *c) {
+  if (c->pstyle != B200_PAIR_EAM || c->ntypes != 1 || c->xf_n >= c->stride) return B200_OK;
+  CK(cudaSetDevice(c->device));
+  invalidate_graphs(c);  // a kernel argument
+  c->xf_n = 0;
+  CK(dalloc(&c->xf, c->stride));
+  c->xf_n = c->stride;
+  return B200_OK;
+}
+
 int alloc_cells(b200_ctx *c) {
   if (c->ncells + 1 > c->ncell_alloc) {
     invalidate_graphs(c);
@@ -1187,8 +1200,8 @@ const char *b200_last_error(const b200_ctx *c) { return c ? c->err.c_str() : "nu
 long long b200_bytes(const b200_ctx *c) {
   if (!c) return 0;
   long long s = (long long)c->stride;
-  long long b = s * (3 * 32 + 2 * 24 + 24 + 5 * 4 + 16 + 32 + 16 + 4) + c->nlist_alloc * 4 +
-                (long long)c->ncell_alloc * 8;
+  long long b = s * (2 * 32 + 2 * 24 + 24 + 5 * 4 + 16 + 32 + 16 + 4) + c->nlist_alloc * 4 +
+                (long long)c->ncell_alloc * 8 + c->xf_n * 32LL;
   return b;
 }
 
@@ -1344,7 +1357,7 @@ int b200_set_eam(b200_ctx *c, int ntypes, int nrho, double drho, int nr, double 
   c->ntypes = ntypes;
   c->pstyle = B200_PAIR_EAM;
   invalidate_graphs(c);
-  return B200_OK;
+  return alloc_xf(c);
 }
 
 int b200_upload_atoms(b200_ctx *c, int n, const double *x, const double *v, const int *type,
@@ -1388,7 +1401,6 @@ int b200_upload_atoms(b200_ctx *c, int n, const double *x, const double *v, cons
     CK(dalloc(&c->rho, stride));
     CK(dalloc(&c->fp, stride));
     CK(dalloc(&c->fpf, stride));
-    CK(dalloc(&c->xf, stride));
     CK(dalloc(&c->slot, stride));
     CK(dalloc(&c->perm, stride));
     CK(dalloc(&c->cell_tmp, stride));
@@ -1402,6 +1414,7 @@ int b200_upload_atoms(b200_ctx *c, int n, const double *x, const double *v, cons
     c->nlist_alloc = 0;
     dfree(c->nlist);
   }
+  if (int rc = alloc_xf(c)) return rc;
   c->n = n;
   CK(cudaMemsetAsync(c->f, 0, 3 * (size_t)c->stride * sizeof(double), c->stream));
   // host sources are copied into the staging buffer; device sources are read
@@ -2271,7 +2284,7 @@ int b200_adj_set_positions(b200_ctx *c, const double *x) {
   rc = rebuild_sync(c);
   if (rc) return rc;
   c->sorted_once = true;
-  c->adj_held = true;
+  c->adj_held = c->pstyle == B200_PAIR_LJ_CUT;
   return B200_OK;
 }
 

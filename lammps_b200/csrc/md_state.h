@@ -137,9 +137,10 @@ struct b200_ctx {
   int out_next = 0;
   double *rho = nullptr, *fp = nullptr;
   float *fpf = nullptr;
-  // eam, one element: position and F' records (EamArgs::xf); force matching:
-  // the positions given (adj_held)
+  // eam, one element: position and F' records (EamArgs::xf); no other pair
+  // style has them (alloc_xf)
   double4 *xf = nullptr;
+  int xf_n = 0;
   // split EAM compute (b200_eam_density, then b200_eam_force): the eflag /
   // vflag of the density call and its per-atom embedding energies
   int eam_split_eflag = -1, eam_split_vflag = -1;
@@ -176,8 +177,9 @@ struct b200_ctx {
   double *adj_gs = nullptr;    // force-matching scratch: G in the sorted order
   double *adj_gtab = nullptr;  // force-matching parameter gradients
   int adj_n = 0;
-  // xf holds the positions b200_adj_set_positions was given, and nothing has
-  // changed atoms, lists or settings since
+  // the positions b200_adj_set_positions was given are held (x and y of each
+  // atom in xqb, z in rho: an lj/cut context between runs has no other use for
+  // these), and nothing has changed atoms, lists or settings since
   bool adj_held = false;
   double *ev = nullptr;          // [0] eng, [1..6] virial, [7] sum m v^2
   int *status = nullptr;         // ST_* words
