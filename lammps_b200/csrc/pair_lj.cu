@@ -176,14 +176,15 @@ struct Fp64Pairs {
 };
 
 // One atom's pair forces in FP64 (this thread's lane of the TPA threads of
-// atom i): adds to fx, fy, fz (and to acc with EV).
-template <int TPA, bool EV, bool SINGLE, bool BATCH>
-__device__ __forceinline__ void lj_atom_fp64(const PairArgs &a, const double4 *__restrict__ x4,
+// atom i): adds to fx, fy, fz (and to acc with EV).  COH: the kernel writes x4
+// later, so no load of it may be a read-only one.
+template <int TPA, bool EV, bool SINGLE, bool BATCH, bool COH = false>
+__device__ __forceinline__ void lj_atom_fp64(const PairArgs &a, const double4 *x4,
                                              const double *tab, int nt2, int i, int lane,
                                              bool active, double &fx, double &fy, double &fz,
                                              double (&acc)[7]) {
   if (!active) return;
-  const double4 xi = x4[i];
+  const double4 xi = ld_pos<COH>(&x4[i]);
   const BoxGeom &box = BATCH ? a.reps.box[a.reps.rep_of_atom[i]] : a.box;
   const Fp64Pairs<EV, SINGLE> pairs(a, box, a.cell[i], tab, nt2);
   auto slabs = [&](auto wrap_tag) {
@@ -193,7 +194,7 @@ __device__ __forceinline__ void lj_atom_fp64(const PairArgs &a, const double4 *_
     walk_list<TPA>(a.nlist, a.stride, i, a.numneigh[i], lane, [&](const unsigned (&ee)[4], int m) {
       double4 xj[4];
 #pragma unroll
-      for (int u = 0; u < 4; u++) xj[u] = ld_pos<false>(&x4[u < m ? md_entry_j(ee[u]) : i]);
+      for (int u = 0; u < 4; u++) xj[u] = ld_pos<COH>(&x4[u < m ? md_entry_j(ee[u]) : i]);
       pairs.template four<WRAP, false>(pairs, xi, ee, xj, m, fx, fy, fz, acc);
     });
   };
@@ -320,15 +321,16 @@ struct MixedPairs {
   }
 };
 
-template <int TPA, bool EV, bool SINGLE, bool BATCH, bool ISO>
-__device__ __forceinline__ void lj_atom_mixed(const PairArgs &a, const int4 *__restrict__ xq,
+// COH as in lj_atom_fp64.
+template <int TPA, bool EV, bool SINGLE, bool BATCH, bool ISO, bool COH = false>
+__device__ __forceinline__ void lj_atom_mixed(const PairArgs &a, const int4 *xq,
                                               const float *tabf, int nt2, int i, int lane,
                                               bool active, double &fx, double &fy, double &fz,
                                               double (&acc)[7]) {
   if (!active) return;
   const BoxGeom &box = BATCH ? a.reps.box[a.reps.rep_of_atom[i]] : a.box;
   const MixedPairs<EV, SINGLE, ISO> pairs(a, box, tabf, nt2);
-  const int4 xi = xq[i];
+  const int4 xi = ld_pos<COH>(&xq[i]);
   const int nslab = (a.numneigh[i] + 3) >> 2;
   const int pe = md_pad_entry(i);
   if constexpr (TPA == 1) {
@@ -353,7 +355,7 @@ __device__ __forceinline__ void lj_atom_mixed(const PairArgs &a, const int4 *__r
                                      (unsigned)a3.x, (unsigned)a3.y, (unsigned)a3.z, (unsigned)a3.w};
       int4 xall[16];
 #pragma unroll
-      for (int u = 0; u < 16; u++) xall[u] = __ldg(&xq[md_entry_j(eall[u])]);
+      for (int u = 0; u < 16; u++) xall[u] = ld_pos<COH>(&xq[md_entry_j(eall[u])]);
       pairs.template group<8>(xi, xall, fx, fy, fz, acc);
       pairs.template group<8>(xi, xall + 8, fx, fy, fz, acc);
       a0 = b0;
@@ -372,7 +374,7 @@ __device__ __forceinline__ void lj_atom_mixed(const PairArgs &a, const int4 *__r
       w.prefetch();
       int4 xall[G];
 #pragma unroll
-      for (int u = 0; u < G; u++) xall[u] = __ldg(&xq[md_entry_j(w.cur[u])]);
+      for (int u = 0; u < G; u++) xall[u] = ld_pos<COH>(&xq[md_entry_j(w.cur[u])]);
       pairs.template group<G>(xi, xall, fx, fy, fz, acc);
       w.advance();
     }
@@ -635,8 +637,7 @@ __device__ __forceinline__ int rep_atom(const int2 *__restrict__ ranges, int r0,
 }
 
 template <int TPA, bool MIXED, bool SINGLE, bool ISO>
-__global__ void __launch_bounds__(512) k_rep_step(PairArgs a, const double4 *__restrict__ x4,
-                                                   const int4 *__restrict__ xq, RepStepArgs s) {
+__global__ void __launch_bounds__(512) k_rep_step(PairArgs a, double4 *x4, int4 *xq, RepStepArgs s) {
   namespace cg = cooperative_groups;
   __shared__ double tab[6 * TABSZ];
   __shared__ bool last;
@@ -668,10 +669,11 @@ __global__ void __launch_bounds__(512) k_rep_step(PairArgs a, const double4 *__r
     double fx = 0.0, fy = 0.0, fz = 0.0;
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
     if (MIXED)
-      lj_atom_mixed<TPA, false, SINGLE, true, ISO>(a, xq, tabf, nt2, i, lane, active, fx, fy, fz,
-                                                   acc);
+      lj_atom_mixed<TPA, false, SINGLE, true, ISO, true>(a, xq, tabf, nt2, i, lane, active, fx, fy,
+                                                         fz, acc);
     else
-      lj_atom_fp64<TPA, false, SINGLE, true>(a, x4, tab, nt2, i, lane, active, fx, fy, fz, acc);
+      lj_atom_fp64<TPA, false, SINGLE, true, true>(a, x4, tab, nt2, i, lane, active, fx, fy, fz,
+                                                   acc);
     lj_atom_store<TPA, false, false>(a, i, lane, active, fx, fy, fz, acc);
   }
   // 2. every CTA of the cluster has read the group's positions
@@ -681,8 +683,8 @@ __global__ void __launch_bounds__(512) k_rep_step(PairArgs a, const double4 *__r
   for (int k = k0 + (int)threadIdx.x; k < k1; k += blockDim.x) {
     const int i = rep_atom(s.ranges, r0, r1, k);
     double ke = 0.0;
-    moved |= md_nve_fused_atom<false>(i, a.stride, s.dtv, s.dtf, s.mass, const_cast<double4 *>(x4),
-                                      s.v, a.f, MIXED ? const_cast<int4 *>(xq) : nullptr,
+    moved |= md_nve_fused_atom<false>(i, a.stride, s.dtv, s.dtf, s.mass, x4,
+                                      s.v, a.f, MIXED ? xq : nullptr,
                                       a.reps.box[a.reps.rep_of_atom[i]], s.xhold, s.triggersq, ke);
   }
   if (s.xhold && __any_sync(0xffffffffu, moved) && (threadIdx.x & 31) == 0) {
@@ -718,10 +720,8 @@ cudaError_t launch_rep_t(b200_ctx *c, const PairArgs &a, const RepStepArgs &s) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (c->ntypes == 1)
-    return cudaLaunchKernelEx(&cfg, k_rep_step<TPA, MIXED, true, ISO>, a, (const double4 *)c->x4,
-                              (const int4 *)c->xq, s);
-  return cudaLaunchKernelEx(&cfg, k_rep_step<TPA, MIXED, false, ISO>, a, (const double4 *)c->x4,
-                            (const int4 *)c->xq, s);
+    return cudaLaunchKernelEx(&cfg, k_rep_step<TPA, MIXED, true, ISO>, a, c->x4, c->xq, s);
+  return cudaLaunchKernelEx(&cfg, k_rep_step<TPA, MIXED, false, ISO>, a, c->x4, c->xq, s);
 }
 
 template <int TPA, bool EV, bool ATOM, bool SINGLE, bool BATCH>
