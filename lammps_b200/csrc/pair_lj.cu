@@ -128,20 +128,20 @@ struct Fp64Pairs {
       delz = __dsub_rn(xi.z, xj.z);
     }
   }
-  // the first m of four entries ee with their positions xj; `of` forms the
+  // the first m of N entries ee with their positions xj; `of` forms the
   // separations (this, or MultiShift).  FINITE: every xj is finite, or the
   // caller looks at the sums and calls again without it.
-  template <bool WRAP, bool FINITE, class S>
-  __device__ __forceinline__ void four(const S &of, const double4 &xi, const unsigned (&ee)[4],
-                                       const double4 (&xj)[4], int m, double &fx, double &fy,
+  template <bool WRAP, bool FINITE, int N, class S>
+  __device__ __forceinline__ void some(const S &of, const double4 &xi, const unsigned (&ee)[N],
+                                       const double4 (&xj)[N], int m, double &fx, double &fy,
                                        double &fz, double (&acc)[7]) const {
     const int ti = (int)xi.w;
     // Branch-free: an FP64 pair term is a chain of about twenty dependent
-    // operations, and only without branches do the four entries' chains
+    // operations, and only without branches do the entries' chains
     // overlap.  An entry past m or past the cutoff gets a zero separation
     // (drop_unless) or, with FINITE, a zero factor.
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
+    for (int u = 0; u < N; u++) {
       double delx, dely, delz;
       of.template sep<WRAP>(ee[u], xi, xj[u], delx, dely, delz);
       const double rsq = dsq3(delx, dely, delz);
@@ -195,7 +195,7 @@ __device__ __forceinline__ void lj_atom_fp64(const PairArgs &a, const double4 *x
       double4 xj[4];
 #pragma unroll
       for (int u = 0; u < 4; u++) xj[u] = ld_pos<COH>(&x4[u < m ? md_entry_j(ee[u]) : i]);
-      pairs.template four<WRAP, false>(pairs, xi, ee, xj, m, fx, fy, fz, acc);
+      pairs.template some<WRAP, false>(pairs, xi, ee, xj, m, fx, fy, fz, acc);
     });
   };
   // one path per warp: lanes on either path would run one after the other
@@ -538,8 +538,8 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
       }
     } else {
       const double4 *x4 = static_cast<const double4 *>(s.cur);
-      auto walk = [&](auto wrap_tag, auto finite_tag) {
-        constexpr bool WRAP = decltype(wrap_tag)::value, FINITE = decltype(finite_tag)::value;
+      auto walk = [&](auto wrap_tag) {
+        constexpr bool WRAP = decltype(wrap_tag)::value;
         for (int k = 0; k < cnt; k += G * DEPTH) {
           unsigned ee[DEPTH][G];
           double4 xs[DEPTH][G];
@@ -553,18 +553,23 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
             }
 #pragma unroll
           for (int d = 0; d < DEPTH; d++)
-            dp.template four<WRAP, FINITE>(shift, xi, ee[d], xs[d], min(G, cnt - k - d * G), fx, fy,
+            dp.template some<WRAP, true>(shift, xi, ee[d], xs[d], min(G, cnt - k - d * G), fx, fy,
                                            fz, acc);
         }
       };
-      if (wrap) walk(std::true_type{}, std::true_type{});
-      else walk(std::false_type{}, std::true_type{});
+      if (wrap) walk(std::true_type{});
+      else walk(std::false_type{});
       // a neighbour that is not finite (or a force that is not): once more,
       // dropping rejected pairs (32,000 atoms: 1,725 us a run with this, 1,720
       // without, 1,803 with drop_unless in the loop)
       if (!isfinite(fx + fy + fz)) {
         fx = fy = fz = 0.0;
-        walk(std::true_type{}, std::false_type{});
+#pragma unroll 1
+        for (int e = 0; e < cnt; e++) {
+          const unsigned ee[1] = {(unsigned)entry(e)};
+          const double4 xs[1] = {ld_pos<true>(&x4[md_entry_j(ee[0])])};
+          dp.template some<true, false>(shift, xi, ee, xs, 1, fx, fy, fz, acc);
+        }
       }
     }
     fx = lane_sum<TPA>(fx);
