@@ -241,8 +241,9 @@ int b200_get_launch(const b200_ctx *ctx, int *threads_per_atom, int *block_size)
      4 fix nve final half-step (+ kinetic energy and thermo row on output steps)
    b200_get_timing returns milliseconds summed over the timed steps.
    on = 2 times whole pieces instead, with the run's own step form kept
-   (lj/cut forces and both half-steps in one launch): two stream events around
-   each piece; phase 0 = initial half-steps at chunk starts, 1 = rebuilds,
+   (forces and both half-steps in one launch, or several steps in one where the
+   box is small): two stream events around each piece, and the steps of one
+   launch share its time equally; phase 0 = initial half-steps at chunk starts, 1 = rebuilds,
    2 = forces with their half-steps; 3 and 4 stay zero. */
 int b200_set_timing(b200_ctx *ctx, int on);
 /* on = 1 (default): b200_run replays captured CUDA graphs of the step's

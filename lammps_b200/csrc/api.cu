@@ -961,11 +961,13 @@ int wait_decision(b200_ctx *c, bool *rebuild, int *ago = nullptr) {
 
 // `nsteps` fused non-output steps in one launch; with the distance criterion
 // it may end early.  *done: steps run; *rebuild: the decision for the step
-// after them.
+// after them.  `ev` (optional): two events around the launch.
 int run_multi(b200_ctx *c, const MultiPlan &plan, int nsteps, int ago, double dtv, double dtf,
-              int *done, bool *rebuild) {
+              int *done, bool *rebuild, cudaEvent_t *ev) {
+  if (ev) CK(cudaEventRecord(ev[0], c->stream));
   int rc = launch_multi(c, plan, nsteps, ago, dtv, dtf, c->every, c->check);
   if (rc) return rc;
+  if (ev) CK(cudaEventRecord(ev[1], c->stream));
   *done = nsteps;
   *rebuild = false;
   if (c->check) {
@@ -1891,12 +1893,15 @@ int b200_run(b200_ctx *c, int nsteps, double dt, double ftm2v, int thermo_every,
     int rc = ensure_events(c, (size_t)(MD_NPHASE + 1) * chunk);
     if (rc) return rc;
   }
-  // timing mode 2: two events around each piece, at most four pieces a step
+  // timing mode 2: two events around each piece, at most four pieces a step,
+  // and the steps of a multi-step launch at its first
   std::vector<signed char> piece_kind;
+  std::vector<int> piece_steps;
   if (c->timing_pieces) {
     int rc = ensure_events(c, (size_t)8 * chunk);
     if (rc) return rc;
     piece_kind.assign((size_t)4 * chunk, -1);
+    piece_steps.assign(chunk, 1);
   }
   {
     int rc = ensure_graphs(c, dtv, dtf, ftm2v);
@@ -1952,9 +1957,9 @@ int b200_run(b200_ctx *c, int nsteps, double dt, double ftm2v, int thermo_every,
     bool pre_done = false;
     // the decision of the coming step, when a multi-step launch has posted it
     bool told = false, told_rebuild = false;
-    const MultiPlan multi = c->timing || c->timing_pieces || !c->use_graphs ? MultiPlan()
-                                                                           : multi_plan(c);
-    if (c->timing_pieces) std::fill(piece_kind.begin(), piece_kind.end(), (signed char)-1);
+    const MultiPlan multi = c->timing || !c->use_graphs ? MultiPlan() : multi_plan(c);
+    std::fill(piece_kind.begin(), piece_kind.end(), (signed char)-1);
+    std::fill(piece_steps.begin(), piece_steps.end(), 1);
     for (long long t = s; t <= s_end; t++) {
       cudaEvent_t *ev = c->timing ? &c->ev_pool[(size_t)(t - s) * (MD_NPHASE + 1)] : nullptr;
       // piece k of step t; timing mode 2 brackets it with two stream events
@@ -2006,8 +2011,14 @@ int b200_run(b200_ctx *c, int nsteps, double dt, double ftm2v, int thermo_every,
           k++;
         if (k > 1) {
           int done = 0;
-          rc = run_multi(c, multi, k, ago, dtv, dtf, &done, &told_rebuild);
+          const size_t slot = (size_t)(t - s) * 4 + 2;
+          rc = run_multi(c, multi, k, ago, dtv, dtf, &done, &told_rebuild,
+                         c->timing_pieces ? &c->ev_pool[2 * slot] : nullptr);
           if (rc) return rc;
+          if (c->timing_pieces) {
+            piece_kind[slot] = PIECE_FUSED;
+            piece_steps[t - s] = done;
+          }
           told = c->check != 0;
           ago += done - 1;
           t += done - 1;
@@ -2060,9 +2071,11 @@ int b200_run(b200_ctx *c, int nsteps, double dt, double ftm2v, int thermo_every,
     if (c->timing_pieces) {
       // mode 2: phase 0 the initial half-step pieces (chunk starts), 1 the
       // rebuilds, 2 the force pieces with their half-steps (the one-launch
-      // step for lj/cut)
+      // step, or a launch of several, whose time its steps share equally)
+      const size_t first = c->step_ms.size();
+      c->step_ms.resize(first + (size_t)(s_end - s + 1), 0.f);
       for (long long t = s; t <= s_end; t++) {
-        float step = 0.f;
+        float *step = c->step_ms.data() + first + (t - s);
         for (int k = 0; k < 4; k++) {
           const size_t slot = (size_t)(t - s) * 4 + k;
           const int kind = piece_kind[slot];
@@ -2070,9 +2083,9 @@ int b200_run(b200_ctx *c, int nsteps, double dt, double ftm2v, int thermo_every,
           float ms = 0.f;
           CK(cudaEventElapsedTime(&ms, c->ev_pool[2 * slot], c->ev_pool[2 * slot + 1]));
           c->phase_ms[kind == PIECE_PRE ? 0 : (kind == PIECE_REBUILD ? 1 : 2)] += ms;
-          step += ms;
+          const int share = k == 2 ? piece_steps[t - s] : 1;
+          for (int q = 0; q < share; q++) step[q] += ms / share;
         }
-        c->step_ms.push_back(step);
       }
       c->phase_steps += s_end - s + 1;
     }

@@ -474,7 +474,8 @@ class System:
 
     def set_timing(self, on=True):
         """True (1): phase events inside every step's pieces; 2: events around
-        whole pieces with the run's own step form kept."""
+        whole pieces with the run's own step form kept (the steps of a launch
+        of several share its time equally)."""
         self._ck(self._L.b200_set_timing(self._h, int(on)))
 
     def timing(self, reset=False):
