@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_sort_all(SortArgs A) {
   // Looked at before the first change of the cell counts: a launch that gives
   // up leaves them as they are, and counting on top of them would place atoms
   // past the arrays.
-  if (__syncthreads_or(gave_up)) return;
+  if (gave_up) return;
   if (act) slot = atomicAdd(&A.cell_count[c], 1);
   if (md_grid_barrier(A.bar, false, true, A.status) < 0) return;
   if (blockIdx.x == 0) {
@@ -587,8 +587,8 @@ __global__ void __launch_bounds__(kNeighThreads, 8) k_neigh_tiles(NeighArgs A) {
     s_img[id][2] = (signed char)iz;
     s_start[id + 1] = cnt;
   }
-  // after a sort that gave up, cell_start may never have been written
-  if (__syncthreads_or(gave_up)) return;
+  if (gave_up) return;  // cell_start may never have been written
+  __syncthreads();
   if (warp == 0) {  // prefix sum of the counts, two per lane
     const int i0 = 2 * lane, i1 = 2 * lane + 1;
     const int c0 = i0 < NST ? s_start[i0 + 1] : 0, c1 = i1 < NST ? s_start[i1 + 1] : 0;
