@@ -600,7 +600,9 @@ int autotune_step(b200_ctx *c) {
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   const int cand[4] = {1, 2, 4, 8};
-  // eight lanes never win on a box that fills the chip many times over
+  // eight lanes never win on a box that fills the chip many times over (202,612
+  // atoms, us a step with the best and with eight: lj mixed 40 and 56, FP64 65
+  // and 92, eam 103 and 133, FP64 214 and 277)
   const int ncand = c->n >= 200000 ? 3 : 4;
   float tmin[4] = {1e30f, 1e30f, 1e30f, 1e30f};
   auto step = [&]() -> cudaError_t {
@@ -667,11 +669,15 @@ int autotune_step(b200_ctx *c) {
       best = tmin[k];
       best_tpa = cand[k];
     }
-  // the repeat changes the shape only where that clearly pays: near-ties
-  // would otherwise go either way from run to run, and with them the
-  // summation order
+  // The repeat keeps the shape of the setup's search unless another is 3 %
+  // faster, the search's own margin for a tie: two searches differ by up to
+  // 1 %, and a tie (2 and 4 lanes at 32,000 FP64 atoms: 11.3 and 11.2 us) would
+  // otherwise go either way from run to run, and with it the summation order.
+  // A margin of 7 % gave up 4 to 7 % where thermal positions favour more lanes
+  // than the lattice: eam, 256,000 atoms, one lane 155.6 us a step, two 144.9;
+  // FP64 305.6 and 289.2.
   for (int k = 0; k < 4; k++)
-    if (tpa_was == cand[k] && best > 0.93f * tmin[k]) best_tpa = tpa_was;
+    if (tpa_was == cand[k] && best > 0.97f * tmin[k]) best_tpa = tpa_was;
   c->tpa = best_tpa;
   c->tuned = true;
   return B200_OK;
