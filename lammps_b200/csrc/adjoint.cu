@@ -324,12 +324,18 @@ AdjTables make_tables(const b200_ctx *c, const double *lj1, const double *lj2,
 
 }  // namespace
 
-// Threads per atom of both passes.  With one, the chip is full from about
-// 32,000 atoms on (54,647 atoms, FP64, forward and backward: 1,072 us with
-// one, 1,088 two, 1,108 four, 1,141 eight); smaller boxes take up to eight
-// (8,000 atoms, mixed: 861 us with eight, 901 with one).
+// Threads per atom of both passes: as many as the chip has room for.  Forward
+// and backward call, two types, us with 1, 2, 4 and 8 (mixed | FP64):
+//    8,000   112  92  78  74 | 125  91  83  76
+//   10,976   112  87  80  70 | 125  96  83  80
+//   13,500   112  86  79  78 | 125  96  82  82
+//   23,328   107  90  81  84 | 126 103  99  98
+//   28,880   108 108 104 103 | 129 108 108 115
+//   42,592   118 101 101 111 | 141 134 132 135
+//   55,296   120 120 116 127 | 140 153 141 152
+// (one type alike; with four, fewer threads win a little earlier)
 static int adj_tpa(int n) {
-  return n >= 32000 ? 1 : n >= 16000 ? 2 : n >= 10000 ? 4 : 8;
+  return n >= 45000 ? 1 : n >= 26000 ? 2 : n >= 12000 ? 4 : 8;
 }
 
 static AdjArgs adj_args(b200_ctx *c, const double *lj1, const double *lj2, const double *cutsq) {
