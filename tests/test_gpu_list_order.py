@@ -39,5 +39,5 @@ def test_order(n, edge, cut):
     assert (np.abs(d) <= 1).all()
     key = (((d[:, 2] + 1) * 3 + d[:, 1] + 1) * 3 + d[:, 0] + 1) * np.int64(n) + j
     same = i[1:] == i[:-1]
-    assert same.sum() > n // 2
+    assert same.sum() > 100  # neighbours compared (few in the dilute box)
     assert (np.diff(key)[same] > 0).all()
