@@ -519,12 +519,10 @@ __device__ __forceinline__ bool md_nve_fused_atom(int i, int stride, double dtv,
 // After kBarrierPolls (a few seconds) it gives up and returns -1, which ends
 // the block; so do the others at this barrier or the next.  The host finds
 // ST_BARRIER set; sorts and list builds that are already queued return at once.
-// A word with kBarrierExpired in it gives up at the first poll; one that gives
-// up puts that into the word `next`, if given.
+// A word with kBarrierExpired in it gives up at the first poll.
 constexpr unsigned kBarrierPolls = 1u << 22;
 constexpr unsigned kBarrierExpired = 0x8000u;  // above any number of blocks
-__device__ __forceinline__ int md_grid_barrier(unsigned *slot, bool flag, bool wait, int *status,
-                                               unsigned *next = nullptr) {
+__device__ __forceinline__ int md_grid_barrier(unsigned *slot, bool flag, bool wait, int *status) {
   __shared__ int s_or;
   const int any = __syncthreads_or(flag ? 1 : 0);
   if (threadIdx.x == 0) {
@@ -539,7 +537,6 @@ __device__ __forceinline__ int md_grid_barrier(unsigned *slot, bool flag, bool w
       r = (v >> 16) != 0u;
       if ((v & 0xffffu) != gridDim.x) {
         atomicExch(&status[ST_BARRIER], 1);
-        if (next) *next = kBarrierExpired;
         r = -1;
       }
     }
@@ -561,14 +558,6 @@ struct MultiArgs {
 };
 // words of one launch: two barriers a step, at most a run chunk's steps
 #define MD_BAR_WORDS 512
-
-// A step's barrier.  One that gives up expires the next launch's first barrier
-// too (block 0 comes here after it has zeroed that word), so that a chunk of
-// queued launches waits for one time-out, not for one each.
-__device__ __forceinline__ int md_multi_barrier(const MultiArgs &m, int word, bool flag, bool wait,
-                                                int *status) {
-  return md_grid_barrier(m.bar + word, flag, wait, status, m.bar_next);
-}
 
 // The schedule after step j of the launch (0-based): Neighbor::decide for the
 // step that follows (src/neighbor.cpp:1294-1309).
@@ -859,7 +848,7 @@ __device__ __forceinline__ int md_multi_next(const StepArgs &s, const MultiArgs 
   bool rebuild = !s.check && cand;
   if (!last || (s.check && cand)) {
     // after the last step only the block that posts the decision waits
-    const int r = md_multi_barrier(m, word, moved, !last || blockIdx.x == 0, s.status);
+    const int r = md_grid_barrier(m.bar + word, moved, !last || blockIdx.x == 0, s.status);
     if (r < 0) return -1;
     if (s.check && cand) rebuild = r != 0;
   }

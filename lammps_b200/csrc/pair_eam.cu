@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(kMultiThreads, DEPTH == 1 ? 4 : 2)
       } else if (MIXED) a.fpf[i] = (float)fpi;
       else a.fp[i] = fpi;
     }
-    if (md_multi_barrier(m, 2 * j, false, true, s.status) < 0) return;
+    if (md_grid_barrier(m.bar + 2 * j, false, true, s.status) < 0) return;
     fpi = from_first<TPA>(fpi);
     // forces
     double fx = 0.0, fy = 0.0, fz = 0.0;
