@@ -92,4 +92,4 @@ def test_a_clump_costs_no_later_box(clump):
     s.neigh_build()
     after = seconds(s)
     s.close()
-    assert after < 1.2 * alone, (alone, after)
+    assert after < 1.5 * alone, (alone, after)  # a third of the resident blocks takes three times
