@@ -426,9 +426,13 @@ int alloc_xf(b200_ctx *c) {
   if (c->pstyle != B200_PAIR_EAM || c->ntypes != 1 || c->xf_n >= c->stride) return B200_OK;
   CK(cudaSetDevice(c->device));
   invalidate_graphs(c);  // a kernel argument
+  const bool had = c->have_atoms, sorted = c->sorted_once;
   c->xf_n = 0;
+  c->have_atoms = c->sorted_once = false;  // no pass runs without them
   CK(dalloc(&c->xf, c->stride));
   c->xf_n = c->stride;
+  c->have_atoms = had;
+  c->sorted_once = sorted;
   return B200_OK;
 }
 
