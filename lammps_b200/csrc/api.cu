@@ -372,6 +372,10 @@ int init_cutoffs_and_cells(b200_ctx *c) {
     return set_err(c, B200_ERR_ARG, "too many cells (%lld)", ncells);
   if ((int)ncells != c->ncells) invalidate_graphs(c);  // scan launch shape changes
   c->ncells = (int)ncells;
+  // another system: whether two-cell tiles can be staged is open again
+  if (c->narrow && (std::abs(c->n - c->narrow_n) > c->narrow_n / 8 ||
+                    std::abs(c->ncells - c->narrow_cells) > c->narrow_cells / 8))
+    c->narrow = false;
   c->tile_cells = md_tile_cells(c);  // set by n and ncells, which both invalidate the graphs
   return B200_OK;
 }
@@ -542,13 +546,16 @@ int pair_compute_dev(b200_ctx *c, bool ev, bool atom, double *eatom, double *vat
 // rebuild with overflow recovery (host-synchronous; setup and b200_neigh_build)
 int rebuild_sync(b200_ctx *c) {
   for (int attempt = 0; attempt < 3; attempt++) {
-    static_assert(ST_OVERFLOW == ST_MAXNEIGH + 1 && ST_MAXSTAGE == ST_MAXNEIGH + 2, "one clear");
-    CK(cudaMemsetAsync(c->status + ST_MAXNEIGH, 0, 3 * sizeof(int), c->stream));
+    static_assert(ST_OVERFLOW == ST_MAXNEIGH + 1 && ST_MAXSTAGE == ST_MAXNEIGH + 2 &&
+                      ST_UNSTAGED == ST_MAXNEIGH + 3,
+                  "one clear");
+    CK(cudaMemsetAsync(c->status + ST_MAXNEIGH, 0, 4 * sizeof(int), c->stream));
     CK(md_rebuild(c, nullptr));
     int rc = read_status(c);
     if (rc) return rc;
     if (c->status_host[ST_LOST] || c->status_host[ST_BARRIER]) return status_errors(c);
-    if (md_stage_feedback(c, c->status_host[ST_MAXSTAGE], true)) invalidate_graphs(c);
+    if (md_stage_feedback(c, c->status_host[ST_MAXSTAGE], c->status_host[ST_UNSTAGED], true))
+      invalidate_graphs(c);
     if (!c->status_host[ST_OVERFLOW]) return B200_OK;
     if (c->one_user > 0) return status_errors(c);
     int need = c->status_host[ST_MAXNEIGH];
@@ -2045,7 +2052,7 @@ int b200_run(b200_ctx *c, int nsteps, double dt, double ftm2v, int thermo_every,
     rc = read_status(c);
     if (rc) return rc;
     if (c->status_host[ST_LOST] || c->status_host[ST_BARRIER]) return status_errors(c);
-    if (md_stage_feedback(c, c->status_host[ST_MAXSTAGE], false)) {
+    if (md_stage_feedback(c, c->status_host[ST_MAXSTAGE], 0, false)) {
       // a builder tile staged more atoms than its shared memory held (it
       // took the slower global-memory path): larger staging from now on
       invalidate_graphs(c);

@@ -27,12 +27,12 @@
 
 // status words in device memory (read by the host after a step or a run)
 enum {
-  // the first three are cleared together before a build (rebuild_sync)
+  // the first four are cleared together before a build (rebuild_sync)
   ST_MAXNEIGH = 0,   // largest per-atom full-list count seen at the last build
   ST_OVERFLOW = 1,   // a build exceeded the list capacity (sticky)
   ST_MAXSTAGE = 2,   // most shared memory (16-byte units) one builder tile needed
+  ST_UNSTAGED = 3,   // atoms of builder tiles that no capacity could stage
   ST_MOVED = 12,     // some atom moved more than half the skin (check yes)
-  ST_REBUILD = 3,    // decision of the current step
   ST_AGO = 4,        // steps since the last build (Neighbor::ago)
   ST_NCALLS = 5,     // builds since setup (Neighbor::ncalls)
   ST_NDANGER = 6,    // dangerous builds (Neighbor::ndanger)
@@ -44,7 +44,8 @@ enum {
   ST_HALO_BAD = 13,     // a halo pack/unpack index was outside [0, n)
   ST_BADTYPE = 14,      // 1 + index of an uploaded atom with a type outside [1, ntypes]
   ST_BARRIER = 15,      // a grid barrier of a multi-step launch gave up
-  ST_COUNT = 16
+  ST_REBUILD = 16,      // decision of the current step
+  ST_COUNT = 17
 };
 
 struct BoxGeom {

@@ -159,6 +159,10 @@ struct b200_ctx {
   int capacity = 0;     // entries per atom
   int stage_need = 0;   // shared memory (16-byte units) per builder tile seen by earlier builds
   int tile_cells = 1;   // cells along x owned by one builder CTA (md_tile_cells)
+  // a build of these atoms and cells had too many atoms in two-cell tiles that
+  // could not be staged (md_stage_feedback)
+  bool narrow = false;
+  int narrow_n = 0, narrow_cells = 0;
   long long nlist_alloc = 0;
 
   // run-chunk snapshot for overflow replay (x4, v, f, xhold planes + ids)
@@ -265,7 +269,7 @@ inline bool md_q_iso(const b200_ctx *c) {
 cudaError_t md_rebuild(b200_ctx *c, const int *d_flag);
 int md_tile_cells(const b200_ctx *c);
 int md_stage_cap(const b200_ctx *c);
-bool md_stage_feedback(b200_ctx *c, int staged_max, bool lower);
+bool md_stage_feedback(b200_ctx *c, int staged_max, int unstaged, bool lower);
 // LAMMPS half list derived from the full list; returns entry count via *total
 cudaError_t md_half_list(b200_ctx *c, int *d_num, int *d_jowner, int *d_jimage, long long cap,
                          long long *total);

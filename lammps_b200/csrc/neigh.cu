@@ -656,8 +656,11 @@ __global__ void __launch_bounds__(kNeighThreads, 8) k_neigh_tiles(NeighArgs A) {
   const bool stageable = need <= kStageUnitsMax && maxw <= max_chunks(TC) && nstage < 65504 &&
                          cols <= kMaxCols && ra < 32.f;
   const bool staged = stageable && need <= A.units;
-  // for the next build's capacity: a tile that none can stage does not count
-  if (tid == 0 && stageable) atomicMax(&A.status[ST_MAXSTAGE], need);
+  // for the next build's capacity, and for the tiles' width
+  if (tid == 0) {
+    if (stageable) atomicMax(&A.status[ST_MAXSTAGE], need);
+    else atomicAdd(&A.status[ST_UNSTAGED], s_start[own0 + ow] - s_start[own0]);
+  }
   const int a0 = s_src[own0];
   const int nown = s_start[own0 + ow] - s_start[own0];
 
@@ -1080,12 +1083,16 @@ static bool mean_tile_fits(const b200_ctx *c, int tc) {
 //   44: 5,832 cells 347 and 331 us; 62: 4,096 cells 444 and 508; 93: 2,744
 //     cells 1,122 and 1,104; from 108 on, where a tile of two no longer fits
 //     (mean_tile_fits), 891 and 7,744
-// so two from seven tiles per SM and up to 50 atoms per cell.  Four cells took
+// so two from seven tiles per SM and up to 50 atoms per cell on the mean, unless
+// the atoms are so uneven that many two-cell tiles cannot be staged (a slab in
+// vacuum; md_stage_feedback).  Four cells took
 // 41.5 ms where two take 41.1 (a run of 4,000,000 atoms).  Replica boxes are a
 // few cells wide, so half of their two-cell tiles would own one cell (11.78
 // against 11.66 ms).
 int md_tile_cells(const b200_ctx *c) {
-  return !c->nrep && c->ncells >= 7 * md_sms(c) && (double)c->n <= 50.0 * c->ncells ? 2 : 1;
+  return !c->nrep && !c->narrow && c->ncells >= 7 * md_sms(c) && (double)c->n <= 50.0 * c->ncells
+             ? 2
+             : 1;
 }
 
 // Shared memory of the builder tiles, in 16-byte units: what a tile of the
@@ -1122,9 +1129,20 @@ int md_stage_cap2(const b200_ctx *c) {
 // After a build: raise the capacity when some tile needed more than the
 // current one holds and, with `lower` (staged_max is of a single build of the
 // current atoms), bring it down when no tile needs that much any more: it
-// would cost every later system resident blocks.  Returns true when the
-// capacity changed (the caller re-captures its graphs).
-bool md_stage_feedback(b200_ctx *c, int staged_max, bool lower) {
+// would cost every later system resident blocks.  Such a build also narrows the
+// tiles to one cell when more than a fiftieth of the atoms (`unstaged`) lie in
+// two-cell tiles that no capacity can stage: a slab of 219,488 atoms, 127 per
+// cell, in a box three times as long, 12.4 ms a build with two, 1.2 with one.
+// Returns true when the launch changed (the caller re-captures its graphs).
+bool md_stage_feedback(b200_ctx *c, int staged_max, int unstaged, bool lower) {
+  if (lower && c->tile_cells == 2 && unstaged > c->n / 50) {
+    c->narrow = true;
+    c->narrow_n = c->n;
+    c->narrow_cells = c->ncells;
+    c->tile_cells = 1;
+    c->stage_need = 0;
+    return true;
+  }
   auto cap_now = [&] {
     const int cap2 = md_stage_cap2(c);
     return cap2 > 0 ? cap2 : md_stage_cap(c);

@@ -31,16 +31,11 @@ def box(per_cell, cells, ntypes, clump=0, s=None):
     return s, x, edge
 
 
-@pytest.mark.parametrize("per_cell,cells,ntypes,clump", [
-    (52, 11, 1, 0), (110, 11, 1, 0), (145, 11, 2, 0), (170, 11, 1, 0), (40, 11, 1, 600)])
-def test_list(per_cell, cells, ntypes, clump):
-    s, x, edge = box(per_cell, cells, ntypes, clump)
-    s.neigh_build()
+def check_sample(s, x, edge):
+    """Every pair that names one of 150 atoms (the first twenty among them)."""
     n = len(x)
     num, jo, ji = s.half_list()
     assert s.neigh_stats()["full_total"] == 2 * len(jo)
-    s.close()
-    # 150 atoms' neighbours, the clump's among them: every pair that names one
     some = np.zeros(n, bool)
     some[::n // 130] = True
     some[:20] = True
@@ -57,6 +52,15 @@ def test_list(per_cell, cells, ntypes, clump):
         r2[a] = 2.0
         want.append(a * n + np.nonzero(r2 <= 1.0)[0])
     assert np.array_equal(np.sort(got), np.sort(np.concatenate(want)))
+
+
+@pytest.mark.parametrize("per_cell,cells,ntypes,clump", [
+    (52, 11, 1, 0), (110, 11, 1, 0), (145, 11, 2, 0), (170, 11, 1, 0), (40, 11, 1, 600)])
+def test_list(per_cell, cells, ntypes, clump):
+    s, x, edge = box(per_cell, cells, ntypes, clump)
+    s.neigh_build()
+    check_sample(s, x, edge)
+    s.close()
 
 
 def seconds(s, builds=10):
@@ -93,3 +97,44 @@ def test_a_clump_costs_no_later_box(clump):
     after = seconds(s)
     s.close()
     assert after < 1.5 * alone, (alone, after)  # a third of the resident blocks takes three times
+
+
+def test_slab():
+    """A dense slab in a box three times as long: its mean density is that of a
+    thin fluid, its tiles are not.  The list stays the same while the builder
+    finds its width and memory, and a build costs what the slab alone costs."""
+    s, x, edge = box(125, 11, 1)
+    alone = seconds(s)
+    s.close()
+    s, _, _ = box(125, 11, 1)
+    tall = edge * np.array([1.0, 1.0, 3.0])
+    s.set_box(np.zeros(3), tall)
+    s.set_atoms(x)
+    for _ in range(3):
+        s.neigh_build()
+        check_sample(s, x, tall)
+    after = seconds(s)
+    s.close()
+    assert after < 2.0 * alone, (alone, after)  # ten times by the global-memory path
+
+
+def test_width_follows_the_box():
+    """The width that a slab asked for does not stay for a thin fluid, nor does
+    the thin fluid's for the slab."""
+    s, x, edge = box(125, 11, 1)
+    tall = edge * np.array([1.0, 1.0, 3.0])
+    thin, y, wide = box(20, 20, 1)
+    alone = seconds(thin)
+    thin.close()
+    for _ in range(2):
+        s.set_box(np.zeros(3), tall)
+        s.set_atoms(x)
+        for _ in range(3):
+            s.neigh_build()
+        check_sample(s, x, tall)
+        s.set_box(np.zeros(3), wide)
+        s.set_atoms(y)
+        s.neigh_build()
+        check_sample(s, y, wide)
+        assert seconds(s) < 1.5 * alone
+    s.close()
